@@ -1413,7 +1413,7 @@ zc_status zc_sim_create(const zc_sim_desc *d, zc_sim **out) {
   TRYC(dalloc(&s->d_emf, 6));
   TRYC(dalloc(&s->stage, (size_t)(s->nx + 3) * (s->ny + 3) * 3));
   {
-    const int BW = (TX + 6) & ~3, BH = TY + 3;
+    const int BW = push_box_w(TX, s->fast), BH = TY + 3;
     for (int b = 0; b < 2; ++b) {
       TRYC(make_map(&s->tmK_EB[b], s->EB[b], G, 6, BW, BH));
       TRYC(make_map(&s->tmY_EB[b], s->EB[b], G, 6, kYeeBW, kYeeBH));
@@ -1822,7 +1822,7 @@ zc_status zc_set_ext_fld(zc_sim *s, int Et, const float E0[3], const float *Eg, 
   if (!s->EBp) {
     TRY(dalloc(&s->EBp, 6 * s->G.plane));
     CK(cudaMemsetAsync(s->EBp, 0, sizeof(float) * 6 * s->G.plane, s->st));
-    const int BW = (s->TX + 6) & ~3, BH = s->TY + 3;
+    const int BW = push_box_w(s->TX, s->fast), BH = s->TY + 3;
     TRY(make_map(&s->tmK_EBp, s->EBp, s->G, 6, BW, BH));
   }
   TRY(refresh_particle_fields(s));

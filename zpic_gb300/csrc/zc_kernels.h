@@ -106,6 +106,18 @@ __device__ __forceinline__ void spill_particle(const Spill &S, int *errbits, con
 }
 #endif
 
+// columns of a tile's staged E/B box: the tile, one column before it and two
+// after, up to a multiple of 4 and to a pitch that suits the gather.  A warp
+// reads the nodes of some 16 cells of a row, in two rows.  The fast builds
+// read 8-byte pairs, half a warp (8 cells, 9 nodes) at a time: with a pitch
+// of 8 modulo 16 pairs the two rows lie 16 banks apart.  The exact builds
+// read 4-byte values, 17 nodes at a time: 12 modulo 32 keeps most apart.
+// (36 columns, the least for a 32-column tile, put the two rows 4 banks
+// apart: 18 conflicts a unit of 32 particles at 2048^2, 14 with 40 and pairs.)
+__host__ __device__ constexpr int push_box_w(int TX, bool fast) {
+  return TX == 32 ? (fast ? 40 : 44) : (TX == 16 ? (fast ? 24 : 20) : 12);
+}
+
 // particles
 bool tile_supported(int TX, int TY);
 cudaError_t launch_push_tiles(const PushLaunch &a, cudaStream_t st);

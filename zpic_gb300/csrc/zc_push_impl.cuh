@@ -15,18 +15,18 @@
 //                 its current deposited with the zigzag scheme.  Tiles are
 //                 kept sorted by cell, so the lanes of a warp mostly share a
 //                 cell: their gathers are broadcasts, and the current of the
-//                 segment every particle starts with (it lies in the
-//                 particle's own cell) is summed across the lanes of a cell
-//                 with a segmented warp-shuffle reduction before one lane per
-//                 cell deposits it.  The fast and exact builds deposit with
+//                 segment of a particle that stays in its cell is summed in
+//                 the lane's registers (deterministic builds: across the lanes
+//                 of a cell, with a segmented warp-shuffle reduction) before
+//                 it is deposited.  The fast and exact builds deposit with
 //                 float reductions on the global J planes, which L2 performs
 //                 natively; the deterministic builds accumulate a shared
 //                 integer J tile (exact, order-independent sums) and add it
-//                 to the global fixed-point planes.  Cell-crossing motions (a
-//                 few per cent) wait in a per-warp shared-memory queue and are
-//                 split and deposited a warp's worth at a time, so the split
-//                 code runs with (nearly) full warps.  Particles that stay
-//                 are compacted in order; particles that leave go to the
+//                 to the global fixed-point planes.  Cell-crossing particles
+//                 (a few per cent) wait in a per-warp shared-memory queue and
+//                 are finished (motion split and deposited, new cell, leaving
+//                 or staying) a warp's worth at a time, so that code runs with
+//                 (nearly) full warps.  Particles that leave go to the
 //                 tile's outbox, from which the destination tile pulls them
 //                 at the start of the next step's push.
 //   k_push_spill  the same physics for particles that did not fit a tile,
@@ -168,6 +168,75 @@ __device__ __forceinline__ float lerp2(const F &f, int c, int a, int b, float wa
          (f(c, a, b + 1) * (1.0f - wa) + f(c, a + 1, b + 1) * wa) * wb;
 }
 
+// staggered bilinear interpolation at (x, y) of cell (i, j) of the accessor
+// frame (interpolate_fld, particles.c:1029-1071)
+template <class F>
+__device__ __forceinline__ void gather(const F &fld, int i, int j, float x, float y, float &ex, float &ey, float &ez,
+                                       float &bx, float &by, float &bz) {
+  const int ih = i + ((x < 0.5f) ? -1 : 0);
+  const int jh = j + ((y < 0.5f) ? -1 : 0);
+  const float w1h = x + ((x < 0.5f) ? 0.5f : -0.5f);
+  const float w2h = y + ((y < 0.5f) ? 0.5f : -0.5f);
+  ex = lerp2(fld, 0, ih, j, w1h, y);
+  ey = lerp2(fld, 1, i, jh, x, w2h);
+  ez = lerp2(fld, 2, i, j, x, y);
+  bx = lerp2(fld, 3, i, jh, x, w2h);
+  by = lerp2(fld, 4, ih, j, w1h, y);
+  bz = lerp2(fld, 5, ih, jh, w1h, w2h);
+}
+
+#ifdef ZC_FAST
+// Fast builds: Ex and By are interpolated at the same nodes with the same
+// weights, and so are Ey and Bx.  The tile keeps each of the two as pairs
+// (one 8-byte load instead of two of 4), and all six components are
+// interpolated two at a time with packed float pairs: 16 loads and 18 packed
+// operations a particle instead of 24 and 36.
+template <int BW, int PL>
+struct TilePairs {
+  const float2 *xb, *yb;  // (Ex, By), (Ey, Bx)
+  const float *ez, *bz;
+};
+
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 lerp2p(float2 a, float2 b, float2 c, float2 d, float2 wx, float2 wy) {
+  const float2 lo = __ffma2_rn(wx, sub2(b, a), a), hi = __ffma2_rn(wx, sub2(d, c), c);
+  return __ffma2_rn(wy, sub2(hi, lo), lo);
+}
+
+template <int BW, int PL>
+__device__ __forceinline__ void gather(const TilePairs<BW, PL> &f, int i, int j, float x, float y, float &ex,
+                                       float &ey, float &ez, float &bx, float &by, float &bz) {
+  const bool lx = x < 0.5f, ly = y < 0.5f;
+  const float xh = x + (lx ? 0.5f : -0.5f), yh = y + (ly ? 0.5f : -0.5f);
+  const int s = (j + 1) * BW + (i + 1);
+  const int sx = s - (lx ? 1 : 0), sy = s - (ly ? BW : 0), sc = sx - (ly ? BW : 0);
+  const float2 *a = f.xb + sx, *b = f.yb + sy;
+  const float2 r0 = lerp2p(a[0], a[1], a[BW], a[BW + 1], make_float2(xh, xh), make_float2(y, y));
+  const float2 r1 = lerp2p(b[0], b[1], b[BW], b[BW + 1], make_float2(x, x), make_float2(yh, yh));
+  const float *e = f.ez + s, *g = f.bz + sc;
+  const float2 r2 = lerp2p(make_float2(e[0], g[0]), make_float2(e[1], g[1]), make_float2(e[BW], g[BW]),
+                           make_float2(e[BW + 1], g[BW + 1]), make_float2(x, xh), make_float2(y, yh));
+  ex = r0.x;
+  by = r0.y;
+  ey = r1.x;
+  bx = r1.y;
+  ez = r2.x;
+  bz = r2.y;
+}
+
+// the arguments here are sums of 1 and squares: never denormal
+__device__ __forceinline__ float rsqrt_ftz(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float rcp_ftz(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+#endif
+
 struct Seg {
   float x0, x1, y0, y1, dx, dy, qvz;
   int ix, iy;
@@ -181,26 +250,29 @@ struct SegCurrent {
 };
 
 __device__ __forceinline__ SegCurrent segment_current(const Seg &s, float qnx, float qny) {
-#ifdef ZC_FAST_ALGEBRA
-  // the same weights, re-associated (fast build only): Jx, Jy from the
-  // segment's mid-point; each Jz corner q (a (c + d/2) + b (d - c/2)) with
-  // a, b its start / end x weights and c, d its start / end y weights
+#ifdef ZC_FAST
+  // the same weights, re-associated (fast builds), two at a time: Jx, Jy
+  // from the segment's mid-point; with p, m = c + d/2, d - c/2 of the start /
+  // end y weights c, d of a row, the Jz corners of that row are
+  // q (a p + b m), a, b the start / end x weights, which add up to q (p + m)
   SegCurrent r;
   const float jx = qnx * s.dx, jy = qny * s.dy;
   const float ym = 0.5f * (s.y0 + s.y1), xm = 0.5f * (s.x0 + s.x1);
-  r.v[1] = jx * ym;
-  r.v[0] = jx - r.v[1];
-  r.v[3] = jy * xm;
-  r.v[2] = jy - r.v[3];
-  const float c0 = 1.0f - s.y0, d0 = 1.0f - s.y1;
-  const float p0 = c0 + 0.5f * d0, m0 = d0 - 0.5f * c0;
+  const float2 j1 = __fmul2_rn(make_float2(jx, jy), make_float2(ym, xm));
+  const float2 j0 = sub2(make_float2(jx, jy), j1);
   const float p1 = s.y0 + 0.5f * s.y1, m1 = s.y1 - 0.5f * s.y0;
-  const float a0 = 1.0f - s.x0, b0 = 1.0f - s.x1;
-  const float q = s.qvz;
-  r.v[4] = q * (a0 * p0 + b0 * m0);
-  r.v[5] = q * (s.x0 * p0 + s.x1 * m0);
-  r.v[6] = q * (a0 * p1 + b0 * m1);
-  r.v[7] = q * (s.x0 * p1 + s.x1 * m1);
+  const float2 q = make_float2(s.qvz, s.qvz);
+  const float2 qp = __fmul2_rn(q, make_float2(1.5f - p1, p1)), qm = __fmul2_rn(q, make_float2(0.5f - m1, m1));
+  const float2 z1 = __ffma2_rn(make_float2(s.x1, s.x1), qm, __fmul2_rn(make_float2(s.x0, s.x0), qp));
+  const float2 z0 = sub2(__fadd2_rn(qp, qm), z1);
+  r.v[0] = j0.x;
+  r.v[1] = j1.x;
+  r.v[2] = j0.y;
+  r.v[3] = j1.y;
+  r.v[4] = z0.x;
+  r.v[5] = z1.x;
+  r.v[6] = z0.y;
+  r.v[7] = z1.y;
   return r;
 #else
   const float s0x0 = 1.0f - s.x0, s0x1 = s.x0;
@@ -317,26 +389,31 @@ __device__ __forceinline__ Seg zigzag_first(const D &dep, int ix, int iy, int di
   return a;
 }
 
-// gather + Boris + move for one particle at cell (i, j) of the accessor
-// frame (particles.c:1029-1207); leaves the displacement in (mx, my) and the
-// cell shift in (di, dj), returns the kinetic-energy term utsq/(gamma+1).
-// `bad` flags a motion of one cell or more (or NaN), which the deposit does
-// not support.  A trimmed position of exactly 1.0f (x1 = -tiny, +1 rounds up)
-// is legal, as in the reference.
+// displacement (cells) and q v_z of a particle with the new momentum
+__device__ __forceinline__ void displacement(float ux, float uy, float uz, float &mx, float &my, float &qvz,
+                                             const PushConst &C) {
+#ifdef ZC_FAST
+  const float rg = rsqrt_ftz(1.0f + ux * ux + uy * uy + uz * uz);
+#else
+  const float rg = 1.0f / sqrtf(1.0f + ux * ux + uy * uy + uz * uz);
+#endif
+  mx = C.dt_dx * rg * ux;
+  my = C.dt_dy * rg * uy;
+  qvz = C.q * uz * rg;
+}
+
+// gather + Boris for one particle at cell (i, j) of the accessor frame
+// (particles.c:1029-1207); leaves the displacement in (mx, my), returns the
+// kinetic-energy term utsq/(gamma+1).  A motion of one cell or more (or NaN)
+// is not supported by the deposit: the callers flag it.  A trimmed position
+// of exactly 1.0f (x + mx = -tiny, +1 rounds up) is legal, as in the
+// reference.
 template <class F>
-__device__ __forceinline__ float push_particle(const F &fld, int i, int j, float &x, float &y, float &ux,
-                                               float &uy, float &uz, float &mx, float &my, float &x1, float &y1,
-                                               int &di, int &dj, float &qvz, bool &bad, const PushConst &C) {
-  const int ih = i + ((x < 0.5f) ? -1 : 0);
-  const int jh = j + ((y < 0.5f) ? -1 : 0);
-  const float w1h = x + ((x < 0.5f) ? 0.5f : -0.5f);
-  const float w2h = y + ((y < 0.5f) ? 0.5f : -0.5f);
-  float ex = lerp2(fld, 0, ih, j, w1h, y);
-  float ey = lerp2(fld, 1, i, jh, x, w2h);
-  float ez = lerp2(fld, 2, i, j, x, y);
-  float bx = lerp2(fld, 3, i, jh, x, w2h);
-  float by = lerp2(fld, 4, ih, j, w1h, y);
-  float bz = lerp2(fld, 5, ih, jh, w1h, w2h);
+__device__ __forceinline__ float push_particle(const F &fld, int i, int j, float x, float y, float &ux,
+                                               float &uy, float &uz, float &mx, float &my, float &qvz,
+                                               const PushConst &C) {
+  float ex, ey, ez, bx, by, bz;
+  gather(fld, i, j, x, y, ex, ey, ez, bx, by, bz);
 
   const float tem = C.tem;
   ex *= tem;
@@ -344,13 +421,23 @@ __device__ __forceinline__ float push_particle(const F &fld, int i, int j, float
   ez *= tem;
   float tx = ux + ex, ty = uy + ey, tz = uz + ez;
   const float u2 = tx * tx + ty * ty + tz * tz;
+#ifdef ZC_FAST
+  const float g2 = 1.0f + u2, ig = rsqrt_ftz(g2);
+  const float kin = u2 * rcp_ftz(g2 * ig + 1.0f);
+  const float tg = tem * ig;
+#else
   const float g = sqrtf(1.0f + u2);
   const float kin = u2 / (g + 1);
   const float tg = tem / g;
+#endif
   bx *= tg;
   by *= tg;
   bz *= tg;
+#ifdef ZC_FAST
+  const float s2 = 2.0f * rcp_ftz(1.0f + bx * bx + by * by + bz * bz);
+#else
   const float s2 = 2.0f / (1.0f + bx * bx + by * by + bz * bz);
+#endif
   float vx = tx + ty * bz - tz * by;
   float vy = ty + tz * bx - tx * bz;
   float vz = tz + tx * by - ty * bx;
@@ -364,17 +451,7 @@ __device__ __forceinline__ float push_particle(const F &fld, int i, int j, float
   uy = ty + ey;
   uz = tz + ez;
 
-  const float rg = 1.0f / sqrtf(1.0f + ux * ux + uy * uy + uz * uz);
-  mx = C.dt_dx * rg * ux;
-  my = C.dt_dy * rg * uy;
-  bad = !(fabsf(mx) < 1.0f && fabsf(my) < 1.0f);
-  x1 = x + mx;
-  y1 = y + my;
-  di = (x1 >= 1.0f) - (x1 < 0.0f);
-  dj = (y1 >= 1.0f) - (y1 < 0.0f);
-  x1 -= di;
-  y1 -= dj;
-  qvz = C.q * uz * rg;
+  displacement(ux, uy, uz, mx, my, qvz, C);
   return kin;
 }
 
@@ -410,25 +487,43 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 // warps after the own ones and appended after slot np.  The main loop has
 // no block-wide barrier.
 //
-// Warp w takes the chunks w, w + NW, ... of kChunk slots, 32 slots at a
-// time.  In the float builds lane l meets the chunk's particles l kLaneRun
-// ... l kLaneRun + kLaneRun - 1 of the sorted order one after another, and
-// sums their single-segment currents in registers while they stay in one
-// cell; a lane adds its sums to J when its cell changes.  The deterministic
-// builds read every chunk in cell order across the lanes and pre-reduce
-// with segmented warp sums of fixed-point parts.
+// Every warp takes an equal, contiguous share of the tile's slots, 32 slots
+// (a unit) at a time.  In the float builds lane l meets the particles
+// l kLaneRun ... l kLaneRun + kLaneRun - 1 of a chunk of the sorted order one
+// after another, and sums their single-segment currents in registers while
+// they stay in one cell; a lane adds its sums to J when its cell changes.
+// The deterministic builds read every chunk in cell order across the lanes
+// and pre-reduce with segmented warp sums of fixed-point parts.
+//
+// What bounds it (fast build, 2048^2 cells, 67 M particles): no single unit.
+// A launch takes 0.940 ms against 0.49 ms for its 48 bytes a particle at the
+// measured HBM rate, with 57 % of the issue slots, 60 % of the L1 data passes,
+// 62 % of the SM's request port (the reductions on J) and 43 % of DRAM in
+// use, and a third of a warp's time spent waiting for its next particles.
+// It took 0.993 ms and 446 instructions a unit (307 now) before the work of
+// cell-crossing particles moved out of the main loop, the float pairs, the
+// contiguous shares and the particle prefetch in registers; writing the tile back in cell order from here (in
+// place of the sort pass) was slower (1.13 ms): scattered 16-byte stores
+// make L2 fetch what they do not cover.
 // ---------------------------------------------------------------------------
-// resident CTAs per SM the float builds are compiled for: 7 (up to 72
-// registers a thread) measured faster than 8 (64, with spills) and 6
+// resident CTAs per SM the float builds are compiled for: 6 (up to 80
+// registers a thread) measured faster than 7 (72, spilling in the main loop;
+// the shared memory of 7 tiles leaves little L1 to catch the spills: 1.058
+// against 0.942 ms a 2048^2 launch) and 5 (0.931 there, but 8 % slower on
+// grids of about a thousand tiles, which then take two rounds)
 #ifndef ZC_PUSH_MIN_CTAS
-#define ZC_PUSH_MIN_CTAS 7
+#define ZC_PUSH_MIN_CTAS 6
 #endif
 template <int TX, int TY, int NT, bool DET>
 __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push_tiles(const __grid_constant__ CUtensorMap tm_eb,
                                                    Particles pin,
                                                    Particles pout, TileSet T, Outbox Oin, Outbox O, Spill S,
                                                    double *ekin_tile, int *err, PushConst C, FixedJ fj) {
-  constexpr int BW = (TX + 3 + 3) & ~3;  // halo box width, multiple of 4 floats
+#ifdef ZC_FAST
+  constexpr int BW = push_box_w(TX, true);
+#else
+  constexpr int BW = push_box_w(TX, false);
+#endif
   constexpr int BH = TY + 3;
   constexpr int PL = BW * BH;
   constexpr int NW = NT / 32;
@@ -439,17 +534,14 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   __shared__ unsigned long long s_ekin[2];                // fixed-point kinetic energy (DET)
   __shared__ __align__(8) uint64_t bar;
   __shared__ double sred[NW];
-  // per-warp queue of cell-crossing motions, deposited 32 at a time so that
-  // the split code runs with (nearly) full warps: flushed from QFLUSH
-  // waiting motions on, so at most QFLUSH - 1 + 32 are held
-  constexpr int QFLUSH = DET ? 24 : 32;
-  constexpr int QCAP = QFLUSH - 1 + 32;
-  __shared__ float qf[NW][5][QCAP];  // x0, y0, dx, dy, qvz
-  __shared__ int qi[NW][QCAP];       // local cell and shifts, packed
-  // prefetched particles, 32 slots per warp: each lane reads its slot into
-  // registers before it copies the next slot's particle into it
-  __shared__ __align__(16) float4 pf_u[NW][32];
-  __shared__ __align__(16) float2 pf_xy[NW][32];
+  // per-warp queue of the particles that need more than the common case (see
+  // `finish`): x, y before and ux, uy, uz after the push, the cell word and
+  // the own slot; finished 32 at a time, so at most 31 wait when the next
+  // unit's 32 lanes queue theirs
+  constexpr int QCAP = 63;
+  __shared__ float qf[NW][5][QCAP];
+  __shared__ unsigned qc[NW][QCAP];
+  __shared__ int qs[NW][QCAP];
   __shared__ int nb[8], s_nnb;        // distinct neighbour tiles
   // incoming particles bound for this tile, listed as (outbox slot << 4 |
   // neighbour) so that they are pushed in full warps
@@ -466,44 +558,106 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   int errbits = 0;
   int qcount = 0;  // warp-uniform
 
+  const unsigned base = (unsigned)T.off[t];  // (tile offsets are below 2^31)
+  const int cap = T.cap[t];
+  const int n_own = T.np[t];
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
-    int c = 0;
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        if (!dx && !dy) continue;
-        int x = tx + dx, y = ty + dy;
-        y += (y < 0) ? C.nty : 0;
-        y -= (y >= C.nty) ? C.nty : 0;
-        if (x < 0 || x >= C.ntx) {
-          if (C.mw) continue;
-          x = (x + C.ntx) % C.ntx;
-        }
-        const int id = x + y * C.ntx;
-        bool dup = (id == t);
-        for (int m = 0; m < c; ++m) dup |= (nb[m] == id);
-        if (!dup) nb[c++] = id;
-      }
-    s_nnb = c;
+    mbar_expect_tx(&bar, 6 * PL * 4);
+    tma_load_3d(sEB, &tm_eb, cx0, cy0, 0, &bar);
     s_nin = 0;
     s_app = 0;
     s_leave = 0;
     s_ekin[0] = 0;
     s_ekin[1] = 0;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    mbar_expect_tx(&bar, 6 * PL * 4);
-    tma_load_3d(sEB, &tm_eb, cx0, cy0, 0, &bar);
+  if (warp == NW - 1) {
+    // the distinct neighbour tiles, one a lane
+    const int m = lane + (lane >= 4);  // 3 x 3 without the middle
+    int x = tx + m % 3 - 1, y = ty + m / 3 - 1;
+    y += (y < 0) ? C.nty : 0;
+    y -= (y >= C.nty) ? C.nty : 0;
+    const bool out = x < 0 || x >= C.ntx;
+    x += (x < 0) ? C.ntx : 0;
+    x -= (x >= C.ntx) ? C.ntx : 0;
+    const int id = x + y * C.ntx;
+    const bool is = lane < 8 && !(out && C.mw) && id != t;
+    const unsigned same = __match_any_sync(0xffffffffu, is ? id : -1 - lane);
+    const bool first = is && __ffs(same) - 1 == lane;
+    const unsigned fm = __ballot_sync(0xffffffffu, first);
+    if (first) nb[__popc(fm & below)] = id;
+    if (lane == 0) s_nnb = __popc(fm);
+  }
+  // This warp's slots: an equal share of the tile's units of 32 slots, one
+  // contiguous run (equal to a unit, so that no warp waits a chunk's time for
+  // another at the end).  Its first unit is on its way before the fields are.
+  const int units = (n_own + 31) / 32;
+  const int share = units / NW, extra = units % NW;
+  const int c_begin = 32 * (warp * share + min(warp, extra));
+  const int c_end = min(n_own, c_begin + 32 * (share + (warp < extra ? 1 : 0)));
+  // this lane's slot in the unit that starts at slot c
+  const auto slot_of = [&](int c) {
+    if constexpr (DET) {
+      const int c0 = c & ~(kChunk - 1), j = (c & (kChunk - 1)) + lane;
+      if (c0 + kChunk <= n_own) return c0 + (j % kLaneRun) * 32 + j / kLaneRun;
+    }
+    return c + lane;
+  };
+  // a lane without a particle carries the last unit's particle, a hole's
+  // zero momenta, or these zeros: finite values whose results `valid` masks;
+  // its position is set to the cell centre (a hole's is stale)
+  float4 nu = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 nxy = make_float2(0.f, 0.f);
+  int ns = slot_of(c_begin);
+  if (c_begin < c_end && ns < n_own) {
+    nu = __ldcs(&pin.u[base + ns]);
+    nxy = __ldcs(&pin.xy[base + ns]);
   }
   if constexpr (DET)
     for (int k = threadIdx.x; k < 3 * LAY::N; k += NT) sJi[k] = 0;
+  __syncthreads();
+  // the outboxes of this warp's neighbours: counts and first entries
+  constexpr int NBW = (8 + NW - 1) / NW;
+  const int nnb = s_nnb;
+  int in_n[NBW], in_dst[NBW];
+#pragma unroll
+  for (int q = 0; q < NBW; ++q) {
+    const int m = warp + q * NW;
+    in_n[q] = m < nnb ? Oin.cnt[nb[m]] : 0;
+    in_dst[q] = (m < nnb && lane < Oin.cap) ? Oin.dst[(long long)nb[m] * Oin.cap + lane] : -1;
+  }
   const bool loaded = mbar_wait_bounded(&bar, 0);
   if (!loaded) errbits |= ERR_TIMEOUT;
-  __syncthreads();
 
+#ifdef ZC_FAST
+  // in place: planes Ex Ey Ez Bx By Bz -> Ez, Bz, pairs (Ex, By), (Ey, Bx)
+  {
+    constexpr int NK = (PL + NT - 1) / NT;
+    float v[NK][6];
+#pragma unroll
+    for (int n = 0; n < NK; ++n) {
+      const int k = min((int)threadIdx.x + n * NT, PL - 1);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) v[n][c] = sEB[c * PL + k];
+    }
+    __syncthreads();
+    float2 *xb = reinterpret_cast<float2 *>(sEB + 2 * PL), *yb = xb + PL;
+#pragma unroll
+    for (int n = 0; n < NK; ++n) {
+      const int k = min((int)threadIdx.x + n * NT, PL - 1);
+      sEB[k] = v[n][2];
+      sEB[PL + k] = v[n][5];
+      xb[k] = make_float2(v[n][0], v[n][4]);
+      yb[k] = make_float2(v[n][1], v[n][3]);
+    }
+    __syncthreads();
+  }
+  const TilePairs<BW, PL> fld{reinterpret_cast<const float2 *>(sEB + 2 * PL),
+                              reinterpret_cast<const float2 *>(sEB + 4 * PL), sEB, sEB + PL};
+#else
   const TileFields<BW, PL> fld{sEB};
+#endif
   const PushConst Cl = C;
   const auto dep = [&] {
     if constexpr (DET)
@@ -511,93 +665,65 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
     else
       return TileCurrentGlobal{fj.f + (size_t)(cy0 + 1) * fj.pitch + (cx0 + 1), fj.pitch, fj.plane};
   }();
-  const long long base = T.off[t];
-  const int cap = T.cap[t];
-  const int n_own = T.np[t];
   const long long obase = (long long)t * O.cap;
-  const int nnb = s_nnb;
   float ks = 0.f, kc = 0.f;
   long long khi = 0, klo = 0;  // DET: fixed-point kinetic energy of this thread's particles
-  // float builds: this lane's running single-segment current and its local
-  // cell (-1: none)
+  // float builds: this lane's running single-segment current and its cell
+  // word (kHole: none)
   SegCurrent acc;
 #pragma unroll
   for (int q = 0; q < 8; ++q) acc.v[q] = 0.f;
-  int acc_key = -1;
+  unsigned acc_cell = kHole;
+  // the bits of a cell word that all cells of this tile share
+  const unsigned tile_mask = ~((unsigned)(TX - 1) | (unsigned)(TY - 1) << 16);
+  const unsigned tile_word = (unsigned)cx0 | (unsigned)cy0 << 16;
 
-  // deposits queued motion e of this warp (all segments, direct atomics)
-  auto deposit_queued = [&](int e) {
-    const int w = qi[warp][e];
-    const int qli = w & 0xff, qlj = (w >> 8) & 0xff, qdi = ((w >> 16) & 3) - 1, qdj = ((w >> 18) & 3) - 1;
-    const Seg a = zigzag_first(dep, qli, qlj, qdi, qdj, qf[warp][0][e], qf[warp][1][e], qf[warp][2][e],
-                               qf[warp][3][e], Cl.qnx, Cl.qny, qf[warp][4][e]);
-    add_current(dep, a.ix, a.iy, segment_current(a, Cl.qnx, Cl.qny));
-  };
-
-  // one particle per lane: push, deposit, boundary, output; the 32 lanes of
-  // a warp call it together (warp-level collectives only).  `oslot` is the
-  // lane's own slot (>= 0: the output goes back there, a particle or a
-  // hole) or negative (no own slot); `incoming` marks arriving particles,
-  // which are appended after slot np if they stay.
-  auto process = [&](bool valid, int oslot, bool incoming, int ix, int iy, float x, float y, float ux, float uy,
-                     float uz) {
-    // every lane runs the same instructions; invalid lanes carry a zero
-    // particle and are masked out by `valid` where it matters
-    int li = ix - cx0, lj = iy - cy0;
-    errbits |= (valid && ((unsigned)li >= (unsigned)TX || (unsigned)lj >= (unsigned)TY)) ? ERR_ESCAPE : 0;
-    li = min(max(li, 0), TX - 1);  // keeps the accesses inside the halo
-    lj = min(max(lj, 0), TY - 1);
-    ix = cx0 + li;
-    iy = cy0 + lj;
-    float mx, my, x1, y1, qvz;
-    int di, dj;
-    bool bad;
-    const float kin = push_particle(fld, li, lj, x, y, ux, uy, uz, mx, my, x1, y1, di, dj, qvz, bad, Cl);
-    if constexpr (DET) {
-      long long h, l;
-      efix_split(valid ? kin : 0.0f, h, l);
-      khi += h;
-      klo += l;
-    } else {
-      kahan_add(ks, kc, valid ? kin : 0.f);
+  // Finishes the last (at most 32) queued particles of this warp: the
+  // current of all segments of the motion, the new cell, and the particle to
+  // its slot, to the end of the tile or to the outbox.  Cell crossings (a few
+  // per cent of the particles), the columns a window shift moves out of the
+  // tile and arrivals come here; everything that only they need (the split,
+  // the boundary, the destination tile, the slot counters) stays out of the
+  // main loop and runs with nearly full warps.
+  auto finish = [&]() {
+    const int nq = min(qcount, 32);
+    qcount -= nq;
+    const bool act = lane < nq;
+    const int e = qcount + (act ? lane : 0);
+    const unsigned cw = qc[warp][e];
+    const int oslot = qs[warp][e];
+    float x = qf[warp][0][e], y = qf[warp][1][e];
+    const float ux = qf[warp][2][e], uy = qf[warp][3][e], uz = qf[warp][4][e];
+    int ix = (int)(cw & 0xffffu), iy = (int)(cw >> 16);
+    int di = 0, dj = 0, code = 0, dest = 0;  // code: 0 gone, 1 stays, 2 leaves
+    if (act) {
+      float mx, my, qvz;
+      displacement(ux, uy, uz, mx, my, qvz, Cl);  // as the push had it
+      errbits |= !(fabsf(mx) < 1.0f && fabsf(my) < 1.0f) ? ERR_ESCAPE : 0;
+      float x1 = x + mx, y1 = y + my;
+      di = (x1 >= 1.0f) - (x1 < 0.0f);
+      dj = (y1 >= 1.0f) - (y1 < 0.0f);
+      x1 -= di;
+      y1 -= dj;
+      const Seg a = zigzag_first(dep, ix & (TX - 1), iy & (TY - 1), di, dj, x, y, mx, my, Cl.qnx, Cl.qny, qvz);
+      add_current(dep, a.ix, a.iy, segment_current(a, Cl.qnx, Cl.qny));
+      x = x1;
+      y = y1;
+      const bool keep = apply_boundary(ix, iy, di, dj, Cl);
+      // (the cell is inside the grid when the particle is kept; dest is unused otherwise)
+      dest = (int)((unsigned)ix / TX) + (int)((unsigned)iy / TY) * Cl.ntx;
+      code = keep ? ((dest == t) ? 1 : 2) : 0;
+      if (oslot >= 0) {
+        if (code == 1) store_particle(pout, base + oslot, ix, iy, x, y, ux, uy, uz);
+        else store_hole(pout, base + oslot);
+      }
     }
-    errbits |= (valid && bad) ? ERR_ESCAPE : 0;
-    const bool split = valid && ((di != 0) || (dj != 0));
-    const bool single = valid && !split;
-    // the whole motion inside the cell: one segment (particles.c:781-797);
-    // crossing motions are queued below and contribute nothing here: every
-    // contribution is proportional to dx, dy or qvz, so zeroing those three
-    // zeroes all eight
-    Seg a;
-    a.x0 = x;
-    a.y0 = y;
-    a.dx = single ? mx : 0.f;
-    a.dy = single ? my : 0.f;
-    a.x1 = x + mx;
-    a.y1 = y + my;
-    a.qvz = single ? qvz * 0.5f : 0.f;
-    a.ix = li;
-    a.iy = lj;
-    SegCurrent cur = segment_current(a, Cl.qnx, Cl.qny);
-    const float sx0 = x, sy0 = y, smx = mx, smy = my, sqvz = qvz;
-    const int spk = li | (lj << 8) | ((di + 1) << 16) | ((dj + 1) << 18);
-    x = x1;
-    y = y1;
-    const bool keep = apply_boundary(ix, iy, di, dj, Cl);
-    // (the cell is inside the grid when the particle is kept; dest is unused otherwise)
-    const int dest = (int)((unsigned)ix / TX) + (int)((unsigned)iy / TY) * Cl.ntx;
-    const int code = (valid && keep) ? ((dest == t) ? 1 : 2) : 0;  // 1 stays, 2 leaves
-
-    // output, before the current sums so that the particle's registers are
-    // free while they run: an own slot takes the particle back, or a hole
-    if (oslot >= 0) {
-      if (code == 1) store_particle(pout, base + oslot, ix, iy, x, y, ux, uy, uz);
-      else store_hole(pout, base + oslot);
-    }
+    __syncwarp();
     // leavers to the outbox, arrivals that stay appended after slot np: one
     // shared-memory atomic per warp and kind
+    const bool app = code == 1 && oslot < 0;
     const unsigned mleave = __ballot_sync(0xffffffffu, code == 2);
-    const unsigned mapp = incoming ? __ballot_sync(0xffffffffu, code == 1) : 0u;
+    const unsigned mapp = __ballot_sync(0xffffffffu, app);
     if (mleave | mapp) {
       int lb = 0, ab = 0;
       if (lane == 0) {
@@ -614,12 +740,83 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
         } else {
           spill_particle(S, &errbits, ix, iy, x, y, ux, uy, uz);
         }
-      } else if (incoming && code == 1) {
+      } else if (app) {
         const int s = n_own + ab + __popc(mapp & below);
         if (s < cap) store_particle(pout, base + s, ix, iy, x, y, ux, uy, uz);
         else spill_particle(S, &errbits, ix, iy, x, y, ux, uy, uz);
       }
     }
+    __syncwarp();  // the queue is read before it is filled again
+  };
+
+  // One particle per lane: push, and in the common case (it stays in its
+  // cell) current and output right here: the cell word is written back as it
+  // was read.  The other particles are queued for `finish`.  The 32 lanes of
+  // a warp call it together (warp-level collectives only).  `oslot` is the
+  // lane's own slot (>= 0) or negative (none); `incoming` marks arriving
+  // particles, which have no slot yet and all go through the queue.  A lane
+  // without a particle (`valid` false) runs the same instructions on finite
+  // values; its slot, a hole, is written as the hole it is.
+  auto process = [&](bool valid, int oslot, bool incoming, unsigned cw, float x, float y, float ux, float uy,
+                     float uz) {
+    // the cell in the tile (sizes are powers of two, the tile starts at a
+    // multiple of them): always inside the staged halo
+    errbits |= (valid && ((cw ^ tile_word) & tile_mask)) ? ERR_ESCAPE : 0;
+    const int li = (int)(cw & (TX - 1)), lj = (int)((cw >> 16) & (TY - 1));
+    float mx, my, qvz;
+    const float x0 = x, y0 = y;
+    const float kin = push_particle(fld, li, lj, x, y, ux, uy, uz, mx, my, qvz, Cl);
+    if constexpr (DET) {
+      long long h, l;
+      efix_split(valid ? kin : 0.0f, h, l);
+      khi += h;
+      klo += l;
+    } else {
+      kahan_add(ks, kc, valid ? kin : 0.f);
+    }
+    const float x1 = x0 + mx, y1 = y0 + my;
+    // inside [0, 1) on both axes, as unsigned bit patterns (negative values,
+    // -0 and NaN compare above); `finish` tells the cases apart
+    const unsigned top = max((unsigned)__float_as_int(x1), (unsigned)__float_as_int(y1));
+    const bool queue = valid && (incoming || top >= 0x3f800000u || li < Cl.shift);
+    const bool single = valid && !queue;
+    // the output, before the current sums so that the particle's registers
+    // are free while they run
+    if (oslot >= 0 && !queue) {
+      pout.u[base + oslot] = make_float4(ux, uy, uz, __int_as_float((int)(valid ? cw - (unsigned)Cl.shift : kHole)));
+      pout.xy[base + oslot] = make_float2(x1, y1);
+    }
+    {
+      const unsigned qm = __ballot_sync(0xffffffffu, queue);
+      if (qm) {
+        if (queue) {
+          const int e = qcount + __popc(qm & below);
+          qf[warp][0][e] = x0;
+          qf[warp][1][e] = y0;
+          qf[warp][2][e] = ux;
+          qf[warp][3][e] = uy;
+          qf[warp][4][e] = uz;
+          qc[warp][e] = cw;
+          qs[warp][e] = oslot;
+        }
+        qcount += __popc(qm);
+        __syncwarp();
+      }
+    }
+    // the whole motion inside the cell: one segment (particles.c:781-797);
+    // the other lanes contribute nothing here: every contribution is
+    // proportional to dx, dy or qvz, so zeroing those three zeroes all eight
+    Seg a;
+    a.x0 = x0;
+    a.y0 = y0;
+    a.dx = single ? mx : 0.f;
+    a.dy = single ? my : 0.f;
+    a.x1 = x1;
+    a.y1 = y1;
+    a.qvz = single ? qvz * 0.5f : 0.f;
+    a.ix = li;
+    a.iy = lj;
+    SegCurrent cur = segment_current(a, Cl.qnx, Cl.qny);
 
     if constexpr (DET) {
       // segmented warp reduction of the single-segment currents over runs
@@ -666,53 +863,39 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
     } else {
       // the lane's running sum: added to J when the lane's cell changes
       // (the sum is over this lane's particles of one cell, in order)
-      const int key = li + lj * TX;
-      const bool change = valid && key != acc_key;
-      const bool flush = change && acc_key >= 0;
-      if (__any_sync(0xffffffffu, flush)) {
-        if (flush) add_current(dep, acc_key % TX, acc_key / TX, acc);
-      }
-      const float carry = change ? 0.0f : 1.0f;
+      const bool change = single && cw != acc_cell;
+      if (change && acc_cell != kHole) add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
+      const float carry = change ? 0.0f : 1.0f;  // acc + cur, or cur
+#ifdef ZC_FAST
+      constexpr int pa[4] = {0, 1, 4, 5};  // pairs (0, 2), (1, 3), (4, 6), (5, 7), as they were computed
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc.v[q] = __fmaf_rn(acc.v[q], carry, cur.v[q]);  // acc + cur, or cur
-      acc_key = change ? key : acc_key;
-    }
-
-    // queue the cell-crossing motions; deposit them once QFLUSH are waiting
-    {
-      const unsigned sm = __ballot_sync(0xffffffffu, split);
-      if (sm) {
-        if (split) {
-          const int e = qcount + __popc(sm & below);
-          qf[warp][0][e] = sx0;
-          qf[warp][1][e] = sy0;
-          qf[warp][2][e] = smx;
-          qf[warp][3][e] = smy;
-          qf[warp][4][e] = sqvz;
-          qi[warp][e] = spk;
-        }
-        qcount += __popc(sm);
-        __syncwarp();
-        if (qcount >= QFLUSH) {
-          const int nq = min(qcount, 32);
-          qcount -= nq;
-          if (lane < nq) deposit_queued(qcount + lane);
-          __syncwarp();
-        }
+      for (int k = 0; k < 4; ++k) {
+        const int q = pa[k];
+        const float2 v = __ffma2_rn(make_float2(acc.v[q], acc.v[q + 2]), make_float2(carry, carry),
+                                    make_float2(cur.v[q], cur.v[q + 2]));
+        acc.v[q] = v.x;
+        acc.v[q + 2] = v.y;
       }
+#else
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc.v[q] = __fmaf_rn(acc.v[q], carry, cur.v[q]);
+#endif
+      acc_cell = change ? cw : acc_cell;
     }
   };
 
   // incoming particles: warp w scans the outboxes of neighbours w, w + NW,
   // ... for the slots bound for this tile and lists them; a full list
   // leaves the rest to be pushed right here
-  for (int m = warp; m < nnb; m += NW) {
-    const int src = nb[m];
-    const int n = Oin.cnt[src];
-    const long long ob = (long long)src * Oin.cap;
+#pragma unroll
+  for (int q = 0; q < NBW; ++q) {
+    const int m = warp + q * NW;
+    if (m >= nnb) break;
+    const int n = in_n[q];
+    const long long ob = (long long)nb[m] * Oin.cap;
     for (int e0 = 0; e0 < n; e0 += 32) {
       const int e = e0 + lane;
-      const bool bound = e < n && Oin.dst[ob + e] == t;
+      const bool bound = e < n && (e0 == 0 ? in_dst[q] : Oin.dst[ob + e]) == t;
       const unsigned bm = __ballot_sync(0xffffffffu, bound);
       if (!bm) continue;
       int slot = 0;
@@ -721,81 +904,37 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
       if (bound && slot < INCAP) s_in[slot] = (e << 4) | m;
       const bool over = bound && slot >= INCAP;
       if (__any_sync(0xffffffffu, over)) {
-        PRec r = {0, 0, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (over) r = load_particle(Oin.p, ob + e);
-        process(over, -2, true, r.ix, r.iy, r.x, r.y, r.ux, r.uy, r.uz);
+        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 r = make_float2(0.5f, 0.5f);
+        if (over) u = Oin.p.u[ob + e], r = Oin.p.xy[ob + e];
+        process(over, -1, true, (unsigned)__float_as_int(u.w), r.x, r.y, u.x, u.y, u.z);
+        if (qcount >= 32) finish();
       }
     }
   }
   __syncthreads();
 
-  // own slots: warp w takes chunks w, w + NW, ... of kChunk slots, 32 at a
-  // time (a unit); its next unit is copied into shared memory while it is
-  // pushed.  In a full chunk lane l of the float builds takes slot 32 k + l
-  // at step k, which holds the chunk's particle l kLaneRun + k in cell
-  // order; the deterministic builds take the particle 32 k + l of the cell
-  // order, at its tile_slot.  Every particle goes back to the slot it came
-  // from.
-  {
-    // read and write slots of this lane in unit u; false: no slot
-    const auto slots = [&](int u, int &rs, int &ws) -> bool {
-      const int c0 = (warp + NW * (u / kLaneRun)) * kChunk;
-      const int k = u % kLaneRun;
-      const int i = c0 + k * 32 + lane;
-      if constexpr (DET) {
-        if (c0 + kChunk <= n_own) {
-          const int j = k * 32 + lane;
-          rs = ws = c0 + (j % kLaneRun) * 32 + j / kLaneRun;
-          return true;
-        }
-      }
-      rs = ws = i;
-      return i < n_own;
-    };
-    const auto ubase = [&](int u) { return (warp + NW * (u / kLaneRun)) * kChunk + (u % kLaneRun) * 32; };
-    {
-      int rs, ws;
-      if (ubase(0) < n_own && slots(0, rs, ws)) {
-        cp_async16(&pf_u[warp][lane], &pin.u[base + rs]);
-        cp_async8(&pf_xy[warp][lane], &pin.xy[base + rs]);
-      } else {
-        // a lane without a first particle reads these zeros
-        pf_u[warp][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-        pf_xy[warp][lane] = make_float2(0.f, 0.f);
-      }
+  // own slots, 32 at a time (a unit), the next unit loaded into registers
+  // while one is pushed (staging it in shared memory costs as many
+  // shared-memory passes as half the field gather).  In a full chunk lane l
+  // of the float builds takes slot 32 k + l at step k, which holds the
+  // chunk's particle l kLaneRun + k in cell order; the deterministic builds
+  // take the particle 32 k + l of the cell order, at its tile_slot.  Every
+  // particle goes back to the slot it came from.
+  for (int c = c_begin; c < c_end;) {
+    const float4 uu = nu;
+    const unsigned cw = (unsigned)__float_as_int(uu.w);
+    const int s = ns;
+    const bool inr = s < n_own, valid = inr && cw != kHole;
+    const float x = valid ? nxy.x : 0.5f, y = valid ? nxy.y : 0.5f;
+    c += 32;
+    ns = slot_of(c);
+    if (c < c_end && ns < n_own) {
+      nu = __ldcs(&pin.u[base + ns]);
+      nxy = __ldcs(&pin.xy[base + ns]);
     }
-    cp_async_commit();
-    for (int u = 0; ubase(u) < n_own; ++u) {
-      cp_async_wait<0>();  // this unit's copies (each lane its own slot) are in
-      int rs, ws;
-      const bool inr = slots(u, rs, ws);
-      // a lane without a particle carries whatever its prefetch slot holds
-      // (the last unit's particle, a hole's zero momenta, or the zeros the
-      // slots start with): finite values whose results `valid` masks; its
-      // position is set to the cell centre (a hole's is stale)
-      const float4 uu = pf_u[warp][lane];
-      const float2 xy = pf_xy[warp][lane];
-      const unsigned cw = (unsigned)__float_as_int(uu.w);
-      const bool valid = inr && cw != kHole;
-      PRec r;
-      r.ix = (int)(cw & 0xffffu);
-      r.iy = (int)(cw >> 16);
-      r.x = valid ? xy.x : 0.5f;
-      r.y = valid ? xy.y : 0.5f;
-      r.ux = uu.x;
-      r.uy = uu.y;
-      r.uz = uu.z;
-      {
-        int rn, wn;
-        if (ubase(u + 1) < n_own && slots(u + 1, rn, wn)) {
-          cp_async16(&pf_u[warp][lane], &pin.u[base + rn]);
-          cp_async8(&pf_xy[warp][lane], &pin.xy[base + rn]);
-        }
-      }
-      cp_async_commit();
-      process(valid, inr ? ws : -2, false, r.ix, r.iy, r.x, r.y, r.ux, r.uy, r.uz);
-    }
-    cp_async_wait<0>();
+    process(valid, inr ? s : -1, false, cw, x, y, uu.x, uu.y, uu.z);
+    if (qcount >= 32) finish();
   }
 
   // the listed incoming particles, in units of 32 spread over the warps
@@ -804,18 +943,22 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
     for (int i = warp; i * 32 < nin; i += NW) {
       const int k = i * 32 + lane;
       const bool valid = k < nin;
-      PRec r = {0, 0, 0.f, 0.f, 0.f, 0.f, 0.f};
+      float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+      float2 r = make_float2(0.5f, 0.5f);
       if (valid) {
         const int v = s_in[k];
-        r = load_particle(Oin.p, (long long)nb[v & 15] * Oin.cap + (v >> 4));
+        const long long q = (long long)nb[v & 15] * Oin.cap + (v >> 4);
+        u = Oin.p.u[q];
+        r = Oin.p.xy[q];
       }
-      process(valid, -2, true, r.ix, r.iy, r.x, r.y, r.ux, r.uy, r.uz);
+      process(valid, -1, true, (unsigned)__float_as_int(u.w), r.x, r.y, u.x, u.y, u.z);
+      if (qcount >= 32) finish();
     }
   }
 
-  if (lane < qcount) deposit_queued(lane);  // what is left in the queue
-  if constexpr (!DET)
-    if (acc_key >= 0) add_current(dep, acc_key % TX, acc_key / TX, acc);  // the lanes' last sums
+  finish();  // what is left in the queue
+  if constexpr (!DET)  // the lanes' last sums
+    if (acc_cell != kHole) add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
 
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -888,11 +1031,13 @@ __global__ void __launch_bounds__(NT) k_push_spill(const float *EB, float *J, Fi
       ix = min(max(ix, 0), C.nx - 1);
       iy = min(max(iy, 0), C.ny - 1);
     }
-    float mx, my, x1, y1, qvz;
-    int di, dj;
-    bool bad;
-    const float kin = push_particle(fld, ix, iy, x, y, ux, uy, uz, mx, my, x1, y1, di, dj, qvz, bad, C);
-    if (bad) errbits |= ERR_ESCAPE;
+    float mx, my, qvz;
+    const float kin = push_particle(fld, ix, iy, x, y, ux, uy, uz, mx, my, qvz, C);
+    if (!(fabsf(mx) < 1.0f && fabsf(my) < 1.0f)) errbits |= ERR_ESCAPE;
+    float x1 = x + mx, y1 = y + my;
+    const int di = (x1 >= 1.0f) - (x1 < 0.0f), dj = (y1 >= 1.0f) - (y1 < 0.0f);
+    x1 -= di;
+    y1 -= dj;
     if constexpr (DET) {
       long long h, l;
       efix_split(kin, h, l);
