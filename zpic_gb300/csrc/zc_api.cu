@@ -119,6 +119,7 @@ struct SpeciesState {
   int max_cap = 0;             // largest tile capacity
   int sort_stage = 0;          // particles a tile's sort stages in shared memory
   int spill_cur = 0;
+  bool spill_clean = false;    // the next push's spill count is zero already
   // outboxes: leavers posted by one push, pulled by the next (ob[ob_in]
   // holds the pending ones; its counts are all zero when nothing is pending)
   Outbox ob[2] = {};
@@ -126,7 +127,8 @@ struct SpeciesState {
   int ob_in = 0;
   bool pending = false;
   // energy
-  double *d_ekin_tile = nullptr, *d_ekin_extra = nullptr, *d_ekin = nullptr;
+  double *d_ekin_tile = nullptr, *d_ekin = nullptr;   // partials (tile parts, spill blocks); their sum
+  unsigned long long *d_ekin_fix = nullptr;           // deterministic mode: the spill push's two words
   // window injection drawn on the device (zc_set_device_injection)
   int dinj = 0;
   zc_column_profile dprof{};
@@ -136,7 +138,7 @@ struct SpeciesState {
 struct Counters {
   int iter = 0, n_move = 0;
   std::vector<int> sp_iter, sp_n_move, cur, spill_cur, ob_in;
-  std::vector<bool> pending;
+  std::vector<bool> pending, spill_clean;
   int eb_cur = 0, j_cur = 0;
   bool j0_zero = false;
   long long launch[ZC_NPHASE] = {};
@@ -235,7 +237,6 @@ struct zc_sim {
   bool hist_host = false;         // d_hist is the device address of the caller's host rows
   int *d_hist_n = nullptr;
   int hist_cap = 0, hist_cols = 0, hist_blocks = 0;
-  double **d_ekin_ptrs = nullptr;
   KinSum *d_kin_sums = nullptr;   // with a history: the kinetic sums its row kernel makes
   double *d_hist_part = nullptr;
 };
@@ -620,16 +621,59 @@ zc_status set_current_scale(zc_sim *s, const SpeciesState &p, PushConst &C) {
 zc_status inject_column_device(zc_sim *s, SpeciesState &p);
 int column_lattice(const zc_sim *s, const SpeciesState &p, int n_move, ColumnInject &C, unsigned long long &mask);
 
-// kin_later: the step's history row kernel makes the kinetic sum
-zc_status spec_advance_impl(zc_sim *s, int k, bool kin_later = false) {
-  SpeciesState &p = s->sp[k];
+// The parts every tile is split into when all species are pushed in one
+// launch (push_all), or 0 for one launch a species.  A grid of few tiles does
+// not fill the GPU with one CTA a tile, and its step is bound by its chain of
+// launches.  So species go together when their tiles fit the GPU in one round
+// (kTogetherCtas: 4 CTAs of that kernel a multiprocessor), and tiles are split
+// while the parts still do and leave every warp a unit of 32 slots.  Measured
+// (128^2 cells, two species of 16 a cell, 16x16 tiles): 137 us a step with a
+// push of 64 CTAs a species, a spill launch and a kinetic sum each, 36 with
+// one push launch of 512 CTAs; later in the run, with filaments (tiles of
+// several times the mean), 200 and 65.  Twice the CTAs (two rounds): 43.
+// Runs of a batch share the GPU with the others: together, not split.
+constexpr int kTogetherCtas = 608;
+int push_parts(const zc_sim *s) {
+  const int nsp = (int)s->sp.size();
+  const long long ctas = (long long)nsp * s->ntiles;
+  if (nsp < 1 || nsp > kMaxTogether || ctas > kTogetherCtas) return 0;
+  if (s->batches > 0) return 1;
+  int units = 0;
+  for (const auto &p : s->sp) units = std::max(units, p.ppc[0] * p.ppc[1] * s->TX * s->TY / 32);
+  int parts = 1;
+  while (parts < kMaxParts && 2 * parts * ctas <= kTogetherCtas && 2 * parts * kPushWarps <= units) parts *= 2;
+  return parts;
+}
+
+int spill_blocks(const zc_sim *s) {
+  // (normally empty: a grid sized to the run, so that the many small runs
+  // of a batch do not launch a full grid each for nothing)
+  return std::max(1, std::min(kSpillBlocks, s->ntiles / 4));
+}
+
+// the species' kinetic sum after a push of `parts` parts a tile (0: a launch
+// of its own)
+KinSum kin_sum(const zc_sim *s, const SpeciesState &p, int parts) {
+  const int tiles = s->ntiles * std::max(parts, 1);
+  KinSum K;
+  K.part = p.d_ekin_tile;
+  K.fix = s->deterministic ? p.d_ekin_fix : nullptr;
+  K.out = p.d_ekin;
+  K.n = tiles + (s->deterministic ? 0 : (parts ? kSpillParts : spill_blocks(s)));
+  K.q_mq = p.q * p.m_q;
+  return K;
+}
+
+// The push of species p from its current buffers: cell sort when it is due,
+// the arguments of the launch; *shift: whether its window moves.
+zc_status species_push(zc_sim *s, SpeciesState &p, int parts, PushSpecies &a, int *shift) {
   cudaStream_t st = s->st;
   // moving window: decided after the push, on the species' own counters
   // (spec_move_window, particles.c:621)
-  int shift = 0;
+  *shift = 0;
   if (s->mw) {
     const int it = p.iter + 1;
-    shift = ((it * s->dt) > (s->dx[0] * (p.n_move + 1))) ? 1 : 0;
+    *shift = ((it * s->dt) > (s->dx[0] * (p.n_move + 1))) ? 1 : 0;
   }
   PushConst C;
   C.tem = (float)(0.5 * s->dt / p.m_q);
@@ -642,69 +686,122 @@ zc_status spec_advance_impl(zc_sim *s, int k, bool kin_later = false) {
   C.ny = s->ny;
   C.ntx = s->ntx;
   C.nty = s->nty;
-  C.shift = shift;
+  C.shift = *shift;
   C.mw = s->mw;
   TRY(set_current_scale(s, p, C));
-  const int in = p.spill_cur, out = 1 - p.spill_cur;
-  {
+  const int out = 1 - p.spill_cur;
+  if (!p.spill_clean || s->deterministic) {
     Phase ph(s, ZC_PHASE_SPILL, 0);
-    CK(cudaMemsetAsync(p.d_spill_cnt + out, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(p.d_ekin_extra, 0, 2 * sizeof(double), st));
+    if (!p.spill_clean) CK(cudaMemsetAsync(p.d_spill_cnt + out, 0, sizeof(int), st));
+    if (s->deterministic) CK(cudaMemsetAsync(p.d_ekin_fix, 0, 2 * sizeof(*p.d_ekin_fix), st));
   }
-  PushLaunch a;
-  a.tm_eb = s->EBp ? &s->tmK_EBp : &s->tmK_EB[s->eb_cur];
-  a.pin = p.buf[p.cur];
-  a.pout = p.buf[1 - p.cur];
-  a.T = tiles(p, s->ntiles);
-  a.Oin = p.ob[p.ob_in];
-  a.O = p.ob[1 - p.ob_in];
-  a.S = spill_of(p, out);
-  a.ekin_tile = p.d_ekin_tile;
-  a.err = s->d_err;
-  a.C = C;
-  a.ntiles = s->ntiles;
-  a.TX = s->TX;
-  a.TY = s->TY;
-  a.fast = s->fast;
-  a.det = s->deterministic;
-  a.fj = fixed_j(s);
+  p.spill_clean = false;
   if (s->sort_every > 0 && p.iter % s->sort_every == 0) {
     // keep the tiles sorted by cell (the push warps then share cells)
     Phase ph(s, ZC_PHASE_SORT, 1);
     CK(launch_cellsort(p.buf[p.cur], p.buf[1 - p.cur], p.d_off, p.d_np, layout(s), s->ntiles,
                        s->batches > 0 ? 0 : p.sort_stage, s->d_err, st));
     p.cur = 1 - p.cur;
-    a.pin = p.buf[p.cur];
-    a.pout = p.buf[1 - p.cur];
   }
+  a.pin = p.buf[p.cur];
+  a.pout = p.buf[1 - p.cur];
+  a.T = tiles(p, s->ntiles);
+  a.Oin = p.ob[p.ob_in];
+  a.O = p.ob[1 - p.ob_in];
+  a.Sin = spill_of(p, p.spill_cur);
+  a.S = spill_of(p, out);
+  a.ekin = p.d_ekin_tile;
+  a.ekin_spill = p.d_ekin_tile + (size_t)s->ntiles * std::max(parts, 1);
+  a.ekin_fix = p.d_ekin_fix;
+  a.C = C;
+  return ZC_OK;
+}
+
+PushLaunch push_launch(const zc_sim *s) {
+  PushLaunch a;
+  a.tm_eb = s->EBp ? &s->tmK_EBp : &s->tmK_EB[s->eb_cur];
+  a.one = nullptr;
+  a.all = nullptr;
+  a.EB = s->EBp ? s->EBp : s->EB[s->eb_cur];
+  a.G = s->G;
+  a.err = s->d_err;
+  a.ntiles = s->ntiles;
+  a.TX = s->TX;
+  a.TY = s->TY;
+  a.fast = s->fast;
+  a.det = s->deterministic;
+  a.fj = fixed_j(s);
+  return a;
+}
+
+zc_status species_pushed(zc_sim *s, int k, int shift);
+
+// deterministic mode: the float J that the rest of the step reads, from the
+// fixed-point sums
+zc_status fixed_current(zc_sim *s) {
+  if (!s->deterministic) return ZC_OK;
+  Phase ph(s, ZC_PHASE_ZERO, 1);
+  CK(launch_fixed_to_float(s->Jfix, s->J[0], 3 * s->G.plane, s->st));
+  return ZC_OK;
+}
+
+// the species' kinetic energies, after a push of `parts` parts a tile
+zc_status kin_energies(zc_sim *s, size_t k0, size_t n, int parts) {
+  Phase ph(s, ZC_PHASE_KIN_ENERGY, (int)((n + kMaxTogether - 1) / kMaxTogether));
+  for (size_t k = k0; k < k0 + n; k += kMaxTogether) {
+    const int m = (int)std::min<size_t>(kMaxTogether, k0 + n - k);
+    KinSums K{};
+    for (int i = 0; i < m; ++i) K.k[i] = kin_sum(s, s->sp[k + i], parts);
+    CK(launch_kin_sums(K, m, s->dx[0], s->dx[1], s->st));
+  }
+  return ZC_OK;
+}
+
+// one species by itself
+zc_status spec_advance_impl(zc_sim *s, int k) {
+  SpeciesState &p = s->sp[k];
+  PushSpecies sp;
+  int shift = 0;
+  TRY(species_push(s, p, 0, sp, &shift));
+  PushLaunch a = push_launch(s);
+  a.one = &sp;
   {
     Phase ph(s, ZC_PHASE_PUSH, 1);
-    CK(launch_push_tiles(a, st));
+    CK(launch_push_tiles(a, s->st));
   }
-  const float *EBpart = s->EBp ? s->EBp : s->EB[s->eb_cur];
   {
     Phase ph(s, ZC_PHASE_SPILL, 1);
-    // (normally empty: a grid sized to the run, so that the many small runs
-    // of a batch do not launch a full grid each for nothing)
-    const int spill_blocks = std::max(1, std::min(152, s->ntiles / 4));
-    CK(launch_push_spill(EBpart, s->J[0], fixed_j(s), s->G, p.spill[in], p.d_spill_cnt + in, p.spill_cap,
-                         spill_of(p, out), p.d_ekin_extra, s->d_err, C, spill_blocks, s->fast, s->deterministic,
-                         st));
+    CK(launch_push_spill(a, spill_blocks(s), s->st));
   }
-  if (s->deterministic) {
-    // the float J the rest of the step reads: the fixed-point sum so far
-    Phase ph(s, ZC_PHASE_ZERO, 1);
-    CK(launch_fixed_to_float(s->Jfix, s->J[0], 3 * s->G.plane, st));
+  return species_pushed(s, k, shift);
+}
+
+// every species in one launch, each tile in `parts` parts
+zc_status push_all(zc_sim *s, int parts) {
+  PushAll all;
+  all.nsp = (int)s->sp.size();
+  all.ntiles = s->ntiles;
+  all.parts = parts;
+  int shift[kMaxTogether];
+  for (int k = 0; k < all.nsp; ++k) TRY(species_push(s, s->sp[k], parts, all.sp[k], &shift[k]));
+  PushLaunch a = push_launch(s);
+  a.all = &all;
+  {
+    Phase ph(s, ZC_PHASE_PUSH, all.nsp);  // (the profile counts species' pushes)
+    CK(launch_push_tiles(a, s->st));
   }
+  for (int k = 0; k < all.nsp; ++k) TRY(species_pushed(s, k, shift[k]));
+  return ZC_OK;
+}
+
+// the host side of a push, and the column a window move uncovers
+zc_status species_pushed(zc_sim *s, int k, int shift) {
+  SpeciesState &p = s->sp[k];
+  cudaStream_t st = s->st;
   p.ob_in = 1 - p.ob_in;
   p.pending = true;
   p.cur = 1 - p.cur;
-  p.spill_cur = out;
-  if (!kin_later) {
-    Phase ph(s, ZC_PHASE_KIN_ENERGY, 1);
-    CK(launch_sum_energy(p.d_ekin_tile, s->ntiles, p.d_ekin_extra, p.d_ekin, p.q * p.m_q, s->dx[0], s->dx[1],
-                         s->deterministic, st));
-  }
+  p.spill_cur = 1 - p.spill_cur;
   p.iter += 1;
   if (shift && p.dinj) {
     p.n_move += 1;
@@ -860,9 +957,16 @@ zc_status emf_advance_impl(zc_sim *s, double *epart = nullptr) {
   // them, and clears the raw deposit buffer once the filter has read it
   const bool gc = s->nx >= 3 && s->ny >= 3;
   float *jz = (s->j_cur == 1) ? s->J[0] : nullptr;
+  // ... and the spill counts that the next pushes start from
+  ZeroWords zero{};
+  if ((int)s->sp.size() <= kMaxTogether)
+    for (auto &p : s->sp) {
+      zero.p[zero.n++] = p.d_spill_cnt + (1 - p.spill_cur);
+      p.spill_clean = true;
+    }
   {
     Phase ph(s, ZC_PHASE_YEE, 1);
-    CK(launch_yee(&s->tmY_EB[s->eb_cur], &s->tmY_J[s->j_cur], s->EB[o], s->G, Y, s->d_err, epart, jz, gc, st));
+    CK(launch_yee(&s->tmY_EB[s->eb_cur], &s->tmY_J[s->j_cur], s->EB[o], s->G, Y, s->d_err, epart, jz, gc, zero, st));
   }
   if (jz) s->j0_zero = true;
   s->eb_cur = o;
@@ -894,13 +998,20 @@ zc_status current_zero_impl(zc_sim *s, bool in_step = false) {
   return ZC_OK;
 }
 
-zc_status iter_impl(zc_sim *s) {
+// last: the call's last step.  Only its kinetic energies can be asked for
+// (with a history every step's go into a row), so only it sums them.
+zc_status iter_impl(zc_sim *s, bool last) {
   TRY(current_zero_impl(s, true));
   // with a history, its row kernel makes the kinetic sums, and the Yee
   // kernel sums the new fields' energy (not under a moving window: the
   // window shift follows it)
   const bool hist = s->d_hist != nullptr;
-  for (size_t k = 0; k < s->sp.size(); ++k) TRY(spec_advance_impl(s, (int)k, hist));
+  const int parts = push_parts(s);
+  if (parts) TRY(push_all(s, parts));
+  else
+    for (size_t k = 0; k < s->sp.size(); ++k) TRY(spec_advance_impl(s, (int)k));
+  if (!s->sp.empty()) TRY(fixed_current(s));
+  if (last && !hist && !s->sp.empty()) TRY(kin_energies(s, 0, s->sp.size(), parts));
   TRY(current_update_impl(s));
   const bool fused = hist && !s->mw;
   TRY(emf_advance_impl(s, fused ? s->d_hist_part : nullptr));
@@ -908,7 +1019,7 @@ zc_status iter_impl(zc_sim *s) {
     Phase ph(s, ZC_PHASE_HISTORY, fused ? 1 : 2);
     CK(launch_energy_history(fused ? nullptr : s->EB[s->eb_cur], s->G, s->d_hist_part,
                              fused ? yee_blocks(s->G) : s->hist_blocks, s->d_hist, s->d_hist_n, s->hist_cap,
-                             s->hist_cols, s->d_ekin_ptrs, s->d_kin_sums, (int)s->sp.size(), s->dx[0], s->dx[1],
+                             s->hist_cols, s->d_kin_sums, (int)s->sp.size(), s->dx[0], s->dx[1],
                              s->st));
   }
   return ZC_OK;
@@ -952,6 +1063,7 @@ Counters save_counters(const zc_sim *s) {
     c.spill_cur.push_back(p.spill_cur);
     c.ob_in.push_back(p.ob_in);
     c.pending.push_back(p.pending);
+    c.spill_clean.push_back(p.spill_clean);
   }
   c.eb_cur = s->eb_cur;
   c.j_cur = s->j_cur;
@@ -963,7 +1075,7 @@ Counters save_counters(const zc_sim *s) {
 // the buffer parities a captured graph starts from
 bool same_parities(const Counters &a, const Counters &b) {
   return a.cur == b.cur && a.spill_cur == b.spill_cur && a.ob_in == b.ob_in && a.eb_cur == b.eb_cur &&
-         a.j0_zero == b.j0_zero && (a.iter % 2) == (b.iter % 2);
+         a.spill_clean == b.spill_clean && a.j0_zero == b.j0_zero && (a.iter % 2) == (b.iter % 2);
 }
 
 // the graph g holds n steps from the current state (block-aligned)
@@ -989,7 +1101,7 @@ zc_status capture_steps(zc_sim *s, int n, StepGraph &G, bool instantiate = true)
   if (timed) s->cap_ev = &evs;
   CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
   zc_status st = ZC_OK;
-  for (int k = 0; k < n && st == ZC_OK; ++k) st = iter_impl(s);
+  for (int k = 0; k < n && st == ZC_OK; ++k) st = iter_impl(s, k == n - 1);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(s->st, &g);
   s->cap_ev = nullptr;
@@ -1012,6 +1124,7 @@ zc_status capture_steps(zc_sim *s, int n, StepGraph &G, bool instantiate = true)
     p.spill_cur = before.spill_cur[k];
     p.ob_in = before.ob_in[k];
     p.pending = before.pending[k];
+    p.spill_clean = before.spill_clean[k];
   }
   s->eb_cur = before.eb_cur;
   s->j_cur = before.j_cur;
@@ -1093,6 +1206,7 @@ void account_steps(zc_sim *s, const StepGraph &g) {
     SpeciesState &p = s->sp[k];
     p.iter += n;
     p.pending = g.after.pending[k];
+    p.spill_clean = g.after.spill_clean[k];
     p.cur = g.after.cur[k];
     p.spill_cur = g.after.spill_cur[k];
     p.ob_in = g.after.ob_in[k];
@@ -1181,7 +1295,7 @@ std::vector<long long> block_signature(const zc_sim *s, int n) {
 zc_status step_graph(zc_sim *s, int *nsteps) {
   const int P = block_period(s);
   while (*nsteps > 0 && s->iter % P != 0) {
-    TRY(iter_impl(s));
+    TRY(iter_impl(s, *nsteps == 1));
     --*nsteps;
   }
   int launched = 0;
@@ -1219,7 +1333,7 @@ zc_status step_graph(zc_sim *s, int *nsteps) {
 zc_status step_graph_mw(zc_sim *s, int *nsteps) {
   const int P = block_period(s);
   while (*nsteps > 0 && s->iter % P != 0) {
-    TRY(iter_impl(s));
+    TRY(iter_impl(s, *nsteps == 1));
     --*nsteps;
   }
   constexpr size_t kMaxBlocks = 64;
@@ -1397,10 +1511,6 @@ zc_status zc_sim_create(const zc_sim_desc *d, zc_sim **out) {
   if (s->deterministic) {
     TRYC(dalloc(&s->Jfix, 3 * G.plane));
     cudaMemsetAsync(s->Jfix, 0, sizeof(unsigned long long) * 3 * G.plane, s->st);
-    if ((s->fast ? prepare_push_tiles_fast_det(TX, TY) : prepare_push_tiles_exact_det(TX, TY)) != cudaSuccess) {
-      st = fail(ZC_ECUDA, "deterministic push kernels: shared-memory limit not set");
-      goto bad;
-    }
   }
   TRYC(dalloc(&s->d_err, 1));
   cudaMemsetAsync(s->d_err, 0, sizeof(int), s->st);
@@ -1460,7 +1570,7 @@ zc_status zc_sim_destroy(zc_sim *s) {
     }
     dfree(p.d_spill_cnt);
     dfree(p.d_ekin_tile);
-    dfree(p.d_ekin_extra);
+    dfree(p.d_ekin_fix);
     dfree(p.d_ekin);
   }
   for (int b = 0; b < 2; ++b) {
@@ -1490,7 +1600,6 @@ zc_status zc_sim_destroy(zc_sim *s) {
   dfree(s->d_hist);
   dfree(s->d_hist_n);
   dfree(s->d_hist_part);
-  dfree(s->d_ekin_ptrs);
   dfree(s->d_kin_sums);
   if (s->st) cudaStreamDestroy(s->st);
   delete s;
@@ -1526,11 +1635,11 @@ zc_status zc_species_create(zc_sim *s, const zc_species_desc *d, const zc_part *
   p.spill_cap = std::max(65536, (int)std::min<long long>((long long)np / 32, 1 << 26));
   TRY(alloc_particles(p.spill[0], p.spill_cap));
   TRY(alloc_particles(p.spill[1], p.spill_cap));
-  TRY(dalloc(&p.d_ekin_tile, nt));
-  TRY(dalloc(&p.d_ekin_extra, 2));  // deterministic mode: two fixed-point words
+  TRY(dalloc(&p.d_ekin_tile, (size_t)nt * kMaxParts + kSpillBlocks));
+  TRY(dalloc(&p.d_ekin_fix, 2));
   TRY(dalloc(&p.d_ekin, 1));
   CK(cudaMemsetAsync(p.d_ekin, 0, sizeof(double), s->st));
-  CK(cudaMemsetAsync(p.d_ekin_extra, 0, 2 * sizeof(double), s->st));
+  CK(cudaMemsetAsync(p.d_ekin_fix, 0, 2 * sizeof(*p.d_ekin_fix), s->st));
   TRY(zc_species_set_particles(s, k, parts, np));
   if (id) *id = k;
   return ZC_OK;
@@ -1837,7 +1946,7 @@ zc_status zc_step(zc_sim *s, int nsteps) {
   CK(cudaEventRecord(s->ev0, s->st));
   if (graph_possible(s)) TRY(s->mw ? step_graph_mw(s, &nsteps) : step_graph(s, &nsteps));
   for (int n = 0; n < nsteps; ++n) {
-    TRY(iter_impl(s));
+    TRY(iter_impl(s, n == nsteps - 1));
     // spill lists are drained into the tiles at least every 16 steps
     if ((n & 15) == 15 && n + 1 < nsteps) {
       CK(cudaMemcpyAsync(s->h_pinned, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
@@ -1859,7 +1968,7 @@ zc_status zc_step_async(zc_sim *s, int nsteps) {
   DeviceGuard g(s->device);
   if (graph_possible(s)) TRY(s->mw ? step_graph_mw(s, &nsteps) : step_graph(s, &nsteps));
   for (int n = 0; n < nsteps; ++n) {
-    TRY(iter_impl(s));
+    TRY(iter_impl(s, n == nsteps - 1));
     // every 16 queued steps: wait, and drain a spill list that has filled
     if (++s->queued_steps >= 16) {
       CK(cudaMemcpyAsync(s->h_pinned, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
@@ -1885,6 +1994,8 @@ zc_status zc_spec_advance(zc_sim *s, int k) {
   DeviceGuard g(s->device);
   CK(cudaEventRecord(s->ev0, s->st));
   TRY(spec_advance_impl(s, k));
+  TRY(fixed_current(s));
+  TRY(kin_energies(s, k, 1, 0));
   CK(cudaEventRecord(s->ev1, s->st));
   CK(cudaEventSynchronize(s->ev1));
   cudaEventElapsedTime(&s->last_ms, s->ev0, s->ev1);
@@ -2204,6 +2315,7 @@ zc_status zc_set_graphs(zc_sim *s, int on) {
   return ZC_OK;
 }
 
+zc_status history_sums(zc_sim *s);
 zc_status history_setup(zc_sim *s, double *rows, int max_steps);
 
 zc_status zc_history_enable(zc_sim *s, int max_steps) { return history_setup(s, nullptr, max_steps); }
@@ -2212,6 +2324,18 @@ zc_status zc_history_stream(zc_sim *s, double *rows, int max_steps) {
   if (!s) return fail(ZC_EINVAL, "null simulation handle");
   if (max_steps > 0 && !rows) return fail(ZC_EINVAL, "null row buffer");
   return history_setup(s, rows, max_steps);
+}
+
+// what the history's row kernel sums for every species (it depends on how
+// the species are pushed)
+zc_status history_sums(zc_sim *s) {
+  std::vector<KinSum> sums;
+  for (auto &p : s->sp) sums.push_back(kin_sum(s, p, push_parts(s)));
+  if (!sums.empty() && s->d_kin_sums) {
+    CK(cudaMemcpyAsync(s->d_kin_sums, sums.data(), sizeof(KinSum) * sums.size(), cudaMemcpyHostToDevice, s->st));
+    CK(cudaStreamSynchronize(s->st));
+  }
+  return ZC_OK;
 }
 
 zc_status history_setup(zc_sim *s, double *rows, int max_steps) {
@@ -2226,7 +2350,6 @@ zc_status history_setup(zc_sim *s, double *rows, int max_steps) {
   dfree(s->d_hist);
   dfree(s->d_hist_n);
   dfree(s->d_hist_part);
-  dfree(s->d_ekin_ptrs);
   dfree(s->d_kin_sums);
   s->hist_cap = 0;
   s->hist_cols = 0;
@@ -2249,18 +2372,8 @@ zc_status history_setup(zc_sim *s, double *rows, int max_steps) {
   TRY(dalloc(&s->d_hist_n, 1));
   // partials of the standalone energy pass or of the Yee kernel
   TRY(dalloc(&s->d_hist_part, 6 * (size_t)std::max(s->hist_blocks, yee_blocks(s->G))));
-  TRY(dalloc(&s->d_ekin_ptrs, std::max<size_t>(1, s->sp.size())));
   TRY(dalloc(&s->d_kin_sums, std::max<size_t>(1, s->sp.size())));
-  std::vector<double *> ptrs;
-  std::vector<KinSum> sums;
-  for (auto &p : s->sp) {
-    ptrs.push_back(p.d_ekin);
-    sums.push_back(KinSum{p.d_ekin_tile, p.d_ekin_extra, s->ntiles, s->deterministic, p.q * p.m_q});
-  }
-  if (!ptrs.empty()) {
-    CK(cudaMemcpyAsync(s->d_ekin_ptrs, ptrs.data(), sizeof(double *) * ptrs.size(), cudaMemcpyHostToDevice, s->st));
-    CK(cudaMemcpyAsync(s->d_kin_sums, sums.data(), sizeof(KinSum) * sums.size(), cudaMemcpyHostToDevice, s->st));
-  }
+  TRY(history_sums(s));
   CK(cudaMemsetAsync(s->d_hist_n, 0, sizeof(int), s->st));
   CK(cudaStreamSynchronize(s->st));
   s->hist_cap = max_steps;
@@ -2525,11 +2638,12 @@ zc_status zc_batch_create(zc_sim *const *sims, int nsims, zc_batch **out) {
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
       return bad(fail(ZC_ECUDA, "cudaEventCreate failed"));
   if ((st = form_groups(b, default_groups(nsims))) != ZC_OK) return bad(st);
-  for (zc_sim *s : b->sims) {
-    s->batches += 1;
-    invalidate_graph(s);  // recorded blocks hold the sort of a run alone
-  }
   b->marked = true;
+  for (zc_sim *s : b->sims) s->batches += 1;
+  for (zc_sim *s : b->sims) {
+    invalidate_graph(s);  // recorded blocks hold the sort and the push of a run alone
+    if ((st = history_sums(s)) != ZC_OK) return bad(st);
+  }
   *out = b;
   return ZC_OK;
 }
@@ -2555,7 +2669,9 @@ zc_status zc_batch_destroy(zc_batch *b) {
   if (b->marked)
     for (zc_sim *s : b->sims) {
       s->batches -= 1;
-      if (s->batches == 0) invalidate_graph(s);  // recorded blocks hold the batch's sort
+      if (s->batches > 0) continue;
+      invalidate_graph(s);  // recorded blocks hold the batch's sort and push
+      history_sums(s);
     }
   dfree(b->d_errp);
   dfree(b->d_errs);
@@ -2594,7 +2710,7 @@ zc_status zc_batch_step(zc_batch *b, int nsteps) {
   for (int k = 0; k < n; ++k) {
     zc_sim *s = b->sims[k];
     lead[k] = std::min(nsteps, (P - s->iter % P) % P);
-    for (int i = 0; i < lead[k]; ++i) TRY(iter_impl(s));
+    for (int i = 0; i < lead[k]; ++i) TRY(iter_impl(s, i == nsteps - 1));
     blocks = std::min(blocks, (nsteps - lead[k]) / P);
     aligned = aligned && lead[k] == 0;
   }
@@ -2649,7 +2765,7 @@ zc_status zc_batch_step(zc_batch *b, int nsteps) {
   for (int k = 0; k < n; ++k) {
     zc_sim *s = b->sims[k];
     const int m = nsteps - lead[k] - blocks * P - rest;
-    for (int i = 0; i < m; ++i) TRY(iter_impl(s));
+    for (int i = 0; i < m; ++i) TRY(iter_impl(s, i == m - 1));
   }
   for (zc_sim *s : b->sims) {
     CK(cudaEventRecord(s->ev1, s->st));

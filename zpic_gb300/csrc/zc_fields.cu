@@ -483,11 +483,13 @@ __device__ __forceinline__ void put_mirrored(float *EB, const Grid &G, int c, in
 #endif
 __global__ void __launch_bounds__(256, ZC_YEE_MINB) k_yee(const __grid_constant__ CUtensorMap tm_eb,
                                              const __grid_constant__ CUtensorMap tm_j, float *EBout, Grid G,
-                                             YeeConst Y, int *err, double *epart, float *jzero, int gc) {
+                                             YeeConst Y, int *err, double *epart, float *jzero, int gc,
+                                             const __grid_constant__ ZeroWords zero) {
   constexpr int BW = kYeeBW, BH = kYeeBH, PL = BW * BH;
   __shared__ __align__(128) float sEB[6 * PL];
   __shared__ __align__(128) float sJ[3 * PL];
   __shared__ __align__(8) uint64_t bar;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < zero.n) *zero.p[threadIdx.x] = 0;
   const int bx0 = blockIdx.x * kYeeOX, by0 = blockIdx.y * kYeeOY;
   const int ox = bx0 - 4, oy = by0 - 1;  // buffer coords of smem (0,0)
   if (threadIdx.x == 0) {
@@ -870,10 +872,11 @@ cudaError_t launch_smooth(const float *Jin, float *Jout, const Grid &G, const Sm
 int yee_blocks(const Grid &G) { return ((G.nx + 3 + kYeeOX - 1) / kYeeOX) * ((G.ny + 3 + kYeeOY - 1) / kYeeOY); }
 
 cudaError_t launch_yee(const CUtensorMap *tm_eb, const CUtensorMap *tm_j, float *EBout, const Grid &G,
-                       const YeeConst &Y, int *err, double *epart, float *jzero, bool gc, cudaStream_t st) {
+                       const YeeConst &Y, int *err, double *epart, float *jzero, bool gc, const ZeroWords &zero,
+                       cudaStream_t st) {
   if (gc && (G.nx < 3 || G.ny < 3)) return cudaErrorInvalidValue;  // mirrors would overlap
   dim3 grid((G.nx + 3 + kYeeOX - 1) / kYeeOX, (G.ny + 3 + kYeeOY - 1) / kYeeOY);
-  k_yee<<<grid, 256, 0, st>>>(*tm_eb, *tm_j, EBout, G, Y, err, epart, jzero, gc ? 1 : 0);
+  k_yee<<<grid, 256, 0, st>>>(*tm_eb, *tm_j, EBout, G, Y, err, epart, jzero, gc ? 1 : 0, zero);
   return cudaGetLastError();
 }
 
@@ -919,27 +922,20 @@ __global__ void k_energy_direct(const double *partial, int nblocks, float dx, fl
 // k_emf_energy_final) and the kinetic energy of every species; the row index
 // is a device counter, so a captured step appends where it runs
 __global__ void __launch_bounds__(256) k_energy_history_row(const double *partial, int nblocks, float dx, float dy,
-                                                            double *const *ekin, const KinSum *ks, int nsp,
-                                                            double *hist, int *hist_n, int cap, int cols) {
+                                                            const KinSum *ks, int nsp, double *hist, int *hist_n,
+                                                            int cap, int cols) {
   __shared__ double sred[8];
   const int t = threadIdx.x, c = t >> 5, lane = t & 31;
-  if (ks) {
-    // each species' kinetic energy from its tile partials, by the whole
-    // block (as k_sum_energy would leave it in *ekin), before the row
-    for (int k = 0; k < nsp; ++k) {
-      const KinSum &K = ks[k];
-      double s = 0;
-      for (int i = t; i < K.ntiles; i += 256) s += K.tiles[i];
-      s = block_sum_double<256>(s, sred);
-      if (t == 0) {
-        if (K.det) {
-          const long long *w = reinterpret_cast<const long long *>(K.extra);
-          s += efix_join(w[0], w[1]);
-        } else {
-          s += *K.extra;
-        }
-        *ekin[k] = K.q_mq * s * dx * dy;  // spec->energy (particles.c:1231)
-      }
+  // each species' kinetic energy from its partials, by the whole block (as
+  // k_kin_sums makes it), before the row
+  for (int k = 0; k < nsp; ++k) {
+    const KinSum &K = ks[k];
+    double s = 0;
+    for (int i = t; i < K.n; i += 256) s += K.part[i];
+    s = block_sum_double<256>(s, sred);
+    if (t == 0) {
+      if (K.fix) s += efix_join((long long)K.fix[0], (long long)K.fix[1]);
+      *K.out = K.q_mq * s * dx * dy;  // spec->energy (particles.c:1231)
     }
   }
   __syncthreads();
@@ -951,7 +947,7 @@ __global__ void __launch_bounds__(256) k_energy_history_row(const double *partia
     const double s = partial_sum(partial, nblocks, c);
     if (lane == 0) row[c] = s * (0.5 * dx * dy);
   } else if (t - 6 * 32 < nsp) {  // then one thread per species
-    row[6 + t - 6 * 32] = *ekin[t - 6 * 32];
+    row[6 + t - 6 * 32] = *ks[t - 6 * 32].out;
   }
   __syncthreads();
   if (t == 0) *hist_n = n + 1;
@@ -966,11 +962,11 @@ cudaError_t launch_energy_direct(const float *EB, const Grid &G, double *partial
 }
 
 cudaError_t launch_energy_history(const float *EB, const Grid &G, double *partial, int nblocks, double *hist,
-                                  int *hist_n, int cap, int cols, double *const *ekin, const KinSum *ks, int nsp,
-                                  float dx, float dy, cudaStream_t st) {
+                                  int *hist_n, int cap, int cols, const KinSum *ks, int nsp, float dx, float dy,
+                                  cudaStream_t st) {
   if (nsp > 64) return cudaErrorInvalidValue;
   if (EB) k_emf_energy_partial<<<nblocks, 256, 0, st>>>(EB, G, partial);  // (no EB: partials already made)
-  k_energy_history_row<<<1, 256, 0, st>>>(partial, nblocks, dx, dy, ekin, ks, nsp, hist, hist_n, cap, cols);
+  k_energy_history_row<<<1, 256, 0, st>>>(partial, nblocks, dx, dy, ks, nsp, hist, hist_n, cap, cols);
   return cudaGetLastError();
 }
 

@@ -218,6 +218,20 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// thread-block cluster: barrier in two halves, and an addition to an int of
+// rank 0's shared memory (the variable is at the same place in every CTA)
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ int rank0_add(int *v, int n) {
+  uint32_t a;
+  int old;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(v)));
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(n) : "memory");
+  return old;
+}
+
 // contiguous bulk copy global -> shared, completing on an mbarrier (both
 // addresses 16-byte aligned, bytes a multiple of 16)
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {

@@ -75,15 +75,34 @@ __host__ __device__ __forceinline__ double efix_join(long long hi, long long lo)
   return (double)hi / kEFixHi + (double)lo / kEFixLo;
 }
 
-struct PushLaunch {
-  const CUtensorMap *tm_eb;
+// one species' push
+struct PushSpecies {
   Particles pin, pout;
   TileSet T;
   Outbox Oin, O;                          // pending incoming (previous step), leavers (this step)
-  Spill S;
-  double *ekin_tile;
-  int *err;
+  Spill Sin, S;                           // spilled particles: to push, and those of this step
+  double *ekin;                           // kinetic energy of every tile part
+  double *ekin_spill;                     // and of every block of the spill push
+  unsigned long long *ekin_fix;           // deterministic mode: the spill push's fixed-point words
   PushConst C;
+};
+
+// all species of a small grid in one launch: tiles by clusters of `parts`
+// CTAs, then kSpillParts blocks for the spilled particles of each species
+constexpr int kMaxTogether = 8, kMaxParts = 8, kSpillParts = 8;
+constexpr int kPushWarps = 4;             // warps of a push CTA (float builds)
+struct PushAll {
+  int nsp, ntiles, parts;
+  PushSpecies sp[kMaxTogether];
+};
+
+struct PushLaunch {
+  const CUtensorMap *tm_eb;
+  const PushSpecies *one;                 // one species (or null),
+  const PushAll *all;                     // or all of them
+  const float *EB;                        // the fields the particles see (spill push)
+  Grid G;
+  int *err;
   int ntiles, TX, TY;
   int fast;                               // 1: FMA build of the push kernels
   int det;                                // 1: fixed-point currents into fj
@@ -125,23 +144,13 @@ cudaError_t launch_push_tiles_exact(const PushLaunch &a, cudaStream_t st);
 cudaError_t launch_push_tiles_fast(const PushLaunch &a, cudaStream_t st);
 cudaError_t launch_push_tiles_exact_det(const PushLaunch &a, cudaStream_t st);
 cudaError_t launch_push_tiles_fast_det(const PushLaunch &a, cudaStream_t st);
-// sets the shared-memory limit of the deterministic push kernels of one
-// tile shape on the current device (outside any stream capture)
-cudaError_t prepare_push_tiles_exact_det(int TX, int TY);
-cudaError_t prepare_push_tiles_fast_det(int TX, int TY);
-// spill push; with det, currents go to fj and the kinetic energy to ekin[0..1]
-// read as the two 64-bit fixed-point words of efix_join
-cudaError_t launch_push_spill(const float *EB, float *J, const FixedJ &fj, const Grid &G, const Particles &sin,
-                              const int *sin_cnt, int sin_cap, const Spill &S, double *ekin, int *err,
-                              const PushConst &C, int nblocks, int fast, int det, cudaStream_t st);
-#define ZC_SPILL_LAUNCHER(name)                                                                              \
-  cudaError_t name(const float *EB, float *J, const FixedJ &fj, const Grid &G, const Particles &sin,          \
-                   const int *sin_cnt, int sin_cap, const Spill &S, double *ekin, int *err, const PushConst &C, \
-                   int nblocks, cudaStream_t st)
-ZC_SPILL_LAUNCHER(launch_push_spill_exact);
-ZC_SPILL_LAUNCHER(launch_push_spill_fast);
-ZC_SPILL_LAUNCHER(launch_push_spill_exact_det);
-ZC_SPILL_LAUNCHER(launch_push_spill_fast_det);
+// spill push of a.one, nblocks blocks (at most kSpillBlocks)
+constexpr int kSpillBlocks = 152;
+cudaError_t launch_push_spill(const PushLaunch &a, int nblocks, cudaStream_t st);
+cudaError_t launch_push_spill_exact(const PushLaunch &a, int nblocks, cudaStream_t st);
+cudaError_t launch_push_spill_fast(const PushLaunch &a, int nblocks, cudaStream_t st);
+cudaError_t launch_push_spill_exact_det(const PushLaunch &a, int nblocks, cudaStream_t st);
+cudaError_t launch_push_spill_fast_det(const PushLaunch &a, int nblocks, cudaStream_t st);
 // fixed-point current planes <-> float planes (n values)
 cudaError_t launch_fixed_to_float(const unsigned long long *src, float *dst, size_t n, cudaStream_t st);
 cudaError_t launch_float_to_fixed(const float *src, unsigned long long *dst, size_t n, cudaStream_t st);
@@ -212,10 +221,20 @@ cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *n
 cudaError_t launch_charge(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
                           const int *spill_cnt, int spill_cap, float *rho, int nx, int ny, float q, int mw,
                           cudaStream_t st);
-// with det, extra[0..1] are the two 64-bit fixed-point words of a kinetic
-// energy (efix_join)
-cudaError_t launch_sum_energy(const double *tiles, int ntiles, const double *extra, double *out, float q_mq,
-                              float dx, float dy, int det, cudaStream_t st);
+// the kinetic-energy sum of one species into *out: n partials of tile parts
+// and spill blocks; with fix, the two 64-bit fixed-point words of efix_join
+struct KinSum {
+  const double *part;
+  const unsigned long long *fix;
+  double *out;
+  int n;
+  float q_mq;
+};
+// one block a species
+struct KinSums {
+  KinSum k[kMaxTogether];
+};
+cudaError_t launch_kin_sums(const KinSums &K, int nsp, float dx, float dy, cudaStream_t st);
 
 // fields
 struct YeeConst {
@@ -240,8 +259,14 @@ cudaError_t launch_smooth(const float *Jin, float *Jout, const Grid &G, const Sm
 // doubles a block, yee_blocks(G) blocks.  jzero (or null): a current buffer
 // the kernel clears (3 planes).  gc: the guard cells are written as the
 // guard-cell update leaves them (k_emf_gc then not needed; nx, ny >= 3)
+// zero: words the kernel clears (spill counts)
+struct ZeroWords {
+  int n;
+  int *p[kMaxTogether];
+};
 cudaError_t launch_yee(const CUtensorMap *tm_eb, const CUtensorMap *tm_j, float *EBout, const Grid &G,
-                       const YeeConst &Y, int *err, double *epart, float *jzero, bool gc, cudaStream_t st);
+                       const YeeConst &Y, int *err, double *epart, float *jzero, bool gc, const ZeroWords &zero,
+                       cudaStream_t st);
 int yee_blocks(const Grid &G);
 cudaError_t launch_emf_gc(float *EB, const Grid &G, int mw, cudaStream_t st);
 cudaError_t launch_ext_add(const float *EB, float *EBp, const float *extE, const float *extB, int Etype, int Btype,
@@ -259,20 +284,13 @@ cudaError_t launch_energy_direct(const float *EB, const Grid &G, double *partial
                                  const EkinRefs &K, int nsp, double *emf, double *kin, cudaStream_t st);
 cudaError_t launch_emf_energy(const float *EB, const Grid &G, double *partial, int nblocks, double *out, float dx,
                               float dy, cudaStream_t st);
-// the kinetic-energy sum of one species (what k_sum_energy does)
-struct KinSum {
-  const double *tiles;   // per-tile partials
-  const double *extra;   // spill-list partial (two fixed-point words when det)
-  int ntiles, det;
-  float q_mq;
-};
 // appends one row (6 field-energy components, then each species' kinetic
 // energy) at hist[*hist_n] and increments *hist_n, unless cap rows exist.
-// EB null: the partials are already there (the Yee kernel's).  ks (or null):
-// the kinetic sums are made here first, into *ekin[k]
+// EB null: the partials are already there (the Yee kernel's).  The kinetic
+// sums ks (device memory) are made here first
 cudaError_t launch_energy_history(const float *EB, const Grid &G, double *partial, int nblocks, double *hist,
-                                  int *hist_n, int cap, int cols, double *const *ekin, const KinSum *ks, int nsp,
-                                  float dx, float dy, cudaStream_t st);
+                                  int *hist_n, int cap, int cols, const KinSum *ks, int nsp, float dx, float dy,
+                                  cudaStream_t st);
 // dst[k] = *src[k] for k < n (error words of a batch)
 cudaError_t launch_gather_words(int *const *src, int n, int *dst, cudaStream_t st);
 struct LaserConst {

@@ -710,22 +710,17 @@ __global__ void k_charge_fold(float *rho, int nx, int ny, int mw) {
     for (int i = threadIdx.x; i < nx + 1; i += blockDim.x) rho[i] += rho[i + ny * nrow];
 }
 
-// sum of the per-tile kinetic-energy partials in a fixed order
-__global__ void k_sum_energy(const double *tiles, int ntiles, const double *extra, double *out, float scale_q_mq,
-                             float dx, float dy, int det) {
+// sums of the kinetic-energy partials in a fixed order, one block a species
+__global__ void __launch_bounds__(256) k_kin_sums(const __grid_constant__ KinSums S, float dx, float dy) {
   __shared__ double sred[8];
+  const KinSum &K = S.k[blockIdx.x];
   double s = 0;
-  for (int t = threadIdx.x; t < ntiles; t += 256) s += tiles[t];
+  for (int i = threadIdx.x; i < K.n; i += 256) s += K.part[i];
   s = block_sum_double<256>(s, sred);
   if (threadIdx.x == 0) {
-    if (det) {
-      const long long *w = reinterpret_cast<const long long *>(extra);
-      s += efix_join(w[0], w[1]);
-    } else {
-      s += *extra;
-    }
+    if (K.fix) s += efix_join((long long)K.fix[0], (long long)K.fix[1]);
     // spec->energy = q * m_q * energy * dx * dy  (particles.c:1231)
-    *out = scale_q_mq * s * dx * dy;
+    *K.out = K.q_mq * s * dx * dy;
   }
 }
 
@@ -742,12 +737,9 @@ cudaError_t launch_push_tiles(const PushLaunch &a, cudaStream_t st) {
   return a.fast ? launch_push_tiles_fast(a, st) : launch_push_tiles_exact(a, st);
 }
 
-cudaError_t launch_push_spill(const float *EB, float *J, const FixedJ &fj, const Grid &G, const Particles &sin,
-                              const int *sin_cnt, int sin_cap, const Spill &S, double *ekin, int *err,
-                              const PushConst &C, int nblocks, int fast, int det, cudaStream_t st) {
-  auto f = det ? (fast ? launch_push_spill_fast_det : launch_push_spill_exact_det)
-               : (fast ? launch_push_spill_fast : launch_push_spill_exact);
-  return f(EB, J, fj, G, sin, sin_cnt, sin_cap, S, ekin, err, C, nblocks, st);
+cudaError_t launch_push_spill(const PushLaunch &a, int nblocks, cudaStream_t st) {
+  if (a.det) return a.fast ? launch_push_spill_fast_det(a, nblocks, st) : launch_push_spill_exact_det(a, nblocks, st);
+  return a.fast ? launch_push_spill_fast(a, nblocks, st) : launch_push_spill_exact(a, nblocks, st);
 }
 
 __global__ void k_fixed_to_float(const unsigned long long *src, float *dst, size_t n) {
@@ -897,9 +889,8 @@ cudaError_t launch_charge(const Particles &buf, const int *off, const int *np, i
   return cudaGetLastError();
 }
 
-cudaError_t launch_sum_energy(const double *tiles, int ntiles, const double *extra, double *out, float q_mq,
-                              float dx, float dy, int det, cudaStream_t st) {
-  k_sum_energy<<<1, 256, 0, st>>>(tiles, ntiles, extra, out, q_mq, dx, dy, det);
+cudaError_t launch_kin_sums(const KinSums &K, int nsp, float dx, float dy, cudaStream_t st) {
+  k_kin_sums<<<nsp, 256, 0, st>>>(K, dx, dy);
   return cudaGetLastError();
 }
 

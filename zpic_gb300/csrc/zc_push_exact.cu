@@ -13,8 +13,8 @@ cudaError_t launch_push_tiles_exact(const PushLaunch &a, cudaStream_t st) {
   return exact::launch_push_tiles_variant<false>(a, st);
 }
 
-ZC_SPILL_LAUNCHER(launch_push_spill_exact) {
-  return exact::launch_push_spill_variant<false>(EB, J, fj, G, sin, sin_cnt, sin_cap, S, ekin, err, C, nblocks, st);
+cudaError_t launch_push_spill_exact(const PushLaunch &a, int nblocks, cudaStream_t st) {
+  return exact::launch_push_spill_variant<false>(a, nblocks, st);
 }
 
 }  // namespace zc

@@ -10,15 +10,12 @@ namespace exact_det {
 #include "zc_push_impl.cuh"
 }  // namespace exact_det
 
-cudaError_t prepare_push_tiles_exact_det(int TX, int TY) { return exact_det::prepare_push_variant<true>(TX, TY); }
-
 cudaError_t launch_push_tiles_exact_det(const PushLaunch &a, cudaStream_t st) {
   return exact_det::launch_push_tiles_variant<true>(a, st);
 }
 
-ZC_SPILL_LAUNCHER(launch_push_spill_exact_det) {
-  return exact_det::launch_push_spill_variant<true>(EB, J, fj, G, sin, sin_cnt, sin_cap, S, ekin, err, C, nblocks,
-                                                    st);
+cudaError_t launch_push_spill_exact_det(const PushLaunch &a, int nblocks, cudaStream_t st) {
+  return exact_det::launch_push_spill_variant<true>(a, nblocks, st);
 }
 
 }  // namespace zc

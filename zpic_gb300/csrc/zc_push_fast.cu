@@ -15,8 +15,8 @@ cudaError_t launch_push_tiles_fast(const PushLaunch &a, cudaStream_t st) {
   return fast::launch_push_tiles_variant<false>(a, st);
 }
 
-ZC_SPILL_LAUNCHER(launch_push_spill_fast) {
-  return fast::launch_push_spill_variant<false>(EB, J, fj, G, sin, sin_cnt, sin_cap, S, ekin, err, C, nblocks, st);
+cudaError_t launch_push_spill_fast(const PushLaunch &a, int nblocks, cudaStream_t st) {
+  return fast::launch_push_spill_variant<false>(a, nblocks, st);
 }
 
 }  // namespace zc

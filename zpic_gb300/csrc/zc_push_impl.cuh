@@ -514,11 +514,20 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 #ifndef ZC_PUSH_MIN_CTAS
 #define ZC_PUSH_MIN_CTAS 6
 #endif
-template <int TX, int TY, int NT, bool DET>
-__global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push_tiles(const __grid_constant__ CUtensorMap tm_eb,
-                                                   Particles pin,
-                                                   Particles pout, TileSet T, Outbox Oin, Outbox O, Spill S,
-                                                   double *ekin_tile, int *err, PushConst C, FixedJ fj) {
+//
+// SPLIT: a tile is worked on by a cluster of `parts` CTAs (this one is
+// `rank`), for grids with too few tiles to fill the GPU.  Each stages the
+// tile's fields, pushes its share of the slots and pulls from its share of
+// the neighbours; the counters of leavers and appended arrivals are rank 0's
+// (distributed shared memory).
+template <int TX, int TY, int NT, bool DET, bool SPLIT>
+__device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSpecies &A, int *err, const FixedJ &fj,
+                                          int t, int rank, int parts) {
+  const Particles &pin = A.pin, &pout = A.pout;
+  const TileSet &T = A.T;
+  const Outbox &Oin = A.Oin, &O = A.O;
+  const Spill &S = A.S;
+  const PushConst &C = A.C;
 #ifdef ZC_FAST
   constexpr int BW = push_box_w(TX, true);
 #else
@@ -550,7 +559,6 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   __shared__ int s_nin;
   __shared__ int s_app, s_leave;      // appended arrivals, leavers (warp-aggregated atomics)
 
-  const int t = blockIdx.x;
   const int tx = t % C.ntx, ty = t / C.ntx;
   const int cx0 = tx * TX, cy0 = ty * TY;  // first cell of the tile = buffer coords of its halo
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -559,7 +567,6 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   int qcount = 0;  // warp-uniform
 
   const unsigned base = (unsigned)T.off[t];  // (tile offsets are below 2^31)
-  const int cap = T.cap[t];
   const int n_own = T.np[t];
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -592,10 +599,11 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   // This warp's slots: an equal share of the tile's units of 32 slots, one
   // contiguous run (equal to a unit, so that no warp waits a chunk's time for
   // another at the end).  Its first unit is on its way before the fields are.
+  const int gwarp = SPLIT ? rank * NW + warp : warp, nwarps = SPLIT ? parts * NW : NW;
   const int units = (n_own + 31) / 32;
-  const int share = units / NW, extra = units % NW;
-  const int c_begin = 32 * (warp * share + min(warp, extra));
-  const int c_end = min(n_own, c_begin + 32 * (share + (warp < extra ? 1 : 0)));
+  const int share = units / nwarps, extra = units % nwarps;
+  const int c_begin = 32 * (gwarp * share + min(gwarp, extra));
+  const int c_end = min(n_own, c_begin + 32 * (share + (gwarp < extra ? 1 : 0)));
   // this lane's slot in the unit that starts at slot c
   const auto slot_of = [&](int c) {
     if constexpr (DET) {
@@ -617,18 +625,20 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   if constexpr (DET)
     for (int k = threadIdx.x; k < 3 * LAY::N; k += NT) sJi[k] = 0;
   __syncthreads();
+  if constexpr (SPLIT) cluster_arrive();  // np is read, the counters are zero
   // the outboxes of this warp's neighbours: counts and first entries
   constexpr int NBW = (8 + NW - 1) / NW;
   const int nnb = s_nnb;
   int in_n[NBW], in_dst[NBW];
 #pragma unroll
   for (int q = 0; q < NBW; ++q) {
-    const int m = warp + q * NW;
+    const int m = gwarp + q * nwarps;
     in_n[q] = m < nnb ? Oin.cnt[nb[m]] : 0;
     in_dst[q] = (m < nnb && lane < Oin.cap) ? Oin.dst[(long long)nb[m] * Oin.cap + lane] : -1;
   }
   const bool loaded = mbar_wait_bounded(&bar, 0);
   if (!loaded) errbits |= ERR_TIMEOUT;
+  if constexpr (SPLIT) cluster_wait();
 
 #ifdef ZC_FAST
   // in place: planes Ex Ey Ez Bx By Bz -> Ez, Bz, pairs (Ex, By), (Ey, Bx)
@@ -665,7 +675,6 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
     else
       return TileCurrentGlobal{fj.f + (size_t)(cy0 + 1) * fj.pitch + (cx0 + 1), fj.pitch, fj.plane};
   }();
-  const long long obase = (long long)t * O.cap;
   float ks = 0.f, kc = 0.f;
   long long khi = 0, klo = 0;  // DET: fixed-point kinetic energy of this thread's particles
   // float builds: this lane's running single-segment current and its cell
@@ -727,13 +736,19 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
     if (mleave | mapp) {
       int lb = 0, ab = 0;
       if (lane == 0) {
-        if (mleave) lb = atomicAdd(&s_leave, __popc(mleave));
-        if (mapp) ab = atomicAdd(&s_app, __popc(mapp));
+        if constexpr (SPLIT) {
+          if (mleave) lb = rank0_add(&s_leave, __popc(mleave));
+          if (mapp) ab = rank0_add(&s_app, __popc(mapp));
+        } else {
+          if (mleave) lb = atomicAdd(&s_leave, __popc(mleave));
+          if (mapp) ab = atomicAdd(&s_app, __popc(mapp));
+        }
       }
       lb = __shfl_sync(0xffffffffu, lb, 0);
       ab = __shfl_sync(0xffffffffu, ab, 0);
       if (code == 2) {
         const int s = lb + __popc(mleave & below);
+        const long long obase = (long long)t * O.cap;
         if (s < O.cap) {
           store_particle(O.p, obase + s, ix, iy, x, y, ux, uy, uz);
           O.dst[obase + s] = dest;
@@ -742,7 +757,7 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
         }
       } else if (app) {
         const int s = n_own + ab + __popc(mapp & below);
-        if (s < cap) store_particle(pout, base + s, ix, iy, x, y, ux, uy, uz);
+        if (s < T.cap[t]) store_particle(pout, base + s, ix, iy, x, y, ux, uy, uz);
         else spill_particle(S, &errbits, ix, iy, x, y, ux, uy, uz);
       }
     }
@@ -889,7 +904,7 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   // leaves the rest to be pushed right here
 #pragma unroll
   for (int q = 0; q < NBW; ++q) {
-    const int m = warp + q * NW;
+    const int m = gwarp + q * nwarps;
     if (m >= nnb) break;
     const int n = in_n[q];
     const long long ob = (long long)nb[m] * Oin.cap;
@@ -960,9 +975,14 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
   if constexpr (!DET)  // the lanes' last sums
     if (acc_cell != kHole) add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
 
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    T.np[t] = n_own + min(s_app, cap - n_own);
+  if constexpr (SPLIT) {
+    cluster_arrive();  // every part's leavers and arrivals are counted
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && (!SPLIT || rank == 0)) {
+    T.np[t] = n_own + min(s_app, T.cap[t] - n_own);
     O.cnt[t] = min(s_leave, O.cap);
   }
   if constexpr (DET) {
@@ -977,7 +997,7 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
       if (klo) atomicAdd(&s_ekin[1], (unsigned long long)klo);
     }
     __syncthreads();
-    if (threadIdx.x == 0) ekin_tile[t] = efix_join((long long)s_ekin[0], (long long)s_ekin[1]);
+    if (threadIdx.x == 0) A.ekin[t * parts + rank] = efix_join((long long)s_ekin[0], (long long)s_ekin[1]);
     // the integer J tile goes to the global fixed-point planes (units of
     // 2^-40) with 64-bit integer atomics (cells outside the buffer hold no
     // deposits)
@@ -994,7 +1014,7 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
       errbits |= ERR_TIMEOUT;  // second bounded wait for the load still in flight
   } else {
     const double e = block_sum_double<NT>((double)ks - (double)kc, sred);
-    if (threadIdx.x == 0) ekin_tile[t] = e;
+    if (threadIdx.x == 0) A.ekin[t * parts + rank] = e;
 
     if (threadIdx.x == 0 && !loaded && !mbar_wait_bounded(&bar, 0))
       errbits |= ERR_TIMEOUT;  // second bounded wait for the load still in flight
@@ -1003,26 +1023,33 @@ __global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS) k_push
 }
 
 // ---------------------------------------------------------------------------
-// spill push: same physics from global memory (rarely non-empty)
+// spill push: same physics from global memory (rarely non-empty), by block
+// `block` of `nblocks`; leaves the block's kinetic energy in A.ekin_spill
+// (deterministic builds: adds it to the two words of A.ekin_fix)
 // ---------------------------------------------------------------------------
 template <int NT, bool DET>
-__global__ void __launch_bounds__(NT) k_push_spill(const float *EB, float *J, FixedJ fj, Grid G, Particles sin,
-                                                   const int *sin_cnt, int sin_cap, Spill S, double *ekin,
-                                                   int *err, PushConst C) {
+__device__ __forceinline__ void push_spill(const float *EB, const FixedJ &fj, const Grid &G, const PushSpecies &A,
+                                           int *err, int block, int nblocks) {
   __shared__ double sred[NT / 32];
-  const int n = min(*sin_cnt, sin_cap);
-  if (n == 0) return;  // the usual case: nothing spilled (uniform across the grid)
+  const PushConst &C = A.C;
+  const Particles &sin = A.Sin.p;
+  const Spill &S = A.S;
+  const int n = min(*A.Sin.cnt, A.Sin.cap);
+  if (n == 0) {  // the usual case: nothing spilled (uniform across the blocks)
+    if (!DET && threadIdx.x == 0) A.ekin_spill[block] = 0.0;
+    return;
+  }
   const GlobalFields fld{EB, G.pitch, G.plane};
   const auto dep = [&] {
     if constexpr (DET)
       return GlobalCurrentFixed{fj.p, fj.pitch, fj.plane, &C};
     else
-      return GlobalCurrent{J, G.pitch, G.plane};
+      return GlobalCurrent{fj.f, G.pitch, G.plane};
   }();
   int errbits = 0;
   float ks = 0.f, kc = 0.f;
   long long khi = 0, klo = 0;
-  for (int k = blockIdx.x * NT + threadIdx.x; k < n; k += gridDim.x * NT) {
+  for (int k = block * NT + threadIdx.x; k < n; k += nblocks * NT) {
     const PRec r = load_particle(sin, k);
     int ix = r.ix, iy = r.iy;
     float x = r.x, y = r.y, ux = r.ux, uy = r.uy, uz = r.uz;
@@ -1053,13 +1080,45 @@ __global__ void __launch_bounds__(NT) k_push_spill(const float *EB, float *J, Fi
     if (apply_boundary(ix, iy, di, dj, C)) spill_particle(S, &errbits, ix, iy, x, y, ux, uy, uz);
   }
   if constexpr (DET) {
-    if (khi) atomicAdd(reinterpret_cast<unsigned long long *>(ekin), (unsigned long long)khi);
-    if (klo) atomicAdd(reinterpret_cast<unsigned long long *>(ekin) + 1, (unsigned long long)klo);
+    if (khi) atomicAdd(A.ekin_fix, (unsigned long long)khi);
+    if (klo) atomicAdd(A.ekin_fix + 1, (unsigned long long)klo);
   } else {
     const double e = block_sum_double<NT>((double)ks - (double)kc, sred);
-    if (threadIdx.x == 0 && e != 0.0) atomicAdd(ekin, e);
+    if (threadIdx.x == 0) A.ekin_spill[block] = e;
   }
   if (errbits) atomicOr(err, errbits);
+}
+
+// ---------------------------------------------------------------------------
+// kernels: one species' tiles; its spilled particles; and, for small grids,
+// every species' tiles (each by a cluster of `parts` CTAs) and spilled
+// particles in one launch
+// ---------------------------------------------------------------------------
+template <int TX, int TY, int NT, bool DET>
+__global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS)
+    k_push_tiles(const __grid_constant__ CUtensorMap tm_eb, const __grid_constant__ PushSpecies A, int *err,
+                 FixedJ fj) {
+  push_tile<TX, TY, NT, DET, false>(tm_eb, A, err, fj, blockIdx.x, 0, 1);
+}
+
+template <int NT, bool DET>
+__global__ void __launch_bounds__(NT) k_push_spill(const float *EB, FixedJ fj, Grid G,
+                                                   const __grid_constant__ PushSpecies A, int *err) {
+  push_spill<NT, DET>(EB, fj, G, A, err, blockIdx.x, gridDim.x);
+}
+
+template <int TX, int TY, int NT, bool DET>
+__global__ void __launch_bounds__(NT, DET ? 512 / NT : 4)
+    k_push_all(const __grid_constant__ CUtensorMap tm_eb, const __grid_constant__ PushAll P, const float *EB, Grid G,
+               int *err, FixedJ fj) {
+  const int b = blockIdx.x, ntile = P.nsp * P.ntiles * P.parts;
+  if (b < ntile) {
+    const int q = b / P.parts, k = q / P.ntiles;
+    push_tile<TX, TY, NT, DET, true>(tm_eb, P.sp[k], err, fj, q - k * P.ntiles, b - q * P.parts, P.parts);
+  } else {
+    const int k = (b - ntile) / kSpillParts;
+    push_spill<NT, DET>(EB, fj, G, P.sp[k], err, (b - ntile) % kSpillParts, kSpillParts);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1067,33 +1126,24 @@ __global__ void __launch_bounds__(NT) k_push_spill(const float *EB, float *J, Fi
 // ---------------------------------------------------------------------------
 template <int TX, int TY, bool DET>
 static cudaError_t launch_push_t(const PushLaunch &a, cudaStream_t st) {
-  // 4 warps per CTA (8 CTAs per SM: shorter barriers, CTAs in more phases);
-  // the deterministic build's integer J tile keeps 8 warps per CTA
-  constexpr int NT = (DET && TX * TY >= 256) ? 256 : 128;
-  k_push_tiles<TX, TY, NT, DET><<<a.ntiles, NT, 0, st>>>(*a.tm_eb, a.pin, a.pout, a.T, a.Oin, a.O, a.S,
-                                                           a.ekin_tile, a.err, a.C, a.fj);
+  // 4 warps per CTA (shorter barriers, CTAs in more phases); the
+  // deterministic build's integer J tile keeps 8 warps per CTA
+  constexpr int NT = (DET && TX * TY >= 256) ? 256 : 32 * kPushWarps;
+  if (a.all) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(a.all->nsp * (a.all->ntiles * a.all->parts + kSpillParts));
+    cfg.blockDim = dim3(NT);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = a.all->parts;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_push_all<TX, TY, NT, DET>, *a.tm_eb, *a.all, a.EB, a.G, a.err, a.fj);
+  }
+  k_push_tiles<TX, TY, NT, DET><<<a.ntiles, NT, 0, st>>>(*a.tm_eb, *a.one, a.err, a.fj);
   return cudaGetLastError();
-}
-
-// nothing to prepare: every variant runs with static shared memory only
-template <int TX, int TY, bool DET>
-static cudaError_t prepare_push_t() {
-  return cudaSuccess;
-}
-
-template <bool DET>
-static cudaError_t prepare_push_variant(int TX, int TY) {
-#define ZC_TILE(X, Y) \
-  if (TX == X && TY == Y) return prepare_push_t<X, Y, DET>();
-  ZC_TILE(16, 16)
-  ZC_TILE(8, 8)
-  ZC_TILE(16, 8)
-  ZC_TILE(32, 16)
-  ZC_TILE(32, 32)
-  ZC_TILE(8, 16)
-  ZC_TILE(16, 32)
-#undef ZC_TILE
-  return cudaErrorInvalidValue;
 }
 
 template <bool DET>
@@ -1113,10 +1163,7 @@ static cudaError_t launch_push_tiles_variant(const PushLaunch &a, cudaStream_t s
 }
 
 template <bool DET>
-static cudaError_t launch_push_spill_variant(const float *EB, float *J, const FixedJ &fj, const Grid &G,
-                                             const Particles &sin, const int *sin_cnt, int sin_cap, const Spill &S,
-                                             double *ekin, int *err, const PushConst &C, int nblocks,
-                                             cudaStream_t st) {
-  k_push_spill<256, DET><<<nblocks, 256, 0, st>>>(EB, J, fj, G, sin, sin_cnt, sin_cap, S, ekin, err, C);
+static cudaError_t launch_push_spill_variant(const PushLaunch &a, int nblocks, cudaStream_t st) {
+  k_push_spill<256, DET><<<nblocks, 256, 0, st>>>(a.EB, a.fj, a.G, *a.one, a.err);
   return cudaGetLastError();
 }
