@@ -139,8 +139,8 @@ struct Counters {
   int iter = 0, n_move = 0;
   std::vector<int> sp_iter, sp_n_move, cur, spill_cur, ob_in;
   std::vector<bool> pending, spill_clean;
-  int eb_cur = 0, j_cur = 0;
-  bool j0_zero = false;
+  int eb_cur = 0, j_cur = 0, jr = 0;
+  bool j0_zero = false, j_plain = false;
   long long launch[ZC_NPHASE] = {};
 };
 
@@ -177,12 +177,15 @@ struct zc_sim {
   float *EBp = nullptr, *extE = nullptr, *extB = nullptr;
   int ext_Et = 0, ext_Bt = 0;
   float3 ext_E0{0, 0, 0}, ext_B0{0, 0, 0};
-  float *J[2] = {nullptr, nullptr};
+  // raw deposits (J[0] and J[2] in turn: jr) and the current the fields see
+  float *J[3] = {nullptr, nullptr, nullptr};
+  int jr = 0;
+  bool j_plain = false;  // J[1] holds an unfiltered current (see restore_current)
   int j_cur = 0;
-  bool j0_zero = false;  // J[0] was cleared by the last Yee launch (no clear needed)
+  bool j0_zero = false;  // the raw buffer was cleared by the last field launch (no clear needed)
   unsigned long long *Jfix = nullptr;   // deterministic mode: fixed-point J planes
-  CUtensorMap tmK_EB[2], tmK_EBp, tmK_J;
-  CUtensorMap tmY_EB[2], tmY_J[2];
+  CUtensorMap tmK_EB[2], tmK_EBp;
+  CUtensorMap tmY_EB[2], tmY_J[3], tmF_J[2];
   int TX = 16, TY = 16, ntx = 0, nty = 0, ntiles = 0;
   std::vector<SpeciesState> sp;
   int xtype = 0, ytype = 0, xlevel = 0, ylevel = 0;
@@ -323,7 +326,12 @@ TileSet tiles(SpeciesState &p, int ntiles) { return TileSet{p.d_off, p.d_cap, p.
 
 Spill spill_of(SpeciesState &p, int k) { return Spill{p.spill[k], p.d_spill_cnt + k, p.spill_cap}; }
 
-FixedJ fixed_j(const zc_sim *s) { return FixedJ{s->Jfix, s->G.pitch, s->G.plane, s->J[0]}; }
+// the raw deposit buffer, and the current the fields saw last
+int raw_index(const zc_sim *s) { return s->jr ? 2 : 0; }
+float *raw_j(const zc_sim *s) { return s->J[raw_index(s)]; }
+float *seen_j(const zc_sim *s) { return s->j_cur == 1 ? s->J[1] : raw_j(s); }
+
+FixedJ fixed_j(const zc_sim *s) { return FixedJ{s->Jfix, s->G.pitch, s->G.plane, raw_j(s)}; }
 
 // outbox slots per tile: room for a moving-window column plus crossers
 // (more leavers than slots go to the spill list)
@@ -741,7 +749,7 @@ zc_status species_pushed(zc_sim *s, int k, int shift);
 zc_status fixed_current(zc_sim *s) {
   if (!s->deterministic) return ZC_OK;
   Phase ph(s, ZC_PHASE_ZERO, 1);
-  CK(launch_fixed_to_float(s->Jfix, s->J[0], 3 * s->G.plane, s->st));
+  CK(launch_fixed_to_float(s->Jfix, raw_j(s), 3 * s->G.plane, s->st));
   return ZC_OK;
 }
 
@@ -907,15 +915,10 @@ void smooth_comp(int n, float *sa, float *sb) {  // get_smooth_comp, em2d/curren
   *sb = b / total;
 }
 
-zc_status current_update_impl(zc_sim *s) {
-  cudaStream_t st = s->st;
-  {
-    Phase ph(s, ZC_PHASE_FOLD, s->mw ? 1 : 2);
-    CK(launch_fold(s->J[0], s->G, s->mw, st));
-  }
-  // pass coefficients (current_smooth, em2d/current.c:427-459; the y
-  // binomial pass count is xlevel, as at current.c:449)
-  SmoothPasses px{}, py{};
+// the filter's pass coefficients (current_smooth, em2d/current.c:427-459; the
+// y binomial pass count is xlevel, as at current.c:449)
+void filter_passes(const zc_sim *s, SmoothPasses &px, SmoothPasses &py) {
+  px = py = SmoothPasses{};
   float sa, sb;
   if (s->xtype != 0) {
     for (int i = 0; i < s->xlevel; ++i) px.sa[px.n] = 0.25f, px.sb[px.n++] = 0.5f;
@@ -931,19 +934,27 @@ zc_status current_update_impl(zc_sim *s) {
       py.sa[py.n] = sa, py.sb[py.n++] = sb;
     }
   }
+}
+
+zc_status current_update_impl(zc_sim *s) {
+  cudaStream_t st = s->st;
+  {
+    Phase ph(s, ZC_PHASE_FOLD, s->mw ? 1 : 2);
+    CK(launch_fold(raw_j(s), s->G, s->mw, st));
+  }
+  SmoothPasses px, py;
+  filter_passes(s, px, py);
   int c = 0;
   if (px.n > 0 || py.n > 0) {
     Phase ph(s, ZC_PHASE_SMOOTH, 1);
-    CK(launch_smooth(s->J[0], s->J[1], s->G, px, py, s->mw, st));
+    CK(launch_smooth(raw_j(s), s->J[1], s->G, px, py, s->mw, st));
     c = 1;
   }
   s->j_cur = c;
   return ZC_OK;
 }
 
-// epart: where the Yee kernel leaves the new fields' energy partials (or null)
-zc_status emf_advance_impl(zc_sim *s, double *epart = nullptr) {
-  cudaStream_t st = s->st;
+YeeConst yee_const(const zc_sim *s) {
   YeeConst Y;
   const float dth = s->dt / 2.0f;
   Y.cxb = dth / s->dx[0];
@@ -952,21 +963,46 @@ zc_status emf_advance_impl(zc_sim *s, double *epart = nullptr) {
   Y.cye = s->dt / s->dx[1];
   Y.dt = s->dt;
   Y.mw = s->mw;
-  const int o = 1 - s->eb_cur;
-  // the Yee kernel writes the guard cells as the guard-cell update leaves
-  // them, and clears the raw deposit buffer once the filter has read it
-  const bool gc = s->nx >= 3 && s->ny >= 3;
-  float *jz = (s->j_cur == 1) ? s->J[0] : nullptr;
-  // ... and the spill counts that the next pushes start from
+  return Y;
+}
+
+// the spill counts that the next pushes start from: cleared by a field kernel
+ZeroWords next_spill_counts(zc_sim *s) {
   ZeroWords zero{};
   if ((int)s->sp.size() <= kMaxTogether)
     for (auto &p : s->sp) {
       zero.p[zero.n++] = p.d_spill_cnt + (1 - p.spill_cur);
       p.spill_clean = true;
     }
+  return zero;
+}
+
+// a field advance is done: counters, window move (emf_move_window, emf.c:650)
+zc_status emf_advanced(zc_sim *s) {
+  s->iter += 1;
+  if (s->mw && (s->iter * s->dt) > s->dx[0] * (s->n_move + 1)) {
+    Phase ph(s, ZC_PHASE_WINDOW, 1);
+    const int o = 1 - s->eb_cur;
+    CK(launch_window_shift(s->EB[s->eb_cur], s->EB[o], s->G, s->st));
+    s->eb_cur = o;
+    s->n_move += 1;
+  }
+  return ZC_OK;
+}
+
+// epart: where the Yee kernel leaves the new fields' energy partials (or null)
+zc_status emf_advance_impl(zc_sim *s, double *epart = nullptr) {
+  cudaStream_t st = s->st;
+  const YeeConst Y = yee_const(s);
+  const int o = 1 - s->eb_cur;
+  // the Yee kernel writes the guard cells as the guard-cell update leaves
+  // them, and clears the raw deposit buffer once the filter has read it
+  const bool gc = s->nx >= 3 && s->ny >= 3;
+  float *jz = (s->j_cur == 1) ? raw_j(s) : nullptr;
+  const ZeroWords zero = next_spill_counts(s);
   {
     Phase ph(s, ZC_PHASE_YEE, 1);
-    CK(launch_yee(&s->tmY_EB[s->eb_cur], &s->tmY_J[s->j_cur], s->EB[o], s->G, Y, s->d_err, epart, jz, gc, zero, st));
+    CK(launch_yee(&s->tmY_EB[s->eb_cur], &s->tmY_J[s->j_cur == 1 ? 1 : raw_index(s)], s->EB[o], s->G, Y, s->d_err, epart, jz, gc, zero, st));
   }
   if (jz) s->j0_zero = true;
   s->eb_cur = o;
@@ -978,21 +1014,59 @@ zc_status emf_advance_impl(zc_sim *s, double *epart = nullptr) {
     Phase ph(s, ZC_PHASE_EXT, 1);
     CK(launch_ext_add(s->EB[o], s->EBp, s->extE, s->extB, s->ext_Et, s->ext_Bt, s->ext_E0, s->ext_B0, s->G, st));
   }
-  s->iter += 1;
-  if (s->mw && (s->iter * s->dt) > s->dx[0] * (s->n_move + 1)) {  // emf_move_window, emf.c:650
-    Phase ph(s, ZC_PHASE_WINDOW, 1);
-    CK(launch_window_shift(s->EB[o], s->EB[1 - o], s->G, st));
-    s->eb_cur = 1 - o;
-    s->n_move += 1;
+  return emf_advanced(s);
+}
+
+// fold, filter and Yee advance of a step in one launch (not for more than 4
+// filter passes an axis or grids below 6 cells: *done tells)
+zc_status fields_impl(zc_sim *s, double *epart, bool *done) {
+  SmoothPasses px, py;
+  filter_passes(s, px, py);
+  *done = fields_together(s->G, px, py);
+  if (!*done) return ZC_OK;
+  const int o = 1 - s->eb_cur;
+  ExtField X;
+  if (s->EBp) {
+    X.out = s->EBp;
+    X.E = s->extE;
+    X.B = s->extB;
+    X.Et = s->ext_Et;
+    X.Bt = s->ext_Bt;
+    const float v[6] = {s->ext_E0.x, s->ext_E0.y, s->ext_E0.z, s->ext_B0.x, s->ext_B0.y, s->ext_B0.z};
+    std::memcpy(X.v0, v, sizeof v);
   }
+  const ZeroWords zero = next_spill_counts(s);
+  {
+    Phase ph(s, ZC_PHASE_YEE, 1);
+    CK(launch_fields(&s->tmY_EB[s->eb_cur], &s->tmF_J[s->jr], raw_j(s), s->J[1], s->J[s->jr ? 0 : 2], s->EB[o], X,
+                     s->G, yee_const(s), px, py, s->d_err, epart, zero, s->st));
+  }
+  s->jr ^= 1;
+  s->j0_zero = true;
+  s->j_cur = 1;
+  s->j_plain = px.n == 0 && py.n == 0;
+  s->eb_cur = o;
+  return emf_advanced(s);
+}
+
+// Before a call that works on the raw current by itself: without a filter it
+// holds the last step's folded current (a step leaves it beside the raw
+// buffer, which is cleared for the next).
+zc_status restore_current(zc_sim *s) {
+  if (!s->j_plain) return ZC_OK;
+  CK(cudaMemcpyAsync(raw_j(s), s->J[1], sizeof(float) * 3 * s->G.plane, cudaMemcpyDeviceToDevice, s->st));
+  s->j_plain = false;
+  s->j0_zero = false;
+  s->j_cur = 0;
   return ZC_OK;
 }
 
-// in a step (in_step) a J[0] the last Yee launch cleared is not cleared again
+// in a step (in_step) a raw buffer the last field launch cleared is not cleared again
 zc_status current_zero_impl(zc_sim *s, bool in_step = false) {
   Phase ph(s, ZC_PHASE_ZERO, 0);
-  if (!(in_step && s->j0_zero)) CK(cudaMemsetAsync(s->J[0], 0, sizeof(float) * 3 * s->G.plane, s->st));
+  if (!(in_step && s->j0_zero)) CK(cudaMemsetAsync(raw_j(s), 0, sizeof(float) * 3 * s->G.plane, s->st));
   s->j0_zero = false;
+  s->j_plain = false;
   if (s->deterministic) CK(cudaMemsetAsync(s->Jfix, 0, sizeof(unsigned long long) * 3 * s->G.plane, s->st));
   s->j_cur = 0;
   return ZC_OK;
@@ -1012,9 +1086,14 @@ zc_status iter_impl(zc_sim *s, bool last) {
     for (size_t k = 0; k < s->sp.size(); ++k) TRY(spec_advance_impl(s, (int)k));
   if (!s->sp.empty()) TRY(fixed_current(s));
   if (last && !hist && !s->sp.empty()) TRY(kin_energies(s, 0, s->sp.size(), parts));
-  TRY(current_update_impl(s));
   const bool fused = hist && !s->mw;
-  TRY(emf_advance_impl(s, fused ? s->d_hist_part : nullptr));
+  double *epart = fused ? s->d_hist_part : nullptr;
+  bool done = false;
+  TRY(fields_impl(s, epart, &done));
+  if (!done) {
+    TRY(current_update_impl(s));
+    TRY(emf_advance_impl(s, epart));
+  }
   if (hist) {
     Phase ph(s, ZC_PHASE_HISTORY, fused ? 1 : 2);
     CK(launch_energy_history(fused ? nullptr : s->EB[s->eb_cur], s->G, s->d_hist_part,
@@ -1068,6 +1147,8 @@ Counters save_counters(const zc_sim *s) {
   c.eb_cur = s->eb_cur;
   c.j_cur = s->j_cur;
   c.j0_zero = s->j0_zero;
+  c.jr = s->jr;
+  c.j_plain = s->j_plain;
   for (int k = 0; k < ZC_NPHASE; ++k) c.launch[k] = s->prof_launch[k];
   return c;
 }
@@ -1075,7 +1156,7 @@ Counters save_counters(const zc_sim *s) {
 // the buffer parities a captured graph starts from
 bool same_parities(const Counters &a, const Counters &b) {
   return a.cur == b.cur && a.spill_cur == b.spill_cur && a.ob_in == b.ob_in && a.eb_cur == b.eb_cur &&
-         a.spill_clean == b.spill_clean && a.j0_zero == b.j0_zero && (a.iter % 2) == (b.iter % 2);
+         a.spill_clean == b.spill_clean && a.j0_zero == b.j0_zero && a.jr == b.jr && (a.iter % 2) == (b.iter % 2);
 }
 
 // the graph g holds n steps from the current state (block-aligned)
@@ -1129,6 +1210,8 @@ zc_status capture_steps(zc_sim *s, int n, StepGraph &G, bool instantiate = true)
   s->eb_cur = before.eb_cur;
   s->j_cur = before.j_cur;
   s->j0_zero = before.j0_zero;
+  s->jr = before.jr;
+  s->j_plain = before.j_plain;
   for (int k = 0; k < ZC_NPHASE; ++k) s->prof_launch[k] = before.launch[k];
   if (st != ZC_OK) {
     if (g) cudaGraphDestroy(g);
@@ -1216,6 +1299,8 @@ void account_steps(zc_sim *s, const StepGraph &g) {
   s->eb_cur = g.after.eb_cur;
   s->j_cur = g.after.j_cur;
   s->j0_zero = g.after.j0_zero;
+  s->jr = g.after.jr;
+  s->j_plain = g.after.j_plain;
   for (int k = 0; k < ZC_NPHASE; ++k) s->prof_launch[k] += g.after.launch[k] - g.before.launch[k];
 }
 
@@ -1504,9 +1589,11 @@ zc_status zc_sim_create(const zc_sim_desc *d, zc_sim **out) {
   }
   for (int b = 0; b < 2; ++b) {
     TRYC(dalloc(&s->EB[b], 6 * G.plane));
-    TRYC(dalloc(&s->J[b], 3 * G.plane));
     cudaMemsetAsync(s->EB[b], 0, sizeof(float) * 6 * G.plane, s->st);
-    cudaMemsetAsync(s->J[b], 0, sizeof(float) * 3 * G.plane, s->st);
+  }
+  for (auto &j : s->J) {
+    TRYC(dalloc(&j, 3 * G.plane));
+    cudaMemsetAsync(j, 0, sizeof(float) * 3 * G.plane, s->st);
   }
   if (s->deterministic) {
     TRYC(dalloc(&s->Jfix, 3 * G.plane));
@@ -1527,9 +1614,9 @@ zc_status zc_sim_create(const zc_sim_desc *d, zc_sim **out) {
     for (int b = 0; b < 2; ++b) {
       TRYC(make_map(&s->tmK_EB[b], s->EB[b], G, 6, BW, BH));
       TRYC(make_map(&s->tmY_EB[b], s->EB[b], G, 6, kYeeBW, kYeeBH));
-      TRYC(make_map(&s->tmY_J[b], s->J[b], G, 3, kYeeBW, kYeeBH));
+      TRYC(make_map(&s->tmF_J[b], s->J[2 * b], G, 3, kFieldBW, kFieldBH));
     }
-    TRYC(make_map(&s->tmK_J, s->J[0], G, 3, BW, BH));
+    for (int b = 0; b < 3; ++b) TRYC(make_map(&s->tmY_J[b], s->J[b], G, 3, kYeeBW, kYeeBH));
   }
   if (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->inj_done, cudaEventDisableTiming) != cudaSuccess ||
@@ -1573,10 +1660,8 @@ zc_status zc_sim_destroy(zc_sim *s) {
     dfree(p.d_ekin_fix);
     dfree(p.d_ekin);
   }
-  for (int b = 0; b < 2; ++b) {
-    dfree(s->EB[b]);
-    dfree(s->J[b]);
-  }
+  for (auto &f : s->EB) dfree(f);
+  for (auto &j : s->J) dfree(j);
   dfree(s->Jfix);
   dfree(s->EBp);
   dfree(s->extE);
@@ -1993,6 +2078,7 @@ zc_status zc_spec_advance(zc_sim *s, int k) {
   TRY(check_species(s, k));
   DeviceGuard g(s->device);
   CK(cudaEventRecord(s->ev0, s->st));
+  TRY(restore_current(s));
   TRY(spec_advance_impl(s, k));
   TRY(fixed_current(s));
   TRY(kin_energies(s, k, 1, 0));
@@ -2006,6 +2092,7 @@ zc_status zc_spec_advance(zc_sim *s, int k) {
 zc_status zc_current_update(zc_sim *s) {
   if (!s) return fail(ZC_EINVAL, "null simulation handle");
   DeviceGuard g(s->device);
+  TRY(restore_current(s));
   TRY(current_update_impl(s));
   CK(cudaStreamSynchronize(s->st));
   return ZC_OK;
@@ -2014,6 +2101,7 @@ zc_status zc_current_update(zc_sim *s) {
 zc_status zc_emf_advance(zc_sim *s) {
   if (!s) return fail(ZC_EINVAL, "null simulation handle");
   DeviceGuard g(s->device);
+  TRY(restore_current(s));
   TRY(emf_advance_impl(s));
   CK(cudaStreamSynchronize(s->st));
   return check_errors(s, false);
@@ -2049,7 +2137,7 @@ zc_status zc_get_particle_fields(zc_sim *s, float *E, float *B) {
 zc_status zc_get_current(zc_sim *s, float *J) {
   if (!s || !J) return fail(ZC_EINVAL, "null argument");
   DeviceGuard g(s->device);
-  return grid_down(s, s->J[s->j_cur], J);
+  return grid_down(s, seen_j(s), J);
 }
 
 struct zc_fence {
@@ -2068,7 +2156,7 @@ zc_status zc_copy_grid_async(zc_sim *s, int grid, int comp, float *dst, zc_fence
     case ZC_GRID_B: base = eb + 3 * s->G.plane; break;
     case ZC_GRID_EPART: base = ebp; break;
     case ZC_GRID_BPART: base = ebp + 3 * s->G.plane; break;
-    case ZC_GRID_J: base = s->J[s->j_cur]; break;
+    case ZC_GRID_J: base = seen_j(s); break;
     default: return fail(ZC_EINVAL, "unknown grid %d", grid);
   }
   // interior cell (0, 0) sits at buffer column 1 of buffer row 1
@@ -2119,11 +2207,12 @@ void zc_host_free(void *p) {
 zc_status zc_set_current(zc_sim *s, const float *J) {
   if (!s || !J) return fail(ZC_EINVAL, "null argument");
   DeviceGuard g(s->device);
-  TRY(grid_up(s, J, s->J[0]));
+  TRY(grid_up(s, J, raw_j(s)));
   s->j_cur = 0;
+  s->j_plain = false;
   s->j0_zero = false;
   if (s->deterministic) {
-    CK(launch_float_to_fixed(s->J[0], s->Jfix, 3 * s->G.plane, s->st));
+    CK(launch_float_to_fixed(raw_j(s), s->Jfix, 3 * s->G.plane, s->st));
     CK(cudaStreamSynchronize(s->st));
   }
   return ZC_OK;
@@ -2243,7 +2332,7 @@ zc_status zc_grid_view_get(zc_sim *s, zc_grid_view *v) {
   if (!s || !v) return fail(ZC_EINVAL, "null argument");
   v->E = s->EB[s->eb_cur];
   v->B = s->EB[s->eb_cur] + 3 * s->G.plane;
-  v->J = s->J[s->j_cur];
+  v->J = seen_j(s);
   v->plane = s->G.plane;
   v->pitch = s->G.pitch;
   v->rows = s->G.rows;

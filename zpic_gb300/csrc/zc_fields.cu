@@ -469,13 +469,190 @@ __global__ void __launch_bounds__(32 * kS4Warps, ZC_S4_MINB) k_smooth4(const flo
 // guard cells evolve as in the reference (they matter with a moving window).
 // Out of place: EB in (TMA) -> EB out.
 // ---------------------------------------------------------------------------
+// a field value stored at (bx, by), with external fields also where the
+// particles read it (emf_update_part_fld, em2d/emf.c:838-914)
+__device__ __forceinline__ void put_field(float *EB, const ExtField &X, const Grid &G, int c, int bx, int by, float v) {
+  const size_t k = gidx(G, c, bx, by);
+  EB[k] = v;
+  if (X.out) {
+    const int t = c < 3 ? X.Et : X.Bt;
+    if (t == 1) v += X.v0[c];
+    if (t == 2) v += (c < 3 ? X.E : X.B)[c < 3 ? k : k - 3 * G.plane];
+    X.out[k] = v;
+  }
+}
+
 // a value stored at (bx, by) and at its periodic guard images (xm, ym; -1: none)
-__device__ __forceinline__ void put_mirrored(float *EB, const Grid &G, int c, int bx, int by, int xm, int ym,
-                                             float v) {
-  EB[gidx(G, c, bx, by)] = v;
-  if (xm >= 0) EB[gidx(G, c, xm, by)] = v;
-  if (ym >= 0) EB[gidx(G, c, bx, ym)] = v;
-  if (xm >= 0 && ym >= 0) EB[gidx(G, c, xm, ym)] = v;
+__device__ __forceinline__ void put_mirrored(float *EB, const ExtField &X, const Grid &G, int c, int bx, int by,
+                                             int xm, int ym, float v) {
+  put_field(EB, X, G, c, bx, by, v);
+  if (xm >= 0) put_field(EB, X, G, c, xm, by, v);
+  if (ym >= 0) put_field(EB, X, G, c, bx, ym, v);
+  if (xm >= 0 && ym >= 0) put_field(EB, X, G, c, xm, ym, v);
+}
+
+// J of the output tile and the row and column past it
+struct YeeCurrent {
+  const float *at;   // Jx of the tile's first cell
+  int pitch, plane;
+};
+
+// the advance of one tile from its staged fields and current (every thread
+// has seen the staging complete)
+__device__ __forceinline__ void yee_tile(float *sEB, const YeeCurrent &J, int bx0, int by0, float *EBout,
+                                         const ExtField &ext, const Grid &G, const YeeConst &Y, double *epart,
+                                         float *jzero, int gc) {
+  constexpr int BW = kYeeBW, BH = kYeeBH, PL = BW * BH;
+  const int ox = bx0 - 4, oy = by0 - 1;  // buffer coords of sEB (0, 0)
+  float *Ex = sEB, *Ey = sEB + PL, *Ez = sEB + 2 * PL;
+  float *Bx = sEB + 3 * PL, *By = sEB + 4 * PL, *Bz = sEB + 5 * PL;
+  const float *Jx = J.at, *Jy = J.at + J.plane, *Jz = J.at + 2 * J.plane;
+  const int nx = G.nx, ny = G.ny;
+
+  if (epart == nullptr && !ext.out && bx0 >= 3 && bx0 + kYeeOX <= nx && by0 >= 3 && by0 + kYeeOY <= ny) {
+    // A tile clear of the guard cells and of the cells they copy: every cell
+    // of the three updates exists, a lane a column and a warp a row (the same
+    // operations as below, with a third of the index arithmetic).
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto half_b = [&](int k) {
+      Bx[k] += (-Y.cyb * (Ez[k + BW] - Ez[k]));
+      By[k] += (Y.cxb * (Ez[k + 1] - Ez[k]));
+      Bz[k] += (-Y.cxb * (Ey[k + 1] - Ey[k]) + Y.cyb * (Ex[k + BW] - Ex[k]));
+    };
+    for (int r = warp; r < kYeeOY + 2; r += 8) half_b(r * BW + lane + 3);
+    if (threadIdx.x < 2 * (kYeeOY + 2)) half_b((threadIdx.x >> 1) * BW + 35 + (threadIdx.x & 1));
+    __syncthreads();
+    auto full_e = [&](int r, int c) {
+      const int k = (r + 1) * BW + c + 4, q = r * J.pitch + c;
+      Ex[k] += (+Y.cye * (Bz[k] - Bz[k - BW])) - Y.dt * Jx[q];
+      Ey[k] += (-Y.cxe * (Bz[k] - Bz[k - 1])) - Y.dt * Jy[q];
+      Ez[k] += (+Y.cxe * (By[k] - By[k - 1]) - Y.cye * (Bx[k] - Bx[k - BW])) - Y.dt * Jz[q];
+    };
+    for (int r = warp; r < kYeeOY + 1; r += 8) full_e(r, lane);
+    if (threadIdx.x < kYeeOY + 1) full_e(threadIdx.x, kYeeOX);
+    __syncthreads();
+    for (int r = warp; r < kYeeOY; r += 8) {
+      const int k = (r + 1) * BW + lane + 4;
+      const float bxv = Bx[k] + (-Y.cyb * (Ez[k + BW] - Ez[k]));
+      const float byv = By[k] + (Y.cxb * (Ez[k + 1] - Ez[k]));
+      const float bzv = Bz[k] + (-Y.cxb * (Ey[k + 1] - Ey[k]) + Y.cyb * (Ex[k + BW] - Ex[k]));
+      const size_t at = (size_t)(by0 + r) * G.pitch + bx0 + lane;
+      if (jzero) {
+        float *z = jzero + at;
+        z[0] = 0.f;
+        z[G.plane] = 0.f;
+        z[2 * G.plane] = 0.f;
+      }
+      float *o = EBout + at;
+      o[0] = Ex[k];
+      o += G.plane;
+      o[0] = Ey[k];
+      o += G.plane;
+      o[0] = Ez[k];
+      o += G.plane;
+      o[0] = bxv;
+      o += G.plane;
+      o[0] = byv;
+      o += G.plane;
+      o[0] = bzv;
+    }
+    return;
+  }
+
+  // B1 on buffer cells [bx0-1, bx0+OX] x [by0-1, by0+OY]
+  {
+    constexpr int W = kYeeOX + 2, H = kYeeOY + 2;
+    for (int k = threadIdx.x; k < W * H; k += blockDim.x) {
+      const int bx = bx0 - 1 + k % W, by = by0 - 1 + k / W;
+      if (bx < 0 || bx > nx + 1 || by < 0 || by > ny + 1) continue;
+      const int s = (by - oy) * BW + (bx - ox);
+      Bx[s] += (-Y.cyb * (Ez[s + BW] - Ez[s]));
+      By[s] += (Y.cxb * (Ez[s + 1] - Ez[s]));
+      Bz[s] += (-Y.cxb * (Ey[s + 1] - Ey[s]) + Y.cyb * (Ex[s + BW] - Ex[s]));
+    }
+  }
+  __syncthreads();
+  // E1 on buffer cells [bx0, bx0+OX] x [by0, by0+OY]
+  {
+    constexpr int W = kYeeOX + 1, H = kYeeOY + 1;
+    for (int k = threadIdx.x; k < W * H; k += blockDim.x) {
+      const int bx = bx0 + k % W, by = by0 + k / W;
+      if (bx < 1 || bx > nx + 2 || by < 1 || by > ny + 2) continue;
+      const int s = (by - oy) * BW + (bx - ox), q = (by - by0) * J.pitch + (bx - bx0);
+      Ex[s] += (+Y.cye * (Bz[s] - Bz[s - BW])) - Y.dt * Jx[q];
+      Ey[s] += (-Y.cxe * (Bz[s] - Bz[s - 1])) - Y.dt * Jy[q];
+      Ez[s] += (+Y.cxe * (By[s] - By[s - 1]) - Y.cye * (Bx[s] - Bx[s - BW])) - Y.dt * Jz[q];
+    }
+  }
+  __syncthreads();
+  // B2 on the output tile, then store E1 and B2; with epart, the squares of
+  // the interior cells' new values are summed for the field energy
+  float se[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int k = threadIdx.x; k < kYeeOX * kYeeOY; k += blockDim.x) {
+    const int bx = bx0 + k % kYeeOX, by = by0 + k / kYeeOX;
+    if (bx >= nx + 3 || by >= ny + 3) continue;
+    const int s = (by - oy) * BW + (bx - ox);
+    float bxv = Bx[s], byv = By[s], bzv = Bz[s];
+    if (bx <= nx + 1 && by <= ny + 1) {
+      bxv += (-Y.cyb * (Ez[s + BW] - Ez[s]));
+      byv += (Y.cxb * (Ez[s + 1] - Ez[s]));
+      bzv += (-Y.cxb * (Ey[s + 1] - Ey[s]) + Y.cyb * (Ex[s + BW] - Ex[s]));
+    }
+    if (jzero) {  // the raw deposit buffer, dead once filtered: cleared for the next step
+      jzero[gidx(G, 0, bx, by)] = 0.f;
+      jzero[gidx(G, 1, bx, by)] = 0.f;
+      jzero[gidx(G, 2, bx, by)] = 0.f;
+    }
+    if (gc) {
+      // guard cells as emf_update_gc leaves them (emf.c:573-637): a guard
+      // cell is not stored here; the cell it copies stores its value there
+      // too (periodic in x unless the window moves, always in y)
+      const bool gxc = !Y.mw && (bx == 0 || bx > nx), gyc = (by == 0 || by > ny);
+      if (gxc || gyc) continue;
+      const int xm = Y.mw ? -1 : (bx == nx ? 0 : (bx <= 2 ? nx + bx : -1));
+      const int ym = by == ny ? 0 : (by <= 2 ? ny + by : -1);
+      put_mirrored(EBout, ext, G, 0, bx, by, xm, ym, Ex[s]);
+      put_mirrored(EBout, ext, G, 1, bx, by, xm, ym, Ey[s]);
+      put_mirrored(EBout, ext, G, 2, bx, by, xm, ym, Ez[s]);
+      put_mirrored(EBout, ext, G, 3, bx, by, xm, ym, bxv);
+      put_mirrored(EBout, ext, G, 4, bx, by, xm, ym, byv);
+      put_mirrored(EBout, ext, G, 5, bx, by, xm, ym, bzv);
+    } else {
+      put_field(EBout, ext, G, 0, bx, by, Ex[s]);
+      put_field(EBout, ext, G, 1, bx, by, Ey[s]);
+      put_field(EBout, ext, G, 2, bx, by, Ez[s]);
+      put_field(EBout, ext, G, 3, bx, by, bxv);
+      put_field(EBout, ext, G, 4, bx, by, byv);
+      put_field(EBout, ext, G, 5, bx, by, bzv);
+    }
+    if (epart && bx >= 1 && bx <= nx && by >= 1 && by <= ny) {
+      se[0] += Ex[s] * Ex[s];
+      se[1] += Ey[s] * Ey[s];
+      se[2] += Ez[s] * Ez[s];
+      se[3] += bxv * bxv;
+      se[4] += byv * byv;
+      se[5] += bzv * bzv;
+    }
+  }
+  if (epart) {
+    // warp sums in float (64 cells a warp), then doubles across the warps
+    __shared__ double swe[6][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      float v = se[c];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) swe[c][warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      double v = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v += swe[threadIdx.x][w];
+      epart[(blockIdx.y * gridDim.x + blockIdx.x) * 6 + threadIdx.x] = v;
+    }
+  }
 }
 
 #ifndef ZC_YEE_MINB
@@ -507,105 +684,240 @@ __global__ void __launch_bounds__(256, ZC_YEE_MINB) k_yee(const __grid_constant_
     if (!mbar_wait_bounded(&bar, 0)) return;  // second bounded wait for the copies in flight
   }
 
-  float *Ex = sEB, *Ey = sEB + PL, *Ez = sEB + 2 * PL;
-  float *Bx = sEB + 3 * PL, *By = sEB + 4 * PL, *Bz = sEB + 5 * PL;
-  const float *Jx = sJ, *Jy = sJ + PL, *Jz = sJ + 2 * PL;
-  const int nx = G.nx, ny = G.ny;
+  yee_tile(sEB, YeeCurrent{sJ + BW + 4, BW, PL}, bx0, by0, EBout, ExtField{}, G, Y, epart, jzero, gc);
+}
 
-  // B1 on buffer cells [bx0-1, bx0+OX] x [by0-1, by0+OY]
-  {
-    constexpr int W = kYeeOX + 2, H = kYeeOY + 2;
-    for (int k = threadIdx.x; k < W * H; k += blockDim.x) {
-      const int bx = bx0 - 1 + k % W, by = by0 - 1 + k / W;
-      if (bx < 0 || bx > nx + 1 || by < 0 || by > ny + 1) continue;
-      const int s = (by - oy) * BW + (bx - ox);
-      Bx[s] += (-Y.cyb * (Ez[s + BW] - Ez[s]));
-      By[s] += (Y.cxb * (Ez[s + 1] - Ez[s]));
-      Bz[s] += (-Y.cxb * (Ey[s + 1] - Ey[s]) + Y.cyb * (Ex[s + BW] - Ex[s]));
-    }
+// ---------------------------------------------------------------------------
+// The whole field phase of a step in one launch: guard fold of the deposited
+// current, filter (up to 4 passes an axis), Yee advance, external fields.
+// Three launches (fold, filter, Yee) and a pass over J between them become
+// one; a CTA filters the current of its 32 x 16 tile itself, from the raw
+// deposits of the tile and 4 cells around it.
+//   - raw current: a TMA box where the tile and its halo lie inside the grid
+//     and away from the cells that are folded; else every value is gathered
+//     from its (up to 4) raw places, summed as the folds sum them
+//     (current.c:118-159): columns of a pair first, then rows;
+//   - x passes: a warp a row, two columns a lane, neighbours by shuffles;
+//   - y passes: a thread a column and half the rows, in registers, as k_smooth
+//     (the first pass reads the y guard rows unfiltered);
+//   - the filtered current goes out for the readers of J, and stays in shared
+//     memory for the advance; the raw buffer of the next step is cleared (two
+//     alternate: the neighbours still read this one).
+// Every value is computed with the operations of the separate kernels in
+// their order, so the bits are theirs.
+//
+// What bounds it: latency on small grids (the trip to L2 for the fields, the
+// filter's and the advance's barriers), instruction issue on large ones (96 us
+// at 2048^2 against 52 for its 84 bytes a cell).  The separate launches took,
+// filter included where there is one: 32x24 cells, 3 + 3 passes, 37 us a step
+// (12.7 here, timed with events around the phase); 512^2, 2 + 2, 45 (16.7);
+// 1021x517, 1 + 1 and external fields, 51 (27); wakefield 2000x256, 4 + 0, 45
+// (23); 2048^2, 2 + 2, 109 (96).  5 CTAs a multiprocessor: 4 took 101 at
+// 2048^2, 6 were slower on small grids.
+// ---------------------------------------------------------------------------
+template <int NY>
+__global__ void __launch_bounds__(256, 5) k_fields(const __grid_constant__ CUtensorMap tm_eb,
+                                                   const __grid_constant__ CUtensorMap tm_j, const float *Jraw,
+                                                   float *Jout, float *Jnext, float *EBout,
+                                                   const __grid_constant__ ExtField ext, Grid G, YeeConst Y,
+                                                   const __grid_constant__ SmoothPasses PX,
+                                                   const __grid_constant__ SmoothPasses PY, int *err, double *epart,
+                                                   const __grid_constant__ ZeroWords zero) {
+  constexpr int EPL = kYeeBW * kYeeBH;
+  constexpr int W = kFieldBW, H = kFieldBH, PL = W * H;
+  __shared__ __align__(128) float sEB[6 * EPL];
+  __shared__ __align__(128) float sJ[3 * PL];
+  __shared__ float sg[2][3][W];  // the folded, unfiltered y guard rows -1 and ny (edge tiles)
+  __shared__ __align__(8) uint64_t bar;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < zero.n) *zero.p[threadIdx.x] = 0;
+  const int bx0 = blockIdx.x * kYeeOX, by0 = blockIdx.y * kYeeOY;
+  const int nx = G.nx, ny = G.ny, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jx0 = bx0 - 4, jy0 = by0 - 4;  // buffer coordinates of sJ (0, 0)
+  // columns nx .. nx + 2 and 0 .. 2 (periodic x), rows ny .. ny + 2 and 0 .. 2
+  // are folded; a box clear of them is taken as it lies
+  const bool inner = jx0 >= (Y.mw ? 0 : 3) && jx0 + W <= (Y.mw ? nx + 3 : nx) && jy0 >= 3 && jy0 + H <= ny;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+    mbar_expect_tx(&bar, (6 * EPL + (inner ? 3 * PL : 0)) * 4);
+    tma_load_3d(sEB, &tm_eb, bx0 - 4, by0 - 1, 0, &bar);
+    if (inner) tma_load_3d(sJ, &tm_j, jx0, jy0, 0, &bar);
   }
-  __syncthreads();
-  // E1 on buffer cells [bx0, bx0+OX] x [by0, by0+OY]
-  {
-    constexpr int W = kYeeOX + 1, H = kYeeOY + 1;
-    for (int k = threadIdx.x; k < W * H; k += blockDim.x) {
-      const int bx = bx0 + k % W, by = by0 + k / W;
-      if (bx < 1 || bx > nx + 2 || by < 1 || by > ny + 2) continue;
-      const int s = (by - oy) * BW + (bx - ox);
-      Ex[s] += (+Y.cye * (Bz[s] - Bz[s - BW])) - Y.dt * Jx[s];
-      Ey[s] += (-Y.cxe * (Bz[s] - Bz[s - 1])) - Y.dt * Jy[s];
-      Ez[s] += (+Y.cxe * (By[s] - By[s - 1]) - Y.cye * (Bx[s] - Bx[s - BW])) - Y.dt * Jz[s];
-    }
-  }
-  __syncthreads();
-  // B2 on the output tile, then store E1 and B2; with epart, the squares of
-  // the interior cells' new values are summed for the field energy
-  float se[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int k = threadIdx.x; k < kYeeOX * kYeeOY; k += blockDim.x) {
-    const int bx = bx0 + k % kYeeOX, by = by0 + k / kYeeOX;
-    if (bx >= nx + 3 || by >= ny + 3) continue;
-    const int s = (by - oy) * BW + (bx - ox);
-    float bxv = Bx[s], byv = By[s], bzv = Bz[s];
-    if (bx <= nx + 1 && by <= ny + 1) {
-      bxv += (-Y.cyb * (Ez[s + BW] - Ez[s]));
-      byv += (Y.cxb * (Ez[s + 1] - Ez[s]));
-      bzv += (-Y.cxb * (Ey[s + 1] - Ey[s]) + Y.cyb * (Ex[s + BW] - Ex[s]));
-    }
-    if (jzero) {  // the raw deposit buffer, dead once filtered: cleared for the next step
-      jzero[gidx(G, 0, bx, by)] = 0.f;
-      jzero[gidx(G, 1, bx, by)] = 0.f;
-      jzero[gidx(G, 2, bx, by)] = 0.f;
-    }
-    if (gc) {
-      // guard cells as emf_update_gc leaves them (emf.c:573-637): a guard
-      // cell is not stored here; the cell it copies stores its value there
-      // too (periodic in x unless the window moves, always in y)
-      const bool gxc = !Y.mw && (bx == 0 || bx > nx), gyc = (by == 0 || by > ny);
-      if (gxc || gyc) continue;
-      const int xm = Y.mw ? -1 : (bx == nx ? 0 : (bx <= 2 ? nx + bx : -1));
-      const int ym = by == ny ? 0 : (by <= 2 ? ny + by : -1);
-      put_mirrored(EBout, G, 0, bx, by, xm, ym, Ex[s]);
-      put_mirrored(EBout, G, 1, bx, by, xm, ym, Ey[s]);
-      put_mirrored(EBout, G, 2, bx, by, xm, ym, Ez[s]);
-      put_mirrored(EBout, G, 3, bx, by, xm, ym, bxv);
-      put_mirrored(EBout, G, 4, bx, by, xm, ym, byv);
-      put_mirrored(EBout, G, 5, bx, by, xm, ym, bzv);
-    } else {
-      EBout[gidx(G, 0, bx, by)] = Ex[s];
-      EBout[gidx(G, 1, bx, by)] = Ey[s];
-      EBout[gidx(G, 2, bx, by)] = Ez[s];
-      EBout[gidx(G, 3, bx, by)] = bxv;
-      EBout[gidx(G, 4, bx, by)] = byv;
-      EBout[gidx(G, 5, bx, by)] = bzv;
-    }
-    if (epart && bx >= 1 && bx <= nx && by >= 1 && by <= ny) {
-      se[0] += Ex[s] * Ex[s];
-      se[1] += Ey[s] * Ey[s];
-      se[2] += Ez[s] * Ez[s];
-      se[3] += bxv * bxv;
-      se[4] += byv * byv;
-      se[5] += bzv * bzv;
-    }
-  }
-  if (epart) {
-    // warp sums in float (64 cells a warp), then doubles across the warps
-    __shared__ double swe[6][8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!inner) {
+    // a lane takes columns lane and lane + 32, a warp every eighth row
+    auto col_of = [&](int bx) {  // the column whose value bx shows (-1: outside a moving window's buffer)
+      if (Y.mw) return (bx >= 0 && bx < nx + 3) ? bx : -1;
+      while (bx < 1) bx += nx;
+      while (bx > nx) bx -= nx;
+      return bx;
+    };
+    auto row_of = [&](int by) {
+      while (by < 1) by += ny;
+      while (by > ny) by -= ny;
+      return by;
+    };
+    // the column that is added to column c of a pair (c first, or second for
+    // column nx, whose pair is column 0), and the same for the rows
+    auto pair_of = [&](int c, int n) { return c <= 2 ? n + c : (c == n ? 0 : -1); };
+    // Only the rows and columns that the passes reach.  All first addends are
+    // loaded before any is used, then all second ones: three trips to L2, not
+    // one a value.
+    const int ra = 4 - NY, rb = 4 + kYeeOY + NY, ca = 4 - PX.n, cb = 4 + kYeeOX + PX.n;
+    constexpr int Q = (H + 7) / 8;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int cx = lane + 32 * h;
+      const bool in = cx >= ca && cx <= cb;
+      const int c = in ? col_of(jx0 + cx) : -1, c2 = (Y.mw || c < 0) ? -1 : pair_of(c, nx);
+      float v[Q][3];
+      int r[Q];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      float v = se[c];
+      for (int q = 0; q < Q; ++q) {
+        const int ry = warp + 8 * q;
+        r[q] = (ry >= ra && ry <= rb) ? row_of(jy0 + ry) : 0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) swe[c][warp] = v;
+        for (int comp = 0; comp < 3; ++comp)
+          v[q][comp] = (r[q] > 0 && c >= 0) ? Jraw[comp * G.plane + (size_t)r[q] * G.pitch + c] : 0.f;
+      }
+      // a warp's share of the y guard rows: row ny (warps 0 .. 2) or 1, one component
+      const int ge = warp / 3, gc = warp % 3, gr = ge ? 1 : ny, gr2 = ge ? ny + 1 : 0;
+      const bool guard = NY > 0 && warp < 6 && c >= 0;
+      auto at = [&](int comp, int row, int col) { return Jraw[comp * G.plane + (size_t)row * G.pitch + col]; };
+      float ga = 0.f, gb = 0.f, gA = 0.f, gB = 0.f;
+      if (guard) {
+        ga = at(gc, gr, c);
+        gA = at(gc, gr2, c);
+        if (c2 >= 0) gb = at(gc, gr, c2), gB = at(gc, gr2, c2);
+      }
+      if (c2 >= 0) {
+        float w[Q][3];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int comp = 0; comp < 3; ++comp) w[q][comp] = r[q] > 0 ? at(comp, r[q], c2) : 0.f;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int comp = 0; comp < 3; ++comp)
+            v[q][comp] = c2 == 0 ? w[q][comp] + v[q][comp] : v[q][comp] + w[q][comp];
+        ga = c2 == 0 ? gb + ga : ga + gb;
+        gA = c2 == 0 ? gB + gA : gA + gB;
+      }
+      const float g = ge ? ga + gA : gA + ga;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int r2 = r[q] > 0 ? pair_of(r[q], ny) : -1;
+        if (r2 < 0 || c < 0) continue;
+        float w[3], x[3];
+#pragma unroll
+        for (int comp = 0; comp < 3; ++comp) {
+          w[comp] = at(comp, r2, c);
+          x[comp] = c2 >= 0 ? at(comp, r2, c2) : 0.f;
+        }
+#pragma unroll
+        for (int comp = 0; comp < 3; ++comp) {
+          if (c2 >= 0) w[comp] = c2 == 0 ? x[comp] + w[comp] : w[comp] + x[comp];
+          v[q][comp] = r2 == 0 ? w[comp] + v[q][comp] : v[q][comp] + w[comp];
+        }
+      }
+      if (cx < W) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          if (warp + 8 * q < H)
+#pragma unroll
+            for (int comp = 0; comp < 3; ++comp) sJ[comp * PL + (warp + 8 * q) * W + cx] = v[q][comp];
+        if (NY > 0 && warp < 6) sg[ge][gc][cx] = g;
+      }
+    }
+  }
+  __syncthreads();  // the barrier is set up, the gathered values are there
+  if (!mbar_wait_bounded(&bar, 0)) {
+    if (threadIdx.x == 0) atomicOr(err, ERR_TIMEOUT);
+    if (!mbar_wait_bounded(&bar, 0)) return;  // second bounded wait for the copies in flight
+  }
+  if (PX.n > 0) {
+    // columns whose value is filtered: all (periodic), or the interior ones
+    const int cx = 2 * lane, bx = jx0 + cx;
+    const bool f0 = !Y.mw || (bx >= 1 && bx <= nx), f1 = !Y.mw || (bx + 1 >= 1 && bx + 1 <= nx);
+    for (int ry = warp; ry < H; ry += 8) {
+      // without y passes the y guard rows keep their values
+      if (NY == 0 && (jy0 + ry < 1 || jy0 + ry > ny)) continue;
+      float2 v[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        v[c] = cx < W ? *reinterpret_cast<const float2 *>(sJ + c * PL + ry * W + cx) : make_float2(0.f, 0.f);
+      for (int p = 0; p < PX.n; ++p) {
+        const float sa = PX.sa[p], sb = PX.sb[p];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float l = __shfl_up_sync(0xffffffffu, v[c].y, 1), u = __shfl_down_sync(0xffffffffu, v[c].x, 1);
+          const float a = f3pt(sa, sb, l, v[c].x, v[c].y), b = f3pt(sa, sb, v[c].x, v[c].y, u);
+          v[c].x = f0 ? a : v[c].x;
+          v[c].y = f1 ? b : v[c].y;
+        }
+      }
+      if (cx < W)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *reinterpret_cast<float2 *>(sJ + c * PL + ry * W + cx) = v[c];
     }
     __syncthreads();
-    if (threadIdx.x < 6) {
-      double v = 0;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += swe[threadIdx.x][w];
-      epart[(blockIdx.y * gridDim.x + blockIdx.x) * 6 + threadIdx.x] = v;
-    }
   }
+  if constexpr (NY > 0) {
+    // rows by0 .. by0 + 16 of columns bx0 .. bx0 + 32: 9 rows and 8 a thread
+    constexpr int OW = kYeeOX + 1, R = (kYeeOY + 2) / 2;
+    float res[R];
+    const int col = threadIdx.x % OW, comp = (threadIdx.x / OW) % 3, half = threadIdx.x / (3 * OW);
+    const int bx = bx0 + col, rows = half ? kYeeOY + 1 - R : R;
+    const bool act = half < 2, filt = act && bx >= 1 && bx <= nx;
+    float *c0 = sJ + comp * PL + (4 + half * R) * W + 4 + col;
+    if (filt) {
+      float s0[NY], s1[NY];  // each pass's last two rows
+      const float glo = inner ? 0.f : sg[0][comp][4 + col], ghi = inner ? 0.f : sg[1][comp][4 + col];
+      int j = (by0 + half * R - 1 - NY) % ny;  // interior row of the first row walked
+      if (j < 0) j += ny;
+#pragma unroll
+      for (int rr = 0; rr < R + 2 * NY; ++rr) {
+        if (rr < rows + 2 * NY) {
+          float v = c0[(rr - NY) * W];
+          const int jm = (j == 0) ? ny - 1 : j - 1;  // interior row of the previous row
+#pragma unroll
+          for (int p = 0; p < NY; ++p) {
+            if (rr < 2 * p) break;
+            float e = 0.f;
+            if (rr >= 2 * p + 2) {
+              float lo = s0[p], hi = v;
+              if (p == 0 && !inner) {  // next to a y guard row: as stored
+                lo = (jm == 0) ? glo : lo;
+                hi = (jm == ny - 1) ? ghi : hi;
+              }
+              e = f3pt(PY.sa[p], PY.sb[p], lo, s1[p], hi);
+            }
+            s0[p] = s1[p];
+            s1[p] = v;
+            v = e;
+          }
+          if (rr >= 2 * NY) res[rr - 2 * NY] = v;
+          j = (j + 1 == ny) ? 0 : j + 1;
+        }
+      }
+    }
+    __syncthreads();
+    if (filt)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r < rows) c0[r * W] = res[r];
+    __syncthreads();
+  }
+  if (bx0 + lane < nx + 3)
+    for (int r = warp; r < kYeeOY; r += 8)
+      if (by0 + r < ny + 3) {
+        float *o = Jout + (size_t)(by0 + r) * G.pitch + bx0 + lane;
+        const float *v = sJ + (4 + r) * W + 4 + lane;
+        o[0] = v[0];
+        o[G.plane] = v[PL];
+        o[2 * G.plane] = v[2 * PL];
+      }
+  yee_tile(sEB, YeeCurrent{sJ + 4 * W + 4, W, PL}, bx0, by0, EBout, ext, G, Y, epart, Jnext, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -866,6 +1178,24 @@ cudaError_t launch_smooth(const float *Jin, float *Jout, const Grid &G, const Sm
 #undef ZC_SMOOTH_ROW
 #undef ZC_SMOOTH
   k_smooth<-1, -1><<<grid, block, 0, st>>>(Jin, Jout, G, PX, PY, mw);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fields(const CUtensorMap *tm_eb, const CUtensorMap *tm_j, const float *Jraw, float *Jout,
+                          float *Jnext, float *EBout, const ExtField &ext, const Grid &G, const YeeConst &Y,
+                          const SmoothPasses &PX, const SmoothPasses &PY, int *err, double *epart,
+                          const ZeroWords &zero, cudaStream_t st) {
+  if (!fields_together(G, PX, PY)) return cudaErrorInvalidValue;
+  dim3 grid((G.nx + 3 + kYeeOX - 1) / kYeeOX, (G.ny + 3 + kYeeOY - 1) / kYeeOY);
+#define ZC_FIELDS(N)                                                                                              \
+  if (PY.n == N)                                                                                                  \
+    k_fields<N><<<grid, 256, 0, st>>>(*tm_eb, *tm_j, Jraw, Jout, Jnext, EBout, ext, G, Y, PX, PY, err, epart, zero);
+  ZC_FIELDS(0)
+  ZC_FIELDS(1)
+  ZC_FIELDS(2)
+  ZC_FIELDS(3)
+  ZC_FIELDS(4)
+#undef ZC_FIELDS
   return cudaGetLastError();
 }
 

@@ -267,6 +267,24 @@ struct ZeroWords {
 cudaError_t launch_yee(const CUtensorMap *tm_eb, const CUtensorMap *tm_j, float *EBout, const Grid &G,
                        const YeeConst &Y, int *err, double *epart, float *jzero, bool gc, const ZeroWords &zero,
                        cudaStream_t st);
+// external fields added to what the particles see: types (0 none, 1 uniform,
+// 2 a grid), values per component; out null: none
+struct ExtField {
+  float *out = nullptr;
+  const float *E = nullptr, *B = nullptr;
+  int Et = 0, Bt = 0;
+  float v0[6] = {};
+};
+// fold of the raw deposits Jraw, filter into Jout, Yee advance, external
+// fields and clearing of the next raw buffer, in one launch (periodic guard
+// cells included); tm_j: a box of kFieldBW x kFieldBH x 3 over Jraw
+inline bool fields_together(const Grid &G, const SmoothPasses &PX, const SmoothPasses &PY) {
+  return G.nx >= 6 && G.ny >= 6 && PX.n <= 4 && PY.n <= 4;  // a 4-cell halo, disjoint folds
+}
+cudaError_t launch_fields(const CUtensorMap *tm_eb, const CUtensorMap *tm_j, const float *Jraw, float *Jout,
+                          float *Jnext, float *EBout, const ExtField &ext, const Grid &G, const YeeConst &Y,
+                          const SmoothPasses &PX, const SmoothPasses &PY, int *err, double *epart,
+                          const ZeroWords &zero, cudaStream_t st);
 int yee_blocks(const Grid &G);
 cudaError_t launch_emf_gc(float *EB, const Grid &G, int mw, cudaStream_t st);
 cudaError_t launch_ext_add(const float *EB, float *EBp, const float *extE, const float *extB, int Etype, int Btype,
@@ -328,5 +346,7 @@ void set_error_message(const char *msg);
 constexpr int kYeeOX = 32, kYeeOY = 16;   // Yee output tile (buffer cells)
 constexpr int kYeeBW = kYeeOX + 8;        // TMA box: 4 columns of halo each side
 constexpr int kYeeBH = kYeeOY + 3;
+constexpr int kFieldBW = kYeeOX + 12;     // raw current of a tile: 4 cells before, 8 and 5 after
+constexpr int kFieldBH = kYeeOY + 9;
 
 }  // namespace zc
