@@ -195,6 +195,8 @@ struct zc_sim {
   double *d_part = nullptr, *d_emf = nullptr;
   int energy_blocks = 0;
   float *stage = nullptr;         // AoS staging for grids
+  float *dens = nullptr;          // charge and phase-space densities (grown, kept)
+  size_t dens_n = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0;
   zc_inject_fn inj = nullptr;
@@ -1671,6 +1673,7 @@ zc_status zc_sim_destroy(zc_sim *s) {
   dfree(s->d_part);
   dfree(s->d_emf);
   dfree(s->stage);
+  dfree(s->dens);
   if (s->h_pinned) cudaFreeHost(s->h_pinned);
   if (s->h_inj) cudaFreeHost(s->h_inj);
   for (auto e : s->ev_pool) cudaEventDestroy(e);
@@ -2258,6 +2261,18 @@ zc_status zc_energy_async(zc_sim *s, double emf[6], double *kin) {
   return queue_energy(s, emf, kin);
 }
 
+// room for a density of n values, kept for the next one
+static zc_status density_buffer(zc_sim *s, size_t n, float **d) {
+  if (n > s->dens_n) {
+    dfree(s->dens);  // (the calls that use it wait for the device)
+    s->dens_n = 0;
+    TRY(dalloc(&s->dens, n));
+    s->dens_n = n;
+  }
+  *d = s->dens;
+  return ZC_OK;
+}
+
 zc_status zc_species_charge(zc_sim *s, int k, float *charge) {
   TRY(check_species(s, k));
   if (!charge) return fail(ZC_EINVAL, "null argument");
@@ -2266,13 +2281,12 @@ zc_status zc_species_charge(zc_sim *s, int k, float *charge) {
   TRY(settle(s, p));
   const size_t n = (size_t)(s->nx + 1) * (s->ny + 1);
   float *d = nullptr;
-  TRY(dalloc(&d, n));
+  TRY(density_buffer(s, n, &d));
   CK(cudaMemcpyAsync(d, charge, n * sizeof(float), cudaMemcpyHostToDevice, s->st));
   CK(launch_charge(p.buf[p.cur], p.d_off, p.d_np, s->ntiles, p.spill[p.spill_cur], p.d_spill_cnt + p.spill_cur,
                    p.spill_cap, d, s->nx, s->ny, p.q, s->mw, s->st));
   CK(cudaMemcpyAsync(charge, d, n * sizeof(float), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
-  dfree(d);
   return ZC_OK;
 }
 
@@ -2301,13 +2315,12 @@ zc_status zc_species_phasespace(zc_sim *s, int k, int quant1, int quant2, const 
   P.q = p.q;
   const size_t n = (size_t)pha_nx[0] * pha_nx[1];
   float *d = nullptr;
-  TRY(dalloc(&d, n));
+  TRY(density_buffer(s, n, &d));
   CK(cudaMemcpyAsync(d, buf, n * sizeof(float), cudaMemcpyHostToDevice, s->st));
   CK(launch_phasespace(p.buf[p.cur], p.d_off, p.d_np, s->ntiles, p.spill[p.spill_cur], p.d_spill_cnt + p.spill_cur,
-                       p.spill_cap, d, P, s->st));
+                       p.spill_cap, d, P, layout(s), s->st));
   CK(cudaMemcpyAsync(buf, d, n * sizeof(float), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
-  dfree(d);
   return ZC_OK;
 }
 

@@ -217,7 +217,8 @@ struct PhaConst {
   float x1min, x2min, rdx1, rdx2, dx, dy, q;
 };
 cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
-                              const int *spill_cnt, int spill_cap, float *pha, const PhaConst &P, cudaStream_t st);
+                              const int *spill_cnt, int spill_cap, float *pha, const PhaConst &P,
+                              const LayoutConst &L, cudaStream_t st);
 cudaError_t launch_charge(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
                           const int *spill_cnt, int spill_cap, float *rho, int nx, int ny, float q, int mw,
                           cudaStream_t st);
