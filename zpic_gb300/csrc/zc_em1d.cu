@@ -14,7 +14,9 @@
 // lanes of a warp share cells; E, B, J are the reference's float3 buffers
 // (one lower and two upper guard cells).
 //
-// A step is two kernels.  The push runs one particle per lane: the current
+// A run of steps up to the next cell sort is one cooperative launch (k1_run)
+// where the particles fit the multiprocessors' shared memory; else, and when
+// kernels are timed one by one, a step is two kernels.  The push runs one particle per lane: the current
 // of a motion that stays in its cell is summed over the lanes of the cell
 // (segmented warp reduction) and added to J with one float reduction per
 // node (performed in L2); cell-crossing motions add their two segments
@@ -52,7 +54,7 @@ constexpr int GC0 = 1, GC1 = 2;  // guard cells (em1d/emf.c:59)
 // the fields kernel sums them in a fixed order
 constexpr int kJCopies = 8;
 constexpr int kFieldUnroll = 2;  // grid elements per thread per load round of the fields kernel
-enum { ERR1_ESCAPE = 1, ERR1_OVERFLOW = 2 };
+enum { ERR1_ESCAPE = 1, ERR1_OVERFLOW = 2, ERR1_TIMEOUT = 4 };
 
 struct Parts {
   int *ix;
@@ -151,6 +153,133 @@ __device__ __forceinline__ void run_sum(Seg1 &v, int run_last, unsigned maxlen) 
 }
 
 
+// one particle's gather, push and move (momenta in place)
+struct Move1 {
+  float kin, dx, x1, qvy, qvz;
+  int di;
+};
+__device__ __forceinline__ Move1 push_lane(const float *E, const float *B, int ix, float x, float &ux, float &uy,
+                                           float &uz, const Push1 &C) {
+  Move1 m;
+  // staggered linear gather (particles.c:864-894)
+  const int ih = ix + ((x < 0.5f) ? -1 : 0);
+  const float w1h = x + ((x < 0.5f) ? 0.5f : -0.5f);
+  float ex = lerp1(E, ih, 0, w1h), ey = lerp1(E, ix, 1, x), ez = lerp1(E, ix, 2, x);
+  float bx = lerp1(B, ix, 0, x), by = lerp1(B, ih, 1, w1h), bz = lerp1(B, ih, 2, w1h);
+  // Boris (particles.c:960-1010)
+  ex *= C.tem;
+  ey *= C.tem;
+  ez *= C.tem;
+  float utx = ux + ex, uty = uy + ey, utz = uz + ez;
+  const float u2 = utx * utx + uty * uty + utz * utz;
+  const float gamma = sqrtf(1 + u2);
+  m.kin = u2 / (1 + gamma);
+  const float gtem = C.tem / gamma;
+  bx *= gtem;
+  by *= gtem;
+  bz *= gtem;
+  const float otsq = 2.0f / (1.0f + bx * bx + by * by + bz * bz);
+  ux = utx + uty * bz - utz * by;
+  uy = uty + utz * bx - utx * bz;
+  uz = utz + utx * by - uty * bx;
+  bx *= otsq;
+  by *= otsq;
+  bz *= otsq;
+  utx += uy * bz - uz * by;
+  uty += uz * bx - ux * bz;
+  utz += ux * by - uy * bx;
+  ux = utx + ex;
+  uy = uty + ey;
+  uz = utz + ez;
+  // move (particles.c:1012-1022)
+  const float rg = 1.0f / sqrtf(1.0f + ux * ux + uy * uy + uz * uz);
+  m.dx = C.dt_dx * rg * ux;
+  m.x1 = x + m.dx;
+  m.di = (m.x1 >= 1.0f) - (m.x1 < 0.0f);
+  m.x1 -= m.di;
+  m.qvy = C.q * uy * rg;
+  m.qvz = C.q * uz * rg;
+  return m;
+}
+
+// Sums of 16 values over the warp's 32 lanes: every exchange halves the
+// values a lane holds (16 shuffles in all, where 16 sums of their own take
+// 80), until lane l has half of the sum of value order(l); one more exchange
+// completes it.
+__device__ __forceinline__ float sum16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int h = 8, bit = 16; h >= 1; h >>= 1, bit >>= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const float give = up ? v[q] : v[q + h], keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// the current of a warp's particles, one a lane
+__device__ __forceinline__ void deposit_warp(float *J, bool valid, int ix, float x, const Move1 &m, const Push1 &C) {
+  const int lane = threadIdx.x & 31, di = m.di;
+  const float dx = m.dx, qvy = m.qvy, qvz = m.qvz;
+  // deposit (dep_current_zamb): qvy, qvz halved, split at the cell edge.
+  // a: the motion inside cell ix (all of it, or its part up to the edge);
+  // b: for a crossing, the part inside cell ix + di
+  const float hy = qvy / 2.0f, hz = qvz / 2.0f;
+  const bool split = valid && di != 0;
+  Seg1 a, b = Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
+  if (split) {
+    const int ib = (di == 1);
+    const float delta = (x + dx - ib) / dx;
+    b = seg_current(1 - ib, (x + dx) - di, dx * delta, hy * delta, hz * delta, C.qnx);
+    a = seg_current(x, (float)ib, dx * (1.0f - delta), hy * (1.0f - delta), hz * (1.0f - delta), C.qnx);
+  } else {
+    a = seg_current(x, x + dx, dx, hy, hz, C.qnx);
+  }
+  // the lanes of a cell are contiguous (cell order): each part is summed
+  // over the lanes of the cell and one lane per cell adds the sums, a to
+  // cell ix, b to ix + 1 or ix - 1 (one sum per direction)
+  {
+    const int ix0 = __shfl_sync(0xffffffffu, ix, 0);  // (by every lane, valid or not)
+    if (__all_sync(0xffffffffu, valid && ix == ix0)) {
+      // one cell (the usual case: 128 particles a cell): the sums of the part
+      // inside it and of the parts past its two edges, 5 values each; the
+      // value of lane pair p goes to its node with one reduction a lane
+      const float zu = di == 1 ? 1.f : 0.f, zd = di == -1 ? 1.f : 0.f;
+      float v[16] = {a.jx, a.y0, a.y1, a.z0, a.z1, zu * b.jx, zu * b.y0, zu * b.y1, zu * b.z0, zu * b.z1,
+                     zd * b.jx, zd * b.y0, zd * b.y1, zd * b.z0, zd * b.z1, 0.f};
+      const float sum = sum16(v, lane);
+      const int q = lane >> 1, part = q / 5, e = q % 5;  // (order: value q in lanes 2 q, 2 q + 1)
+      const int node = ix + (part == 1 ? 1 : (part == 2 ? -1 : 0)) + ((e == 2 || e == 4) ? 1 : 0);
+      if ((lane & 1) == 0 && q < 15 && sum != 0.f) red(J, node, e == 0 ? 0 : (e <= 2 ? 1 : 2), sum);
+      return;
+    }
+    const int key = valid ? ix : -1 - lane;
+    const int knext = __shfl_down_sync(0xffffffffu, key, 1);
+    const int kprev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned lastmask = __ballot_sync(0xffffffffu, lane == 31 || knext != key);
+    const int run_last = __ffs(lastmask & (0xffffffffu << lane)) - 1;
+    const unsigned maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(run_last - lane + 1));
+    const bool head = valid && (lane == 0 || kprev != key);
+    const unsigned up = __ballot_sync(0xffffffffu, split && di == 1);
+    const unsigned down = __ballot_sync(0xffffffffu, split && di == -1);
+    Seg1 sa = valid ? a : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
+    run_sum(sa, run_last, maxlen);
+    if (head) add_seg(J, ix, sa);
+    if (up) {
+      Seg1 sb = (di == 1) ? b : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
+      run_sum(sb, run_last, maxlen);
+      if (head) add_seg(J, ix + 1, sb);
+    }
+    if (down) {
+      Seg1 sb = (di == -1) ? b : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
+      run_sum(sb, run_last, maxlen);
+      if (head) add_seg(J, ix - 1, sb);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // push + deposit, one particle per lane, warps over consecutive particles;
 // boundaries, compaction by append, and (last CTA) injection + bookkeeping
@@ -188,103 +317,28 @@ __global__ void __launch_bounds__(256, 4) k1_push(Parts b0, Parts b1, SpecState1
         ix = min(max(ix, 0), C.nx - 1);
       }
     }
-    // staggered linear gather (particles.c:864-894)
-    const int ih = ix + ((x < 0.5f) ? -1 : 0);
-    const float w1h = x + ((x < 0.5f) ? 0.5f : -0.5f);
-    float ex = lerp1(E, ih, 0, w1h), ey = lerp1(E, ix, 1, x), ez = lerp1(E, ix, 2, x);
-    float bx = lerp1(B, ix, 0, x), by = lerp1(B, ih, 1, w1h), bz = lerp1(B, ih, 2, w1h);
-    // Boris (particles.c:960-1010)
-    ex *= C.tem;
-    ey *= C.tem;
-    ez *= C.tem;
-    float utx = ux + ex, uty = uy + ey, utz = uz + ez;
-    const float u2 = utx * utx + uty * uty + utz * utz;
-    const float gamma = sqrtf(1 + u2);
-    const float kin = u2 / (1 + gamma);
-    const float gtem = C.tem / gamma;
-    bx *= gtem;
-    by *= gtem;
-    bz *= gtem;
-    const float otsq = 2.0f / (1.0f + bx * bx + by * by + bz * bz);
-    ux = utx + uty * bz - utz * by;
-    uy = uty + utz * bx - utx * bz;
-    uz = utz + utx * by - uty * bx;
-    bx *= otsq;
-    by *= otsq;
-    bz *= otsq;
-    utx += uy * bz - uz * by;
-    uty += uz * bx - ux * bz;
-    utz += ux * by - uy * bx;
-    ux = utx + ex;
-    uy = uty + ey;
-    uz = utz + ez;
-    // move (particles.c:1012-1022)
-    const float rg = 1.0f / sqrtf(1.0f + ux * ux + uy * uy + uz * uz);
-    const float dx = C.dt_dx * rg * ux;
-    float x1 = x + dx;
-    const int di = (x1 >= 1.0f) - (x1 < 0.0f);
-    x1 -= di;
-    const float qvy = C.q * uy * rg;
-    const float qvz = C.q * uz * rg;
+    const Move1 m = push_lane(E, B, ix, x, ux, uy, uz, C);
+    const float x1 = m.x1;
+    const int di = m.di;
     if (valid) {
-      const float y = kin - kc;
+      const float y = m.kin - kc;
       const float t = ks + y;
       kc = (t - ks) - y;
       ks = t;
-      if (!(fabsf(dx) < 1.0f)) errbits |= ERR1_ESCAPE;
+      if (!(fabsf(m.dx) < 1.0f)) errbits |= ERR1_ESCAPE;
     }
-    // deposit (dep_current_zamb): qvy, qvz halved, split at the cell edge.
-    // a: the motion inside cell ix (all of it, or its part up to the edge);
-    // b: for a crossing, the part inside cell ix + di
-    const float hy = qvy / 2.0f, hz = qvz / 2.0f;
-    const bool split = valid && di != 0;
-    Seg1 a, b = Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (split) {
-      const int ib = (di == 1);
-      const float delta = (x + dx - ib) / dx;
-      b = seg_current(1 - ib, (x + dx) - di, dx * delta, hy * delta, hz * delta, C.qnx);
-      a = seg_current(x, (float)ib, dx * (1.0f - delta), hy * (1.0f - delta), hz * (1.0f - delta), C.qnx);
-    } else {
-      a = seg_current(x, x + dx, dx, hy, hz, C.qnx);
-    }
-    // the lanes of a cell are contiguous (cell order): each part is summed
-    // over the lanes of the cell and one lane per cell adds the sums, a to
-    // cell ix, b to ix + 1 or ix - 1 (one sum per direction)
-    {
-      const int key = valid ? ix : -1 - lane;
-      const int knext = __shfl_down_sync(0xffffffffu, key, 1);
-      const int kprev = __shfl_up_sync(0xffffffffu, key, 1);
-      const unsigned lastmask = __ballot_sync(0xffffffffu, lane == 31 || knext != key);
-      const int run_last = __ffs(lastmask & (0xffffffffu << lane)) - 1;
-      const unsigned maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(run_last - lane + 1));
-      const bool head = valid && (lane == 0 || kprev != key);
-      const unsigned up = __ballot_sync(0xffffffffu, split && di == 1);
-      const unsigned down = __ballot_sync(0xffffffffu, split && di == -1);
-      Seg1 sa = valid ? a : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
-      run_sum(sa, run_last, maxlen);
-      if (head) add_seg(J, ix, sa);
-      if (up) {
-        Seg1 sb = (di == 1) ? b : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
-        run_sum(sb, run_last, maxlen);
-        if (head) add_seg(J, ix + 1, sb);
-      }
-      if (down) {
-        Seg1 sb = (di == -1) ? b : Seg1{0.f, 0.f, 0.f, 0.f, 0.f};
-        run_sum(sb, run_last, maxlen);
-        if (head) add_seg(J, ix - 1, sb);
-      }
-    }
+    deposit_warp(J, valid, ix, x, m, C);
     // boundaries (particles.c:1040-1062); with open boundaries the survivors
     // are appended to the other buffer, a warp at a time
     int nix = ix + di - shift;
     if (C.open) {
       const bool live = valid && nix >= 0 && nix < C.nx;
-      const unsigned m = __ballot_sync(0xffffffffu, live);
+      const unsigned lm = __ballot_sync(0xffffffffu, live);
       int obase = 0;
-      if (lane == 0 && m) obase = atomicAdd(np_out, __popc(m));
+      if (lane == 0 && lm) obase = atomicAdd(np_out, __popc(lm));
       obase = __shfl_sync(0xffffffffu, obase, 0);
       if (live) {
-        const int o = obase + __popc(m & ((1u << lane) - 1));
+        const int o = obase + __popc(lm & ((1u << lane) - 1));
         if (o < C.cap) {
           dst.ix[o] = nix;
           dst.x[o] = x1;
@@ -492,6 +546,25 @@ __device__ __forceinline__ void periodic_gc1(float *E, float *B, int nx) {
   }
 }
 
+__device__ __forceinline__ void mur1(float *e, float *mur, int nx, float dt, float dx) {
+  // first-order Mur (mur_abc, emf.c:379-415); mur = fld[2][3], tmp[2][3]
+  float *fld = mur, *tmp = mur + 6;
+  const float S = (dt - dx) / (dt + dx);
+  const int lo = (0 + GC0) * 3, hi = (nx - 1 + GC0) * 3;
+  fld[1] = tmp[1] + S * (e[lo + 1] - fld[1]);
+  fld[2] = tmp[2] + S * (e[lo + 2] - fld[2]);
+  e[(-1 + GC0) * 3 + 1] = fld[1];
+  e[(-1 + GC0) * 3 + 2] = fld[2];
+  tmp[1] = e[lo + 1];
+  tmp[2] = e[lo + 2];
+  fld[4] = tmp[4] + S * (e[hi + 1] - fld[4]);
+  fld[5] = tmp[5] + S * (e[hi + 2] - fld[5]);
+  e[(nx + GC0) * 3 + 1] = fld[4];
+  e[(nx + GC0) * 3 + 2] = fld[5];
+  tmp[4] = e[hi + 1];
+  tmp[5] = e[hi + 2];
+}
+
 // SM: the four grids (two current buffers, E, B) live in shared memory for
 // the whole kernel, else the kernel works on the global buffers (Jdep and
 // Jout then serve as the filter's two buffers).  Jdep (kJCopies copies,
@@ -606,22 +679,7 @@ __global__ void __launch_bounds__(1024) k1_fields(float *E, float *B, float *Jde
   yee_e1(e, b, J, nx, M.dt, M.dt / M.dx);
   __syncthreads();
   if (M.bc == 2 && threadIdx.x == 0) {
-    // first-order Mur (mur_abc, emf.c:379-415); mur = fld[2][3], tmp[2][3]
-    float *fld = mur, *tmp = mur + 6;
-    const float S = (M.dt - M.dx) / (M.dt + M.dx);
-    const int lo = (0 + GC0) * 3, hi = (nx - 1 + GC0) * 3;
-    fld[1] = tmp[1] + S * (e[lo + 1] - fld[1]);
-    fld[2] = tmp[2] + S * (e[lo + 2] - fld[2]);
-    e[(-1 + GC0) * 3 + 1] = fld[1];
-    e[(-1 + GC0) * 3 + 2] = fld[2];
-    tmp[1] = e[lo + 1];
-    tmp[2] = e[lo + 2];
-    fld[4] = tmp[4] + S * (e[hi + 1] - fld[4]);
-    fld[5] = tmp[5] + S * (e[hi + 2] - fld[5]);
-    e[(nx + GC0) * 3 + 1] = fld[4];
-    e[(nx + GC0) * 3 + 2] = fld[5];
-    tmp[4] = e[hi + 1];
-    tmp[5] = e[hi + 2];
+    mur1(e, mur, nx, M.dt, M.dx);
   }
   __syncthreads();
   yee_b1(e, b, nx, hdt / M.dx);
@@ -665,6 +723,401 @@ __global__ void __launch_bounds__(1024) k1_fields(float *E, float *B, float *Jde
   }
 }
 
+// ---------------------------------------------------------------------------
+// Several steps in one launch: a cooperative grid that stays on the GPU, one
+// grid-wide barrier a step.  A step of the two kernels above takes 31 us (13
+// for the push, 9 for one CTA's fields, the rest between launches) for work
+// that fits the chip; nothing in it is bound by bandwidth.  Here
+//   - every CTA keeps its share of the particles in shared memory for all the
+//     steps (a particle that leaves the grid leaves a hole);
+//   - every CTA keeps E and B there too and advances them by itself, all CTAs
+//     alike: after the barrier each reads the deposited current (from L2) and
+//     makes the filter and the field advance of a few thousand cells, which is
+//     cheaper than a second barrier;
+//   - the deposits go to one of three buffers in turn: the one that was read a
+//     step ago is cleared while nobody uses it;
+//   - the column that a window move uncovers goes to the CTAs in turn;
+//   - waits are bounded: past the limit an error bit is set and every CTA
+//     leaves (the others run into theirs).
+// A step takes 10.5 to 11.6 us (1000 cells, 72 to 127 thousand particles, the
+// cell sort every 16 steps included): about 2 each for the push with its
+// deposit, the barrier, the filter and the advance.  With the particles in
+// global memory, compacted every step, it took 16.
+// ---------------------------------------------------------------------------
+constexpr int kRunSpecies = 4;   // species of a run
+constexpr int kRunCopies = 4;    // copies of a deposit buffer
+constexpr int kRunThreads = 1024;
+constexpr int kBarrierPolls = 1 << 21;
+
+// floats of a grid, rounded up to whole 16-byte units
+__host__ __device__ constexpr int grid_stride1(int nx) { return ((nx + GC0 + GC1) * 3 + 3) & ~3; }
+
+struct RunSpecies1 {
+  Parts b0, b1;
+  SpecState1 *st;
+  const float *lat;          // in-cell positions of the injected lattice
+  int slots;                 // particles a CTA has room for (a multiple of kRunThreads)
+  Push1 C;
+  Inject1 I;
+};
+struct Run1 {
+  int nsp, steps, phase;     // phase: the first step's deposit buffer
+  unsigned bar0;             // the barrier's count before this launch
+  unsigned *bar;
+  float *Jrun;               // deposits [3][kRunCopies][grid_stride1]
+  float *E, *B, *Jout, *mur;
+  FieldState1 *fs;
+  int *err;
+  Fields1 M;
+  RunSpecies1 sp[kRunSpecies];
+};
+
+// all CTAs of the grid; false when the limit ran out
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    int ok = 0;
+    for (int it = 0; it < kBarrierPolls && !ok; ++it) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      ok = (int)(v - target) >= 0;
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// The injected lattice points of a window move that pass the density test
+// (spec_set_x, particles.c:250-300): [*first, *first + result).  All threads
+// of the CTA; the usual cases (all of them, none) need no look at the points.
+__device__ __forceinline__ int lattice_range(const Inject1 &I, const float *lat, int nx, int n_move, int *first) {
+  const int ic = nx - 1;
+  *first = 0;
+  if (I.type == 1) return 0;
+  if (I.type == 0) return I.ppc;
+  const float start = I.start / I.dx - n_move, end = I.end / I.dx - n_move;
+  if ((float)nx <= start) return 0;
+  if ((float)ic > start && (I.type == 2 || (float)nx < end)) return I.ppc;
+  int below = 0, inside = 0;
+  for (int q0 = 0; q0 < I.ppc; q0 += kRunThreads) {
+    const int q = q0 + (int)threadIdx.x;
+    const float pos = q < I.ppc ? lat[q] : 0.f;
+    const bool past = ic + pos > start;
+    below += __syncthreads_count(q < I.ppc && !past);
+    inside += __syncthreads_count(q < I.ppc && past && (I.type == 2 || ic + pos < end));
+  }
+  *first = below;
+  return inside;
+}
+
+__global__ void __launch_bounds__(kRunThreads, 1) k1_run(const __grid_constant__ Run1 R) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ double sred[kRunThreads / 32];
+  __shared__ int s_n[kRunThreads / 32], s_at;
+  __shared__ float s_mur[12];
+  // per species: slots in use (holes among them), first particle, the buffer
+  // that holds them, counters, particles pushed
+  __shared__ int s_used[kRunSpecies], s_i0[kRunSpecies], s_cur[kRunSpecies], s_iter[kRunSpecies], s_move[kRunSpecies];
+  __shared__ unsigned s_pushed[kRunSpecies];
+  const Fields1 &M = R.M;
+  const int nx = M.nx, nf = grid_stride1(nx), nv = (nx + GC0 + GC1) * 3;  // (values past nv: unused)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int oe = 0, ob = nf, oj = 2 * nf, oo = 3 * nf;  // E, B, J and a second buffer
+  for (int k = tid; k < nf; k += kRunThreads) {
+    sm[oe + k] = k < nv ? R.E[k] : 0.f;
+    sm[ob + k] = k < nv ? R.B[k] : 0.f;
+  }
+  if (tid < 12) s_mur[tid] = R.mur[tid];
+  // the species' particles: arrays of `slots` cells, positions and momenta,
+  // after the grids
+  if (tid < R.nsp) {
+    const RunSpecies1 &S = R.sp[tid];
+    const int cur = S.st->cur, n = S.st->np[cur], share = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int i0 = min(n, (int)blockIdx.x * share);
+    s_cur[tid] = cur;
+    s_iter[tid] = S.st->iter;
+    s_move[tid] = S.st->n_move;
+    s_i0[tid] = i0;
+    s_used[tid] = min(min(share, n - i0), S.slots);
+    s_pushed[tid] = 0;
+  }
+  __syncthreads();
+  for (int k = 0, at = 4 * nf; k < R.nsp; ++k) {
+    const RunSpecies1 &S = R.sp[k];
+    const Parts src = s_cur[k] ? S.b1 : S.b0;
+    const int i0 = s_i0[k];
+    int *ix = reinterpret_cast<int *>(sm + at);
+    float *f = sm + at + S.slots;
+    for (int q = tid; q < s_used[k]; q += kRunThreads) {
+      ix[q] = src.ix[i0 + q];
+      f[q] = src.x[i0 + q];
+      f[S.slots + q] = src.ux[i0 + q];
+      f[2 * S.slots + q] = src.uy[i0 + q];
+      f[3 * S.slots + q] = src.uz[i0 + q];
+    }
+    at += 5 * S.slots;
+  }
+  int fiter = R.fs->iter, fmove = R.fs->n_move;
+  int errbits = 0;
+  __syncthreads();
+  for (int step = 0; step < R.steps; ++step) {
+    const bool last = step == R.steps - 1;
+    const int ph = (R.phase + step) % 3;
+    float *J = R.Jrun + ((size_t)ph * kRunCopies + blockIdx.x % kRunCopies) * nf;
+#pragma unroll 1
+    for (int k = 0, at = 4 * nf; k < R.nsp; ++k) {
+      const RunSpecies1 &S = R.sp[k];
+      const Push1 &C = S.C;
+      const int iter = s_iter[k] + step + 1, moved = s_move[k], used = s_used[k];
+      const int shift = (C.mw && ((float)iter * C.dt) > (C.dx * (float)(moved + 1))) ? 1 : 0;
+      int *six = reinterpret_cast<int *>(sm + at);
+      float *f = sm + at + S.slots;
+      float ks = 0.f, kc = 0.f;
+#pragma unroll 1
+      for (int b = 0; b < used; b += kRunThreads) {
+        const int q = b + tid;
+        int ix = q < used ? six[q] : -1;
+        const bool valid = ix >= 0;
+        const unsigned vm = __ballot_sync(0xffffffffu, valid);
+        if (!vm) continue;  // a warp of holes
+        if (lane == 0) atomicAdd(&s_pushed[k], (unsigned)__popc(vm));
+        float x = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+        if (valid) {
+          x = f[q];
+          ux = f[S.slots + q];
+          uy = f[2 * S.slots + q];
+          uz = f[3 * S.slots + q];
+          if (ix >= C.nx) {
+            errbits |= ERR1_ESCAPE;
+            ix = C.nx - 1;
+          }
+        } else {
+          ix = 0;
+        }
+        const Move1 m = push_lane(sm + oe, sm + ob, ix, x, ux, uy, uz, C);
+        if (valid) {
+          const float y = m.kin - kc;
+          const float t = ks + y;
+          kc = (t - ks) - y;
+          ks = t;
+          if (!(fabsf(m.dx) < 1.0f)) errbits |= ERR1_ESCAPE;
+          int nix = ix + m.di - shift;
+          if (!C.open) nix += ((nix < 0) ? C.nx : 0) - ((nix >= C.nx) ? C.nx : 0);
+          six[q] = (nix >= 0 && nix < C.nx) ? nix : -1;
+          f[q] = m.x1;
+          f[S.slots + q] = ux;
+          f[2 * S.slots + q] = uy;
+          f[3 * S.slots + q] = uz;
+        }
+        deposit_warp(J, valid, ix, x, m, C);
+      }
+      if (last) {
+        const double e = zc::block_sum_double<kRunThreads>((double)ks - (double)kc, sred);
+        if (tid == 0 && e != 0.0) atomicAdd(&S.st->ekin_acc, e);
+      }
+      __syncthreads();  // the species' slots and counters are read
+      int n = 0;
+      // the column that the move uncovered (spec_inject_particles)
+      if (shift && blockIdx.x == (unsigned)iter % gridDim.x) {
+        int first;
+        n = lattice_range(S.I, S.lat, C.nx, moved + 1, &first);
+        for (int q = tid; q < n; q += kRunThreads) {
+          const int o = used + q;
+          if (o >= S.slots) {  // (room is sized for every column: cannot happen)
+            errbits |= ERR1_OVERFLOW;
+            continue;
+          }
+          six[o] = C.nx - 1;
+          f[o] = S.lat[first + q];
+          f[S.slots + o] = S.I.ufl[0];
+          f[2 * S.slots + o] = S.I.ufl[1];
+          f[3 * S.slots + o] = S.I.ufl[2];
+        }
+      }
+      if (tid == 0) {
+        s_move[k] = moved + shift;
+        s_used[k] = min(used + n, S.slots);
+      }
+      at += 5 * S.slots;
+    }
+    if (!grid_barrier(R.bar, R.bar0 + (unsigned)(step + 1) * gridDim.x)) {
+      if (tid == 0) atomicOr(R.err, ERR1_TIMEOUT);
+      return;
+    }
+    // the deposited current; the buffer read a step ago is cleared
+    {
+      const float *Jr = R.Jrun + (size_t)ph * kRunCopies * nf;
+      for (int k = 4 * tid; k < nf; k += 4 * kRunThreads) {
+        float4 v[kRunCopies];
+#pragma unroll
+        for (int c = 0; c < kRunCopies; ++c) v[c] = __ldcg(reinterpret_cast<const float4 *>(&Jr[c * nf + k]));
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < kRunCopies; ++c) {
+          sum.x += v[c].x;
+          sum.y += v[c].y;
+          sum.z += v[c].z;
+          sum.w += v[c].w;
+        }
+        *reinterpret_cast<float4 *>(&sm[oj + k]) = sum;
+      }
+      float *Jz = R.Jrun + (size_t)((ph + 2) % 3) * kRunCopies * nf;
+      for (int k = 4 * (blockIdx.x * kRunThreads + tid); k < kRunCopies * nf; k += 4 * gridDim.x * kRunThreads)
+        *reinterpret_cast<float4 *>(&Jz[k]) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    // current fold, filter, field advance, window shift: as k1_fields
+    if (M.cur_periodic) {
+      float *Jc = sm + oj;
+      if (tid < 9) Jc[(tid / 3 - 1 + GC0) * 3 + tid % 3] += Jc[(nx + tid / 3 - 1 + GC0) * 3 + tid % 3];
+      __syncthreads();
+      if (tid < 9) Jc[(nx + tid / 3 - 1 + GC0) * 3 + tid % 3] = Jc[(tid / 3 - 1 + GC0) * 3 + tid % 3];
+      __syncthreads();
+    }
+    for (int p = 0; p < M.S.n; ++p) {
+      const float sa = M.S.sa[p], sb = M.S.sb[p];
+      const float *Ji = sm + oj;
+      float *O = sm + oo;
+      // four values a thread; the guard cells keep theirs
+      for (int k = 4 * tid; k < nf; k += 4 * kRunThreads) {
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 A = k >= 4 ? *reinterpret_cast<const float4 *>(Ji + k - 4) : z;
+        const float4 B = *reinterpret_cast<const float4 *>(Ji + k);
+        const float4 C = k + 4 < nf ? *reinterpret_cast<const float4 *>(Ji + k + 4) : z;
+        float4 r = make_float4(sa * A.y + sb * B.x + sa * B.w, sa * A.z + sb * B.y + sa * C.x,
+                               sa * A.w + sb * B.z + sa * C.y, sa * B.x + sb * B.w + sa * C.z);
+        if (k < GC0 * 3 || k + 4 > (nx + GC0) * 3) {
+          const int lo = GC0 * 3 - k, hi = (nx + GC0) * 3 - k;  // filtered: lo <= e < hi
+          r.x = (0 >= lo && 0 < hi) ? r.x : B.x;
+          r.y = (1 >= lo && 1 < hi) ? r.y : B.y;
+          r.z = (2 >= lo && 2 < hi) ? r.z : B.z;
+          r.w = (3 >= lo && 3 < hi) ? r.w : B.w;
+        }
+        *reinterpret_cast<float4 *>(O + k) = r;
+      }
+      __syncthreads();
+      if (M.cur_periodic) {  // copies of the filtered cells
+        if (tid < 9) {
+          const int g = tid / 3, c = tid % 3, gi = (g == 0) ? -1 : nx + g - 1, from = (g == 0) ? nx - 1 : g - 1;
+          O[(gi + GC0) * 3 + c] = O[(from + GC0) * 3 + c];
+        }
+        __syncthreads();
+      }
+      const int t = oj;
+      oj = oo;
+      oo = t;
+    }
+    if (last && blockIdx.x == 0)
+      for (int k = tid; k < nv; k += kRunThreads) R.Jout[k] = sm[oj + k];
+    const float hdt = M.dt / 2.0f;
+    yee_b1(sm + oe, sm + ob, nx, hdt / M.dx);
+    __syncthreads();
+    yee_e1(sm + oe, sm + ob, sm + oj, nx, M.dt, M.dt / M.dx);
+    __syncthreads();
+    if (M.bc == 2) {
+      if (tid == 0) mur1(sm + oe, s_mur, nx, M.dt, M.dx);
+      __syncthreads();
+    }
+    yee_b1(sm + oe, sm + ob, nx, hdt / M.dx);
+    __syncthreads();
+    if (M.bc == 1) {
+      periodic_gc1(sm + oe, sm + ob, nx);
+      __syncthreads();
+    }
+    fiter += 1;
+    if (M.mw && ((float)fiter * M.dt) > (M.dx * (float)(fmove + 1))) {
+      for (int k = tid; k < nf; k += kRunThreads) {
+        sm[oj + k] = (k < nx * 3) ? sm[oe + k + 3] : 0.f;
+        sm[oo + k] = (k < nx * 3) ? sm[ob + k + 3] : 0.f;
+      }
+      __syncthreads();
+      int t = oe;
+      oe = oj;
+      oj = t;
+      t = ob;
+      ob = oo;
+      oo = t;
+      fmove += 1;
+    }
+  }
+  // The particles back: to their places, or with open ends (or a window) the
+  // survivors appended to the other buffer, one atomic a CTA.
+  {
+    for (int k = 0, at = 4 * nf; k < R.nsp; ++k) {
+      const RunSpecies1 &S = R.sp[k];
+      const bool open = S.C.open;
+      const int cur = s_cur[k], used = s_used[k];
+      const Parts dst = (cur != 0) != open ? S.b1 : S.b0;  // open: the other one
+      const int *six = reinterpret_cast<const int *>(sm + at);
+      const float *f = sm + at + S.slots;
+      for (int b = 0; b < used; b += kRunThreads) {
+        const int q = b + tid, ix = q < used ? six[q] : -1;
+        int o = s_i0[k] + q;
+        if (open) {
+          const unsigned lm = __ballot_sync(0xffffffffu, ix >= 0);
+          if (lane == 0) s_n[warp] = __popc(lm);
+          __syncthreads();
+          if (warp == 0) {
+            const int v = s_n[lane];
+            int inc = v;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+              const int y = __shfl_up_sync(0xffffffffu, inc, d);
+              if (lane >= d) inc += y;
+            }
+            s_n[lane] = inc - v;
+            if (lane == 31) s_at = inc ? atomicAdd(&S.st->np[1 - cur], inc) : 0;
+          }
+          __syncthreads();
+          o = s_at + s_n[warp] + __popc(lm & ((1u << lane) - 1));
+          __syncthreads();
+        }
+        if (ix >= 0) {
+          if (o < S.C.cap) {
+            dst.ix[o] = ix;
+            dst.x[o] = f[q];
+            dst.ux[o] = f[S.slots + q];
+            dst.uy[o] = f[2 * S.slots + q];
+            dst.uz[o] = f[3 * S.slots + q];
+          } else {  // (the host makes room for every column: cannot happen)
+            errbits |= ERR1_OVERFLOW;
+          }
+        }
+      }
+      if (tid == 0)
+        atomicAdd(reinterpret_cast<unsigned long long *>(&S.st->pushed), (unsigned long long)s_pushed[k]);
+      if (blockIdx.x == 0 && tid == 0) {
+        // (the other CTAs read these before the first barrier)
+        if (open) {
+          S.st->np[cur] = 0;
+          S.st->cur = 1 - cur;
+        }
+        S.st->ekin = __ldcg(&S.st->ekin_acc);
+        S.st->ekin_acc = 0.0;
+        S.st->iter = s_iter[k] + R.steps;
+        S.st->n_move = s_move[k];
+      }
+      at += 5 * S.slots;
+    }
+  }
+  if (errbits) atomicOr(R.err, errbits);
+  if (blockIdx.x != 0) return;
+  for (int k = tid; k < nv; k += kRunThreads) {
+    R.E[k] = sm[oe + k];
+    R.B[k] = sm[ob + k];
+  }
+  if (tid < 12) R.mur[tid] = s_mur[tid];
+  if (tid == 0) {
+    R.fs->iter = fiter;
+    R.fs->n_move = fmove;
+  }
+}
+
 // laser launch (emf_add_laser, em1d/emf.c:191-260): the plane-wave pulse
 // added to Ey/Ez at the cell nodes and By/Bz half a cell ahead, with the
 // reference's float/double mix; periodic runs then refresh the guard cells
@@ -685,20 +1138,19 @@ __global__ void __launch_bounds__(1024) k1_laser(float *E, float *B, int nx, zc:
   if (periodic) periodic_gc1(E, B, nx);
 }
 
-// field energy per component (emf.c:590-612): double sums of float squares
+// field energy per component (emf.c:590-612): double sums of float squares, a
+// block a component (24 us by one block, double precision being slow here; 6)
 __global__ void __launch_bounds__(1024) k1_emf_energy(const float *E, const float *B, int nx, float dx, double *out) {
   __shared__ double sred[32];
-  for (int c = 0; c < 6; ++c) {
-    const float *F = (c < 3) ? E : B;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
-      const float v = F[(i + GC0) * 3 + c % 3];
-      s += (double)(v * v);
-    }
-    const double t = zc::block_sum_double<1024>(s, sred);
-    if (threadIdx.x == 0) out[c] = t * (0.5 * dx);
-    __syncthreads();
+  const int c = blockIdx.x;
+  const float *F = (c < 3) ? E : B;
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+    const float v = F[(i + GC0) * 3 + c % 3];
+    s += (double)(v * v);
   }
+  const double t = zc::block_sum_double<1024>(s, sred);
+  if (threadIdx.x == 0) out[c] = t * (0.5 * dx);
 }
 
 // ---------------------------------------------------------------------------
@@ -712,6 +1164,7 @@ struct Species1 {
   long long np_bound = 0;    // upper bound of the device count
   Parts buf[2] = {};
   SpecState1 *d_st = nullptr;
+  float *d_lat = nullptr;    // in-cell positions of an injected cell's particles
 };
 
 }  // namespace zc1
@@ -731,6 +1184,14 @@ struct zc1_sim {
   FieldState1 *d_fs = nullptr;
   int *d_err = nullptr, *d_cnt = nullptr;
   double *d_emf = nullptr;
+  // several steps in one launch (k1_run): its deposit buffers and barrier,
+  // the barrier's count and the next deposit buffer
+  float *Jrun = nullptr;
+  unsigned *run_bar = nullptr;
+  unsigned bar_count = 0;
+  int run_phase = 0;
+  size_t run_smem = 0;     // its shared memory at most (0: it cannot be used)
+  int sms = 1;             // multiprocessors: its CTAs, which wait on one another, at most
   size_t fields_smem = 0;  // dynamic shared memory of the fields kernel (0: global variant)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
@@ -846,6 +1307,7 @@ zc_status check_err(zc1_sim *s) {
   int e = 0;
   CK1(cudaMemcpyAsync(&e, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
   CK1(cudaStreamSynchronize(s->st));
+  if (e & ERR1_TIMEOUT) return fail1(ZC_ETIMEOUT, "a wait for the other blocks of a 1-D step timed out");
   if (e & ERR1_OVERFLOW) return fail1(ZC_EOVERFLOW, "1-D particle buffer full at injection");
   if (e & ERR1_ESCAPE) return fail1(ZC_EPARTICLE_ESCAPE, "a particle moved a cell or more, or left the grid");
   return ZC_OK;
@@ -951,32 +1413,23 @@ int enqueue_sort(zc1_sim *s, Species1 &p) {
   return 3;
 }
 
-// enqueues one step (sim_iter): the push of every species (each followed by
-// its cell sort when `sort`), then the fields kernel; nothing is decided on
-// the host, so the same calls serve eager steps and graph capture.  Returns
-// the kernel count.
-int enqueue_step(zc1_sim *s, bool sort) {
-  int k = 0;
-  for (auto &p : s->sp) {
-    Push1 C;
-    C.tem = (float)(0.5 * s->dt / p.m_q);
-    C.dt_dx = s->dt / s->dx;
-    C.qnx = p.q * s->dx / s->dt;
-    C.q = p.q;
-    C.dt = s->dt;
-    C.dx = s->dx;
-    C.nx = s->nx;
-    C.mw = s->mw;
-    C.open = (s->mw || s->part_open) ? 1 : 0;
-    C.cap = p.cap;
-    C.jstride = 3 * (s->nx + GC0 + GC1);
-    const int pf = prof_begin(s, ZC1_K_PUSH);
-    k1_push<<<push_blocks(s, p.cap), kPushThreads, 0, s->st>>>(p.buf[0], p.buf[1], p.d_st, s->E, s->B, s->Jdep, C,
-                                                            p.inj, s->d_err);
-    prof_end(s, pf);
-    k += 1;
-    if (sort) k += enqueue_sort(s, p);
-  }
+Push1 push_const(const zc1_sim *s, const Species1 &p) {
+  Push1 C;
+  C.tem = (float)(0.5 * s->dt / p.m_q);
+  C.dt_dx = s->dt / s->dx;
+  C.qnx = p.q * s->dx / s->dt;
+  C.q = p.q;
+  C.dt = s->dt;
+  C.dx = s->dx;
+  C.nx = s->nx;
+  C.mw = s->mw;
+  C.open = (s->mw || s->part_open) ? 1 : 0;
+  C.cap = p.cap;
+  C.jstride = 3 * (s->nx + GC0 + GC1);
+  return C;
+}
+
+Fields1 field_const(const zc1_sim *s) {
   Fields1 M;
   M.nx = s->nx;
   M.dt = s->dt;
@@ -985,6 +1438,25 @@ int enqueue_step(zc1_sim *s, bool sort) {
   M.cur_periodic = s->current_periodic;
   M.mw = s->mw;
   M.S = s->smooth;
+  return M;
+}
+
+// enqueues one step (sim_iter): the push of every species (each followed by
+// its cell sort when `sort`), then the fields kernel; nothing is decided on
+// the host, so the same calls serve eager steps and graph capture.  Returns
+// the kernel count.
+int enqueue_step(zc1_sim *s, bool sort) {
+  int k = 0;
+  for (auto &p : s->sp) {
+    const Push1 C = push_const(s, p);
+    const int pf = prof_begin(s, ZC1_K_PUSH);
+    k1_push<<<push_blocks(s, p.cap), kPushThreads, 0, s->st>>>(p.buf[0], p.buf[1], p.d_st, s->E, s->B, s->Jdep, C,
+                                                            p.inj, s->d_err);
+    prof_end(s, pf);
+    k += 1;
+    if (sort) k += enqueue_sort(s, p);
+  }
+  const Fields1 M = field_const(s);
   const int pf = prof_begin(s, ZC1_K_FIELDS);
   if (s->fields_smem)
     k1_fields<true><<<1, 1024, s->fields_smem, s->st>>>(s->E, s->B, s->Jdep, s->Jout, s->mur, s->d_fs, M);
@@ -1063,6 +1535,109 @@ zc_status run_block(zc1_sim *s) {
   return ZC_OK;
 }
 
+// Up to `most` steps in one launch (k1_run), to the next cell sort at the
+// latest; *done: how many.  None when kernels are timed one by one, there are
+// no species or too many, or the grids and every CTA's share of the particles
+// do not fit its shared memory (then the two kernels a step, in graphs).
+//
+// The CTAs: one a multiprocessor when the caller waits for the steps.  One who
+// does not may have other simulations' steps beside these, and launches that
+// fill the GPU would run one after another: a quarter of the multiprocessors
+// then (64 runs of the 1000-cell deck side by side: 21.7 G particles/s against
+// 8.3 with the full grid and 12.9 with the two kernels; one run alone takes
+// 15.2 us a step against 11.0 and 22).  A single step that nobody waits for is
+// left to the two kernels: 25.0 us against 26.9.
+zc_status run_steps(zc1_sim *s, int most, bool waits, int *done) {
+  *done = 0;
+  if (!s->run_smem || s->profile || s->sp.empty() || (int)s->sp.size() > kRunSpecies) return ZC_OK;
+  const int to_sort = s->sort_every - s->sp[0].iter % s->sort_every;
+  const int n = std::min(most, to_sort);
+  if (n == 1 && !waits) return ZC_OK;
+  TRY1(ensure_cap(s, n));
+  long long np = 1;
+  for (auto &p : s->sp) np = std::max(np, p.np_bound);
+  // one CTA a multiprocessor, at least a warp of particles each (a
+  // simulation's own cap counts CTAs of kPushThreads)
+  const int room = waits ? s->sms : std::max(1, s->sms / 4);
+  const int most_ctas =
+      s->push_ctas > 0 ? std::max(1, std::min(s->sms, s->push_ctas * kPushThreads / kRunThreads)) : room;
+  const int grid = (int)std::max<long long>(1, std::min<long long>(most_ctas, np / 256));
+  Run1 R{};
+  R.nsp = (int)s->sp.size();
+  R.steps = n;
+  R.phase = s->run_phase;
+  R.bar0 = s->bar_count;
+  R.bar = s->run_bar;
+  R.Jrun = s->Jrun;
+  R.E = s->E;
+  R.B = s->B;
+  R.Jout = s->Jout;
+  R.mur = s->mur;
+  R.fs = s->d_fs;
+  R.err = s->d_err;
+  R.M = field_const(s);
+  size_t smem = 4 * sizeof(float) * grid_stride1(s->nx);
+  for (int k = 0; k < R.nsp; ++k) {
+    Species1 &p = s->sp[k];
+    const long long share = (p.np_bound + grid - 1) / grid;
+    // the columns of n window moves go round the CTAs
+    const long long cols = (s->mw && p.inj.type != 1) ? (long long)((n + grid - 1) / grid) * p.inj.ppc : 0;
+    const long long slots = (share + cols + kRunThreads - 1) / kRunThreads * kRunThreads;
+    smem += 5 * sizeof(float) * (size_t)slots;
+    if (smem > s->run_smem) return ZC_OK;
+    R.sp[k] = RunSpecies1{p.buf[0], p.buf[1], p.d_st, p.d_lat, (int)slots, push_const(s, p), p.inj};
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kRunThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CK1(cudaLaunchKernelEx(&cfg, k1_run, R));
+  s->bar_count += (unsigned)n * (unsigned)grid;
+  s->run_phase = (s->run_phase + n) % 3;
+  s->launches += 1;
+  if (n == to_sort)
+    for (auto &p : s->sp) s->launches += enqueue_sort(s, p);
+  CK1(cudaGetLastError());
+  for (int i = 0; i < n; ++i) advance_mirror(s);
+  *done = n;
+  return ZC_OK;
+}
+
+zc_status enqueue_steps(zc1_sim *s, int nsteps, bool waits) {
+  if (!s || nsteps < 0) return fail1(ZC_EINVAL, "invalid argument");
+  Guard1 g(s->device);
+  if (!s->timing) {
+    CK1(cudaEventRecord(s->ev0, s->st));
+    s->timing = 1;
+  }
+  int k = 0;
+  while (k < nsteps) {
+    int n = 0;
+    TRY1(run_steps(s, nsteps - k, waits, &n));
+    k += n;
+    if (n) continue;
+    const bool aligned = !s->sp.empty() && s->sort_every > 0 && s->sp[0].iter % s->sort_every == 0;
+    if (aligned && nsteps - k >= s->sort_every) {
+      TRY1(run_block(s));
+      k += s->sort_every;
+    } else {
+      TRY1(step_eager(s));
+      k += 1;
+    }
+    if (s->profile && s->prof_used >= s->prof_graph_slots + 4096) {
+      CK1(cudaStreamSynchronize(s->st));
+      prof_collect(s);
+    }
+  }
+  return ZC_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1089,11 +1664,16 @@ zc_status zc1_create(const zc1_desc *d, zc1_sim **out) {
   s->push_ctas = d->push_ctas > 0 ? d->push_ctas : 0;
   Guard1 g(s->device);
   const size_t gbytes = sizeof(float) * 3 * (s->nx + GC0 + GC1);
+  const size_t rbytes = sizeof(float) * 3 * kRunCopies * grid_stride1(s->nx);
   cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&s->E, gbytes);
   if (e == cudaSuccess) e = cudaMalloc(&s->B, gbytes);
   if (e == cudaSuccess) e = cudaMalloc(&s->Jdep, gbytes * kJCopies);
   if (e == cudaSuccess) e = cudaMalloc(&s->Jout, gbytes);
+  if (e == cudaSuccess) e = cudaMalloc(&s->Jrun, rbytes);
+  if (e == cudaSuccess) e = cudaMemset(s->Jrun, 0, rbytes);
+  if (e == cudaSuccess) e = cudaMalloc(&s->run_bar, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(s->run_bar, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc(&s->mur, sizeof(float) * 12);
   if (e == cudaSuccess) e = cudaMalloc(&s->d_fs, sizeof(FieldState1));
   if (e == cudaSuccess) e = cudaMalloc(&s->d_err, sizeof(int));
@@ -1115,10 +1695,16 @@ zc_status zc1_create(const zc1_desc *d, zc1_sim **out) {
   // what another simulation launches with.
   int optin = 0;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
   const size_t smem = 4 * gbytes;
   if (e == cudaSuccess && smem <= (size_t)optin) {
     e = cudaFuncSetAttribute(k1_fields<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
     if (e == cudaSuccess) s->fields_smem = smem;
+  }
+  // k1_run: what its static arrays (under 4 KB) leave
+  if (e == cudaSuccess) {
+    e = cudaFuncSetAttribute(k1_run, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 4096);
+    if (e == cudaSuccess) s->run_smem = optin - 4096;
   }
   if (e != cudaSuccess) {
     zc1_destroy(s);
@@ -1137,10 +1723,13 @@ void zc1_destroy(zc1_sim *s) {
     free_parts(p.buf[0]);
     free_parts(p.buf[1]);
     cudaFree(p.d_st);
+    cudaFree(p.d_lat);
   }
   cudaFree(s->E);
   cudaFree(s->B);
   cudaFree(s->Jdep);
+  cudaFree(s->Jrun);
+  cudaFree(s->run_bar);
   cudaFree(s->Jout);
   cudaFree(s->mur);
   cudaFree(s->d_fs);
@@ -1199,6 +1788,10 @@ zc_status zc1_add_species(zc1_sim *s, const zc1_species_desc *d, const zc1_part 
     CK1(cudaMemcpy(p.buf[0].uy, uy.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
     CK1(cudaMemcpy(p.buf[0].uz, uz.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
   }
+  std::vector<float> lat(p.inj.ppc);
+  for (int i = 0; i < p.inj.ppc; ++i) lat[i] = (float)((i + 0.5) / p.inj.ppc);
+  CK1(cudaMalloc(&p.d_lat, sizeof(float) * lat.size()));
+  CK1(cudaMemcpy(p.d_lat, lat.data(), sizeof(float) * lat.size(), cudaMemcpyHostToDevice));
   SpecState1 h{};
   h.np[0] = np;
   CK1(cudaMemcpy(p.d_st, &h, sizeof(SpecState1), cudaMemcpyHostToDevice));
@@ -1292,33 +1885,10 @@ zc_status zc1_get_current(zc1_sim *s, float *J) {
   return ZC_OK;
 }
 
-zc_status zc1_step_async(zc1_sim *s, int nsteps) {
-  if (!s || nsteps < 0) return fail1(ZC_EINVAL, "invalid argument");
-  Guard1 g(s->device);
-  if (!s->timing) {
-    CK1(cudaEventRecord(s->ev0, s->st));
-    s->timing = 1;
-  }
-  int k = 0;
-  while (k < nsteps) {
-    const bool aligned = !s->sp.empty() && s->sort_every > 0 && s->sp[0].iter % s->sort_every == 0;
-    if (aligned && nsteps - k >= s->sort_every) {
-      TRY1(run_block(s));
-      k += s->sort_every;
-    } else {
-      TRY1(step_eager(s));
-      k += 1;
-    }
-    if (s->profile && s->prof_used >= s->prof_graph_slots + 4096) {
-      CK1(cudaStreamSynchronize(s->st));
-      prof_collect(s);
-    }
-  }
-  return ZC_OK;
-}
+zc_status zc1_step_async(zc1_sim *s, int nsteps) { return enqueue_steps(s, nsteps, false); }
 
 zc_status zc1_step(zc1_sim *s, int nsteps) {
-  TRY1(zc1_step_async(s, nsteps));
+  TRY1(enqueue_steps(s, nsteps, true));
   return zc1_synchronize(s);
 }
 
@@ -1357,7 +1927,7 @@ zc_status zc1_energy(zc1_sim *s, double emf[6], double *kin) {
   if (!s) return fail1(ZC_EINVAL, "null simulation handle");
   Guard1 g(s->device);
   if (emf) {
-    k1_emf_energy<<<1, 1024, 0, s->st>>>(s->E, s->B, s->nx, s->dx, s->d_emf);
+    k1_emf_energy<<<6, 1024, 0, s->st>>>(s->E, s->B, s->nx, s->dx, s->d_emf);
     CK1(cudaGetLastError());
     CK1(cudaMemcpyAsync(emf, s->d_emf, sizeof(double) * 6, cudaMemcpyDeviceToHost, s->st));
   }
