@@ -20,23 +20,24 @@
 //        backward ones on the periodic grid and vice versa);
 //   deposit: the transpose of the deposit is a gather of the current's
 //        adjoint along the same zigzag segments; its derivative with respect
-//        to the start position, the displacement and v_z comes from running
-//        the deposit code on 5-way forward-mode dual numbers;
-//   push: Boris + move on 9-way dual numbers (momentum, E_p, B_p);
+//        to the start position and the displacement is written out for a
+//        motion inside one cell (the usual case), and comes from running the
+//        deposit code on 4-way forward-mode dual numbers for the others;
+//   push: the reverse of Boris + move, by hand (momentum, E_p, B_p);
 //   gather: its transpose scatters the adjoint of E_p, B_p onto the grid
-//        with the same weights; the derivative of the weights with respect
-//        to the position comes from 2-way dual numbers.
+//        with the same weights; the samples' derivatives with respect to the
+//        position are differences of the same four values.
 // The deposit and the gather are piecewise polynomial in the position: the
 // gradient is that of the piece the trajectory lies in (kinks where a
 // trajectory crosses a cell edge or the half-cell of the staggered gather).
 //
 // Checkpoints: the state (particles, E, B) is kept every K steps of the
 // forward run, which also keeps the pre-step states of its last two
-// segments (of its last one when two would take more than 8 GiB); the
-// reverse sweep walks those back directly, and recomputes every earlier
-// segment of K steps from its checkpoint, keeping its pre-step states, before
-// walking it backwards.  A kept step writes its particles straight into the
-// next step's slot, so keeping costs only the copies of E and B.
+// segments, more for a longer run, as far as 8 GiB go (of its last one when two
+// would take more); the reverse sweep walks those back directly, and recomputes
+// every earlier segment of K steps from its checkpoint, keeping its pre-step
+// states, before walking it backwards.  A kept step writes its particles and
+// fields straight into the next step's slot.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -204,51 +205,119 @@ __device__ __forceinline__ bool active(const State<R> &s, const int *birth, int 
   return s.alive[p] && (!birth || birth[p] <= P.n);
 }
 
-// staggered bilinear gather (interpolate_fld): weights of type T, field
-// samples of type R
-template <class R, class T>
-__device__ __forceinline__ T lerp2(const Planes<R> &g, int c, int a, int b, const T &wa, const T &wb) {
-  return (g(c, a, b) * (R(1) - wa) + g(c, a + 1, b) * wa) * (R(1) - wb) +
-         (g(c, a, b + 1) * (R(1) - wa) + g(c, a + 1, b + 1) * wa) * wb;
+// The nodes around a particle, looked up once: offsets within a plane of the
+// columns and rows of the samples at whole nodes (c, r) and at half nodes
+// (ch, rh), and the weights of the upper node of each (interpolate_fld).  A
+// plane has fewer than 2^32 cells.  (With a wrapped 64-bit index a sample,
+// the gather was two thirds of the push's 1170 instructions.)
+template <class R>
+struct Stencil {
+  unsigned c[2], ch[2], r[2], rh[2];
+  R x, y, xh, yh;
+};
+
+template <class R>
+__device__ __forceinline__ Stencil<R> stencil(int nx, int ny, int mw, int i, int j, R x, R y) {
+  Stencil<R> s;
+  const bool lx = x < R(0.5), ly = y < R(0.5);
+  const unsigned pt = mw ? nx + 3 : nx;
+  const unsigned c0 = mw ? i : wrap(i - 1, nx), c1 = mw ? i + 1 : wrap(i, nx), c2 = mw ? i + 2 : wrap(i + 1, nx);
+  const unsigned r0 = wrap(j - 1, ny) * pt, r1 = wrap(j, ny) * pt, r2 = wrap(j + 1, ny) * pt;
+  s.c[0] = c1;
+  s.c[1] = c2;
+  s.r[0] = r1;
+  s.r[1] = r2;
+  s.ch[0] = lx ? c0 : c1;
+  s.ch[1] = lx ? c1 : c2;
+  s.rh[0] = ly ? r0 : r1;
+  s.rh[1] = ly ? r1 : r2;
+  s.x = x;
+  s.y = y;
+  s.xh = x + (lx ? R(0.5) : R(-0.5));
+  s.yh = y + (ly ? R(0.5) : R(-0.5));
+  return s;
 }
 
-template <class R, class T>
-__device__ __forceinline__ void gather(const Planes<R> &E, const Planes<R> &B, int i, int j, const T &x, const T &y,
-                                       T f[6]) {
-  const bool lx = value(x) < R(0.5), ly = value(y) < R(0.5);
-  const int ih = i + (lx ? -1 : 0), jh = j + (ly ? -1 : 0);
-  const T w1h = x + (lx ? R(0.5) : R(-0.5));
-  const T w2h = y + (ly ? R(0.5) : R(-0.5));
-  f[0] = lerp2(E, 0, ih, j, w1h, y);
-  f[1] = lerp2(E, 1, i, jh, x, w2h);
-  f[2] = lerp2(E, 2, i, j, x, y);
-  f[3] = lerp2(B, 0, i, jh, x, w2h);
-  f[4] = lerp2(B, 1, ih, j, w1h, y);
-  f[5] = lerp2(B, 2, ih, jh, w1h, w2h);
+// a staggered bilinear sample; D: with its derivatives along x and y
+template <bool D, class R>
+__device__ __forceinline__ R sample(const R *g, const unsigned c[2], const unsigned r[2], R wa, R wb, R *dx, R *dy) {
+  const R f00 = g[r[0] + c[0]], f10 = g[r[0] + c[1]], f01 = g[r[1] + c[0]], f11 = g[r[1] + c[1]];
+  const R f0 = f00 * (R(1) - wa) + f10 * wa, f1 = f01 * (R(1) - wa) + f11 * wa;
+  if (D) {
+    *dx = (f10 - f00) * (R(1) - wb) + (f11 - f01) * wb;
+    *dy = f1 - f0;
+  }
+  return f0 * (R(1) - wb) + f1 * wb;
+}
+
+// E and B at a particle (interpolate_fld); pl: cells a plane
+template <bool D, class R>
+__device__ __forceinline__ void gather(const R *E, const R *B, size_t pl, const Stencil<R> &s, R f[6], R dx[6],
+                                       R dy[6]) {
+  f[0] = sample<D>(E, s.ch, s.r, s.xh, s.y, &dx[0], &dy[0]);
+  f[1] = sample<D>(E + pl, s.c, s.rh, s.x, s.yh, &dx[1], &dy[1]);
+  f[2] = sample<D>(E + 2 * pl, s.c, s.r, s.x, s.y, &dx[2], &dy[2]);
+  f[3] = sample<D>(B, s.c, s.rh, s.x, s.yh, &dx[3], &dy[3]);
+  f[4] = sample<D>(B + pl, s.ch, s.r, s.xh, s.y, &dx[4], &dy[4]);
+  f[5] = sample<D>(B + 2 * pl, s.ch, s.rh, s.xh, s.yh, &dx[5], &dy[5]);
 }
 
 // transpose of the gather: adds a[c] times the weights of sample c to the
 // grids (ga for E, gb for B)
 template <class R>
-__device__ __forceinline__ void scatter_add(R *ga, R *gb, const Planes<R> &shape, int i, int j, R x, R y,
-                                            const R a[6]) {
-  const bool lx = x < R(0.5), ly = y < R(0.5);
-  const int ih = i + (lx ? -1 : 0), jh = j + (ly ? -1 : 0);
-  const R w1h = x + (lx ? R(0.5) : R(-0.5));
-  const R w2h = y + (ly ? R(0.5) : R(-0.5));
-  auto put = [&](R *g, int c, int a0, int b0, R wa, R wb, R v) {
+__device__ __forceinline__ void scatter_add(R *ga, R *gb, size_t pl, const Stencil<R> &s, const R a[6]) {
+  auto put = [&](R *g, const unsigned c[2], const unsigned r[2], R wa, R wb, R v) {
     if (v == R(0)) return;
-    atomicAdd(&g[shape.at(c, a0, b0)], v * (R(1) - wa) * (R(1) - wb));
-    atomicAdd(&g[shape.at(c, a0 + 1, b0)], v * wa * (R(1) - wb));
-    atomicAdd(&g[shape.at(c, a0, b0 + 1)], v * (R(1) - wa) * wb);
-    atomicAdd(&g[shape.at(c, a0 + 1, b0 + 1)], v * wa * wb);
+    const R v0 = v * (R(1) - wa), v1 = v * wa;
+    atomicAdd(&g[r[0] + c[0]], v0 * (R(1) - wb));
+    atomicAdd(&g[r[0] + c[1]], v1 * (R(1) - wb));
+    atomicAdd(&g[r[1] + c[0]], v0 * wb);
+    atomicAdd(&g[r[1] + c[1]], v1 * wb);
   };
-  put(ga, 0, ih, j, w1h, y, a[0]);
-  put(ga, 1, i, jh, x, w2h, a[1]);
-  put(ga, 2, i, j, x, y, a[2]);
-  put(gb, 0, i, jh, x, w2h, a[3]);
-  put(gb, 1, ih, j, w1h, y, a[4]);
-  put(gb, 2, ih, jh, w1h, w2h, a[5]);
+  put(ga, s.ch, s.r, s.xh, s.y, a[0]);
+  put(ga + pl, s.c, s.rh, s.x, s.yh, a[1]);
+  put(ga + 2 * pl, s.c, s.r, s.x, s.y, a[2]);
+  put(gb, s.c, s.rh, s.x, s.yh, a[3]);
+  put(gb + pl, s.ch, s.r, s.xh, s.y, a[4]);
+  put(gb + 2 * pl, s.ch, s.rh, s.xh, s.yh, a[5]);
+}
+
+// the same for the sums apart: samples that share a stencil share a node's
+// 8 bytes, (Ex, By) in [0, 2 pl), (Ey, Bx) in [2 pl, 4 pl), then Ez, then Bz
+__device__ __forceinline__ void red2(float *p, float x, float y) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void scatter_pairs(float *g, size_t pl, const Stencil<float> &s, const float a[6]) {
+  if (a[0] == 0.f && a[1] == 0.f && a[2] == 0.f && a[3] == 0.f && a[4] == 0.f && a[5] == 0.f) return;
+  auto pair = [&](float *p, const unsigned c[2], const unsigned r[2], float wa, float wb, float u, float v) {
+    const float w00 = (1.f - wa) * (1.f - wb), w10 = wa * (1.f - wb), w01 = (1.f - wa) * wb, w11 = wa * wb;
+    red2(p + 2 * (size_t)(r[0] + c[0]), u * w00, v * w00);
+    red2(p + 2 * (size_t)(r[0] + c[1]), u * w10, v * w10);
+    red2(p + 2 * (size_t)(r[1] + c[0]), u * w01, v * w01);
+    red2(p + 2 * (size_t)(r[1] + c[1]), u * w11, v * w11);
+  };
+  auto one = [&](float *p, const unsigned c[2], const unsigned r[2], float wa, float wb, float u) {
+    const float u0 = u * (1.f - wa), u1 = u * wa;
+    atomicAdd(p + (r[0] + c[0]), u0 * (1.f - wb));
+    atomicAdd(p + (r[0] + c[1]), u1 * (1.f - wb));
+    atomicAdd(p + (r[1] + c[0]), u0 * wb);
+    atomicAdd(p + (r[1] + c[1]), u1 * wb);
+  };
+  pair(g, s.ch, s.r, s.xh, s.y, a[0], a[4]);
+  pair(g + 2 * pl, s.c, s.rh, s.x, s.yh, a[1], a[3]);
+  one(g + 4 * pl, s.c, s.r, s.x, s.y, a[2]);
+  one(g + 5 * pl, s.ch, s.rh, s.xh, s.yh, a[5]);
+}
+// a component (c: Ex, Ey, Ez, Bx, By, Bz) of the sums
+__device__ __forceinline__ float pair_at(const float *g, size_t pl, int c, unsigned n) {
+  switch (c) {
+    case 0: return g[2 * (size_t)n];
+    case 1: return g[2 * pl + 2 * (size_t)n];
+    case 2: return g[4 * pl + n];
+    case 3: return g[2 * pl + 2 * (size_t)n + 1];
+    case 4: return g[2 * (size_t)n + 1];
+    default: return g[5 * pl + n];
+  }
 }
 
 // Boris push and move (particles.c:1145-1207): momentum, E_p, B_p in;
@@ -371,14 +440,11 @@ __device__ __forceinline__ void segment(Sink &sink, int ix, int iy, const T &x0,
   const T s0x0 = R(1) - x0, s0x1 = x0, s1x0 = R(1) - x1, s1x1 = x1;
   const T s0y0 = R(1) - y0, s0y1 = y0, s1y0 = R(1) - y1, s1y1 = y1;
   const T jx = dx * P.qnx, jy = dy * P.qny;
-  sink.add(0, ix, iy, jx * (R(0.5) * (s0y0 + s1y0)));
-  sink.add(0, ix, iy + 1, jx * (R(0.5) * (s0y1 + s1y1)));
-  sink.add(1, ix, iy, jy * (R(0.5) * (s0x0 + s1x0)));
-  sink.add(1, ix + 1, iy, jy * (R(0.5) * (s0x1 + s1x1)));
-  sink.add(2, ix, iy, qvz * (s0x0 * s0y0 + s1x0 * s1y0 + (s0x0 * s1y0 - s1x0 * s0y0) / R(2)));
-  sink.add(2, ix + 1, iy, qvz * (s0x1 * s0y0 + s1x1 * s1y0 + (s0x1 * s1y0 - s1x1 * s0y0) / R(2)));
-  sink.add(2, ix, iy + 1, qvz * (s0x0 * s0y1 + s1x0 * s1y1 + (s0x0 * s1y1 - s1x0 * s0y1) / R(2)));
-  sink.add(2, ix + 1, iy + 1, qvz * (s0x1 * s0y1 + s1x1 * s1y1 + (s0x1 * s1y1 - s1x1 * s0y1) / R(2)));
+  sink.put(ix, iy, jx * (R(0.5) * (s0y0 + s1y0)), jx * (R(0.5) * (s0y1 + s1y1)), jy * (R(0.5) * (s0x0 + s1x0)),
+           jy * (R(0.5) * (s0x1 + s1x1)), qvz * (s0x0 * s0y0 + s1x0 * s1y0 + (s0x0 * s1y0 - s1x0 * s0y0) / R(2)),
+           qvz * (s0x1 * s0y0 + s1x1 * s1y0 + (s0x1 * s1y0 - s1x1 * s0y0) / R(2)),
+           qvz * (s0x0 * s0y1 + s1x0 * s1y1 + (s0x0 * s1y1 - s1x0 * s0y1) / R(2)),
+           qvz * (s0x1 * s0y1 + s1x1 * s1y1 + (s0x1 * s1y1 - s1x1 * s0y1) / R(2)));
 }
 
 template <class T>
@@ -476,11 +542,41 @@ __device__ __forceinline__ void zigzag(Sink &sink, int ix, int iy, const T &x0, 
 // ---------------------------------------------------------------------------
 // sinks of the deposit
 // ---------------------------------------------------------------------------
-template <class R>
+//
+// The sums over particles are what a step takes its time for (10^6 particles
+// on 256 x 256 cells: without them the push would take half of it, its reverse
+// 40% less; the particles' bytes alone are 10 us).  So in float32, without a
+// window (V4), components that go to one node lie together and go out in one
+// reduction.  The deposit makes 4 of 16 bytes instead of 8 single ones (J is
+// [node][4]): 78 us to 42.  The transpose of the gather makes 8 of 8 bytes and
+// 8 single ones instead of 24 (scatter_pairs): 147 us to 92; all six
+// components of a node in 32 bytes, 12.5 of 16 bytes on average, took longer,
+// most of what they carry being zeros.
+__device__ __forceinline__ void red4(float *p, float x, float y, float z) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(0.f) : "memory");
+}
+
+template <class R, bool V4>
 struct DepositSink {  // forward: J += w * contribution
   Planes<R> J;
   R w;
-  __device__ __forceinline__ void add(int c, int i, int j, R v) const { atomicAdd(&J.f[J.at(c, i, j)], w * v); }
+  __device__ __forceinline__ void put(int i, int j, R x0, R x1, R y0, R y1, R z00, R z10, R z01, R z11) const {
+    if constexpr (V4) {
+      red4(&J.f[4 * J.at(0, i, j)], w * x0, w * y0, w * z00);
+      red4(&J.f[4 * J.at(0, i + 1, j)], R(0), w * y1, w * z10);
+      red4(&J.f[4 * J.at(0, i, j + 1)], w * x1, R(0), w * z01);
+      red4(&J.f[4 * J.at(0, i + 1, j + 1)], R(0), R(0), w * z11);
+    } else {
+      atomicAdd(&J.f[J.at(0, i, j)], w * x0);
+      atomicAdd(&J.f[J.at(0, i, j + 1)], w * x1);
+      atomicAdd(&J.f[J.at(1, i, j)], w * y0);
+      atomicAdd(&J.f[J.at(1, i + 1, j)], w * y1);
+      atomicAdd(&J.f[J.at(2, i, j)], w * z00);
+      atomicAdd(&J.f[J.at(2, i + 1, j)], w * z10);
+      atomicAdd(&J.f[J.at(2, i, j + 1)], w * z01);
+      atomicAdd(&J.f[J.at(2, i + 1, j + 1)], w * z11);
+    }
+  }
 };
 
 // reverse: sums of lambda_J times the contributions (per unit weight), the
@@ -490,6 +586,18 @@ template <class R, int N>
 struct AdjointSink {
   Planes<R> lamJ;
   Dual<R, N> axy, az;
+  __device__ __forceinline__ void put(int i, int j, const Dual<R, N> &x0, const Dual<R, N> &x1, const Dual<R, N> &y0,
+                                      const Dual<R, N> &y1, const Dual<R, N> &z00, const Dual<R, N> &z10,
+                                      const Dual<R, N> &z01, const Dual<R, N> &z11) {
+    add(0, i, j, x0);
+    add(0, i, j + 1, x1);
+    add(1, i, j, y0);
+    add(1, i + 1, j, y1);
+    add(2, i, j, z00);
+    add(2, i + 1, j, z10);
+    add(2, i, j + 1, z01);
+    add(2, i + 1, j + 1, z11);
+  }
   __device__ __forceinline__ void add(int c, int i, int j, const Dual<R, N> &v) {
     const R l = lamJ(c, i, j);
     Dual<R, N> &a = (c == 2) ? az : axy;
@@ -502,31 +610,46 @@ struct AdjointSink {
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
-template <class R>
+// A block's particles: contiguous, whole rounds of the block.
+struct Share {
+  int first, end;
+  __device__ __forceinline__ explicit Share(int np) {
+    const long long rounds = ((long long)np + blockDim.x - 1) / blockDim.x;
+    const long long a = rounds * blockIdx.x / gridDim.x * blockDim.x;
+    const long long b = rounds * (blockIdx.x + 1) / gridDim.x * blockDim.x;
+    first = (int)(a < np ? a : np);
+    end = (int)(b < np ? b : np);
+  }
+};
+
+template <class R, bool V4>
 __global__ void k_adj_push(State<R> s, State<R> o, const R *w, const int *birth, Planes<R> E, Planes<R> B,
                            Planes<R> J, double *ekin, Params<R> P) {
+  const size_t pl = (size_t)E.pitch() * P.ny;
   double ek = 0;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P.np; p += gridDim.x * blockDim.x) {
-    if (!active(s, birth, p, P)) {  // not born yet or gone: carried over unchanged
-      o.ix[p] = s.ix[p];
-      o.iy[p] = s.iy[p];
-      o.alive[p] = s.alive[p];
-      o.x[p] = s.x[p];
-      o.y[p] = s.y[p];
-      o.ux[p] = s.ux[p];
-      o.uy[p] = s.uy[p];
-      o.uz[p] = s.uz[p];
-      continue;
-    }
+  const Share mine(P.np);
+  for (int p = mine.first + threadIdx.x; p < mine.end; p += blockDim.x) {
     const int ix = s.ix[p], iy = s.iy[p];
     const R x = s.x[p], y = s.y[p];
     const R u[3] = {s.ux[p], s.uy[p], s.uz[p]};
+    if (!active(s, birth, p, P)) {  // not born yet or gone: carried over unchanged
+      o.ix[p] = ix;
+      o.iy[p] = iy;
+      o.alive[p] = s.alive[p];
+      o.x[p] = x;
+      o.y[p] = y;
+      o.ux[p] = u[0];
+      o.uy[p] = u[1];
+      o.uz[p] = u[2];
+      continue;
+    }
+    const R wp = w[p];
     R f[6];
-    gather<R, R>(E, B, ix, iy, x, y, f);
-    ek += (double)w[p] * (double)kinetic(u, f, P);
+    gather<false>(E.f, B.f, pl, stencil(P.nx, P.ny, P.mw, ix, iy, x, y), f, (R *)nullptr, (R *)nullptr);
+    if (ekin) ek += (double)wp * (double)kinetic(u, f, P);
     R uo[3], mx, my, qvz;
     boris<R, R>(u, f, f + 3, P, uo, mx, my, qvz);
-    DepositSink<R> sink{J, w[p]};
+    DepositSink<R, V4> sink{J, wp};
     zigzag<R, R>(sink, ix, iy, x, y, mx, my, qvz, P);
     R x1 = x + mx, y1 = y + my;
     const int di = (x1 >= R(1)) - (x1 < R(0)), dj = (y1 >= R(1)) - (y1 < R(0));
@@ -547,19 +670,63 @@ __global__ void k_adj_push(State<R> s, State<R> o, const R *w, const int *birth,
   if (ekin && ek != 0.0) atomicAdd(ekin, ek);
 }
 
-// the contributions of a motion that stays in its cell: one segment
-template <class R, class T, class Sink>
-__device__ __forceinline__ void single_segment(Sink &sink, int ix, int iy, const T &x0, const T &y0, const T &dx,
-                                               const T &dy, const T &qvz, const Params<R> &P) {
-  segment(sink, ix, iy, x0, x0 + dx, y0, y0 + dy, dx, dy, qvz * R(0.5), P);
+// the adjoint current at the nodes that a motion inside a cell deposits to
+template <class R>
+struct CellJ {
+  R x0, x1, y0, y1, z00, z10, z01, z11;
+};
+template <class R>
+__device__ __forceinline__ CellJ<R> cell_current(const R *l, size_t pl, const Stencil<R> &n) {
+  const unsigned n00 = n.r[0] + n.c[0], n10 = n.r[0] + n.c[1], n01 = n.r[1] + n.c[0], n11 = n.r[1] + n.c[1];
+  const R *ly = l + pl, *lz = l + 2 * pl;
+  return CellJ<R>{l[n00], l[n01], ly[n00], ly[n10], lz[n00], lz[n10], lz[n01], lz[n11]};
 }
+
+// Derivatives of the deposit of a motion that stays in its cell, one segment
+// (segment() above with q v_z = 1/2): l times the contributions, l the adjoint
+// current at the cell's nodes, and the derivatives of that sum with respect to
+// (x, y, dx, dy).  The x and y components are linear in the mean position; the
+// z component is the bilinear interpolant g of l at the corners of the motion,
+// (g(x0, y0) + g(x1, y1) + (g(x0, y1) - g(x1, y0)) / 2) / 2.
+template <class R>
+__device__ __forceinline__ void segment_vjp(const CellJ<R> &l, const Stencil<R> &n, R mx, R my, const Params<R> &P,
+                                            R &axy, R &az, R dxy[4], R dz[4]) {
+  const R x0 = n.x, x1 = n.x + mx, y0 = n.y, y1 = n.y + my;
+  // jx = qnx dx at y nodes, jy = qny dy at x nodes
+  const R a0 = l.x0, a1 = l.x1, b0 = l.y0, b1 = l.y1;
+  const R xm = x0 + mx / R(2), ym = y0 + my / R(2), jx = P.qnx * mx, jy = P.qny * my;
+  const R a = fma(a1, ym, a0 * (R(1) - ym)), b = fma(b1, xm, b0 * (R(1) - xm));
+  axy = fma(jx, a, jy * b);
+  dxy[0] = jy * (b1 - b0);
+  dxy[1] = jx * (a1 - a0);
+  dxy[2] = fma(dxy[0], R(0.5), P.qnx * a);
+  dxy[3] = fma(dxy[1], R(0.5), P.qny * b);
+  // z
+  const R z00 = l.z00, z10 = l.z10, z01 = l.z01, z11 = l.z11;
+  const R dx0 = z10 - z00, dx1 = z11 - z01, dy0 = z01 - z00, dy1 = z11 - z10;
+  const R X0 = fma(dx1, y0, dx0 * (R(1) - y0)), X1 = fma(dx1, y1, dx0 * (R(1) - y1));  // dg/dx at y0, y1
+  const R Y0 = fma(dy1, x0, dy0 * (R(1) - x0)), Y1 = fma(dy1, x1, dy0 * (R(1) - x1));  // dg/dy at x0, x1
+  const R l0 = fma(z10, x0, z00 * (R(1) - x0)), u0 = fma(z11, x0, z01 * (R(1) - x0));  // g(x0, .) at the nodes
+  const R l1 = fma(z10, x1, z00 * (R(1) - x1)), u1 = fma(z11, x1, z01 * (R(1) - x1));
+  const R g00 = fma(u0, y0, l0 * (R(1) - y0)), g01 = fma(u0, y1, l0 * (R(1) - y1));
+  const R g10 = fma(u1, y0, l1 * (R(1) - y0)), g11 = fma(u1, y1, l1 * (R(1) - y1));
+  az = R(0.5) * (g00 + g11 + R(0.5) * (g01 - g10));
+  dz[0] = fma(R(0.75), X1, R(0.25) * X0);
+  dz[1] = fma(R(0.75), Y0, R(0.25) * Y1);
+  dz[2] = fma(R(0.5), X1, R(-0.25) * X0);
+  dz[3] = fma(R(0.5), Y1, R(0.25) * Y0);
+}
+
+// resident CTAs of the reverse push (float32), one wave of them, each with a
+// contiguous share: 80 registers.  5 of them 5% slower, 8 (64 registers) spill.
+constexpr int kRevCtas = 6;
 
 // Reverse of one particle step: lam (x, y, ux, uy, uz) of the particle after
 // the step in, before the step out (in place); lamE / lamB receive the
 // transpose of the gather; dw the weight's derivative.  FULL handles any
 // motion (up to three zigzag segments); the light variant only motions
 // that stay in their cell and returns false for the others untouched.
-template <class R, bool FULL>
+template <class R, bool V4, bool FULL>
 __device__ __forceinline__ bool reverse_particle(int p, const State<R> &s, const R *w, const int *birth,
                                                  const Planes<R> &E, const Planes<R> &B, const Planes<R> &lamJ,
                                                  const State<R> &lam, R *lamE, R *lamB, R *dw, const Params<R> &P) {
@@ -567,43 +734,52 @@ __device__ __forceinline__ bool reverse_particle(int p, const State<R> &s, const
   const int ix = s.ix[p], iy = s.iy[p];
   const R x = s.x[p], y = s.y[p];
   const R u[3] = {s.ux[p], s.uy[p], s.uz[p]};
+  // the rest of the particle, ahead of the chain that needs it
+  const R wp = w[p], dw0 = dw[p];
+  const R lx1 = lam.x[p], ly1 = lam.y[p];
+  const R lu1[3] = {lam.ux[p], lam.uy[p], lam.uz[p]};
+  const size_t pl = (size_t)E.pitch() * P.ny;
   // 1. gather with d/dx, d/dy
-  Dual<R, 2> fd[6];
-  gather<R, Dual<R, 2>>(E, B, ix, iy, seed<R, 2>(x, 0), seed<R, 2>(y, 1), fd);
-  R f[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) f[c] = fd[c].v;
+  const Stencil<R> n = stencil(P.nx, P.ny, P.mw, ix, iy, x, y);
+  R f[6], fdx[6], fdy[6];
+  gather<true>(E.f, B.f, pl, n, f, fdx, fdy);
+  CellJ<R> l;
+  if (!FULL) l = cell_current(lamJ.f, pl, n);
   // 2. Boris + move (values)
   R uo[3], mx, my, qvz;
   boris<R, R>(u, f, f + 3, P, uo, mx, my, qvz);
   // 3. deposit with d/d(x, y, mx, my); linear in q v_z
-  AdjointSink<R, 4> sink{lamJ, Dual<R, 4>(R(0)), Dual<R, 4>(R(0))};
+  R axy, az, dxy[4], dz[4];
   if constexpr (FULL) {
+    AdjointSink<R, 4> sink{lamJ, Dual<R, 4>(R(0)), Dual<R, 4>(R(0))};
     zigzag<R, Dual<R, 4>>(sink, ix, iy, seed<R, 4>(x, 0), seed<R, 4>(y, 1), seed<R, 4>(mx, 2), seed<R, 4>(my, 3),
                           Dual<R, 4>(R(1)), P);
+    axy = sink.axy.v;
+    az = sink.az.v;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      dxy[k] = sink.axy.d[k];
+      dz[k] = sink.az.d[k];
+    }
   } else {
     const R x1 = x + mx, y1 = y + my;
     if (x1 >= R(1) || x1 < R(0) || y1 >= R(1) || y1 < R(0)) return false;
-    single_segment<R, Dual<R, 4>>(sink, ix, iy, seed<R, 4>(x, 0), seed<R, 4>(y, 1), seed<R, 4>(mx, 2),
-                                  seed<R, 4>(my, 3), Dual<R, 4>(R(1)), P);
+    segment_vjp(l, n, mx, my, P, axy, az, dxy, dz);
   }
-  const R wp = w[p];
-  dw[p] += sink.axy.v + qvz * sink.az.v;
+  dw[p] = dw0 + (axy + qvz * az);
   R gdep[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) gdep[k] = wp * (sink.axy.d[k] + qvz * sink.az.d[k]);
+  for (int k = 0; k < 4; ++k) gdep[k] = wp * (dxy[k] + qvz * dz[k]);
   // 4. cotangents of the Boris outputs, then its reverse
-  const R lx1 = lam.x[p], ly1 = lam.y[p];
-  const R lu1[3] = {lam.ux[p], lam.uy[p], lam.uz[p]};
   R lu0[3], lef[3], lbf[3];
-  boris_vjp<R>(u, f, f + 3, P, lu1, lx1 + gdep[2], ly1 + gdep[3], wp * sink.az.v, lu0, lef, lbf);
+  boris_vjp<R>(u, f, f + 3, P, lu1, lx1 + gdep[2], ly1 + gdep[3], wp * az, lu0, lef, lbf);
   // 5. position: direct (x1 = x + mx - di), deposit, and the gather weights
   const R l6[6] = {lef[0], lef[1], lef[2], lbf[0], lbf[1], lbf[2]};
   R lx = lx1 + gdep[0], ly = ly1 + gdep[1];
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
-    lx += l6[c] * fd[c].d[0];
-    ly += l6[c] * fd[c].d[1];
+    lx = fma(l6[c], fdx[c], lx);
+    ly = fma(l6[c], fdy[c], ly);
   }
   lam.x[p] = lx;
   lam.y[p] = ly;
@@ -611,92 +787,168 @@ __device__ __forceinline__ bool reverse_particle(int p, const State<R> &s, const
   lam.uy[p] = lu0[1];
   lam.uz[p] = lu0[2];
   // 6. transpose of the gather
-  scatter_add(lamE, lamB, E, ix, iy, x, y, l6);
+  if constexpr (V4) scatter_pairs(lamE, pl, n, l6);
+  else scatter_add(lamE, lamB, pl, n, l6);
   return true;
 }
 
 // the particles whose motion stays in its cell (most of them); the others
 // are listed for k_adj_push_rev_cross
-template <class R>
-__global__ void __launch_bounds__(128) k_adj_push_rev(State<R> s, const R *w, const int *birth, Planes<R> E,
-                                                      Planes<R> B, Planes<R> lamJ, State<R> lam, R *lamE, R *lamB,
-                                                      R *dw, int *cross, int *ncross, Params<R> P) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P.np; p += gridDim.x * blockDim.x)
-    if (!reverse_particle<R, false>(p, s, w, birth, E, B, lamJ, lam, lamE, lamB, dw, P))
+template <class R, bool V4>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? kRevCtas : 3)
+    k_adj_push_rev(State<R> s, const R *w, const int *birth, Planes<R> E, Planes<R> B, Planes<R> lamJ, State<R> lam,
+                   R *lamE, R *lamB, R *dw, int *cross, int *ncross, Params<R> P) {
+  const Share mine(P.np);
+  for (int p = mine.first + threadIdx.x; p < mine.end; p += blockDim.x)
+    if (!reverse_particle<R, V4, false>(p, s, w, birth, E, B, lamJ, lam, lamE, lamB, dw, P))
       cross[atomicAdd(ncross, 1)] = p;
 }
 
 // the listed cell-crossing particles
-template <class R>
+template <class R, bool V4>
 __global__ void __launch_bounds__(128) k_adj_push_rev_cross(State<R> s, const R *w, const int *birth, Planes<R> E,
                                                             Planes<R> B, Planes<R> lamJ, State<R> lam, R *lamE,
                                                             R *lamB, R *dw, const int *cross, const int *ncross,
                                                             Params<R> P) {
   const int n = *ncross;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    reverse_particle<R, true>(cross[k], s, w, birth, E, B, lamJ, lam, lamE, lamB, dw, P);
+    reverse_particle<R, V4, true>(cross[k], s, w, birth, E, B, lamJ, lam, lamE, lamB, dw, P);
 }
 
-// B -= c curl E  (yee_b with c = dt/2)
-template <class R>
-__global__ void k_adj_yee_b(const R *E, R *B, int nx, int ny, R cx, R cy) {
+// The field advance of a periodic step: Yee b/2, e, b/2 (yee_b, yee_e) in one
+// pass, from (E, B) to (En, Bn).  Every cell recomputes the half-step values of
+// its neighbours, from L1: 5 us for 256 x 256 cells, where three kernels and the
+// copies that kept the fields of a step took 20.  A4: the current is [node][4];
+// `clear`, if any, is the next step's, left zero.
+// Cells around a cell: offsets of the columns and rows lo .. lo + 3
+struct Ring {
+  unsigned c[4], r[4];
+  int lo;
+  __device__ __forceinline__ Ring(int i, int j, int nx, int ny, int lo_) : lo(lo_) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      c[k] = wrap(i + lo_ + k, nx);
+      r[k] = (unsigned)wrap(j + lo_ + k, ny) * nx;
+    }
+  }
+  __device__ __forceinline__ unsigned operator()(int a, int b) const { return r[b - lo] + c[a - lo]; }
+};
+
+template <class R, bool A4>
+__global__ void __launch_bounds__(256) k_adj_fields(const R *E, const R *B, const R *J, R *En, R *Bn, float4 *clear,
+                                                    int nx, int ny, R hx, R hy, R cx, R cy, R dt) {
   const size_t pl = (size_t)nx * ny;
+  const R *Ex = E, *Ey = E + pl, *Ez = E + 2 * pl, *Bx = B, *By = B + pl, *Bz = B + 2 * pl;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(k % nx), j = (int)(k / nx);
-    const int ip = wrap(i + 1, nx), jp = wrap(j + 1, ny);
-    const R *Ex = E, *Ey = E + pl, *Ez = E + 2 * pl;
-    B[k] += -cy * (Ez[(size_t)jp * nx + i] - Ez[k]);
-    B[pl + k] += cx * (Ez[(size_t)j * nx + ip] - Ez[k]);
-    B[2 * pl + k] += -cx * (Ey[(size_t)j * nx + ip] - Ey[k]) + cy * (Ex[(size_t)jp * nx + i] - Ex[k]);
+    const Ring at(i, j, nx, ny, -1);
+    // after the first half step of B
+    auto b1x = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return Bx[n] + -hy * (Ez[at(a, b + 1)] - Ez[n]);
+    };
+    auto b1y = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return By[n] + hx * (Ez[at(a + 1, b)] - Ez[n]);
+    };
+    auto b1z = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return Bz[n] + (-hx * (Ey[at(a + 1, b)] - Ey[n]) + hy * (Ex[at(a, b + 1)] - Ex[n]));
+    };
+    // after the step of E
+    auto cur = [&](int c, unsigned n) { return A4 ? J[4 * (size_t)n + c] : J[c * pl + n]; };
+    auto e1x = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return Ex[n] + (cy * (b1z(a, b) - b1z(a, b - 1)) - dt * cur(0, n));
+    };
+    auto e1y = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return Ey[n] + (-cx * (b1z(a, b) - b1z(a - 1, b)) - dt * cur(1, n));
+    };
+    auto e1z = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return Ez[n] + (cx * (b1y(a, b) - b1y(a - 1, b)) - cy * (b1x(a, b) - b1x(a, b - 1)) - dt * cur(2, n));
+    };
+    const R ex = e1x(0, 0), ey = e1y(0, 0), ez = e1z(0, 0);
+    En[k] = ex;
+    En[pl + k] = ey;
+    En[2 * pl + k] = ez;
+    Bn[k] = b1x(0, 0) + -hy * (e1z(0, 1) - ez);
+    Bn[pl + k] = b1y(0, 0) + hx * (e1z(1, 0) - ez);
+    Bn[2 * pl + k] = b1z(0, 0) + (-hx * (e1y(1, 0) - ey) + hy * (e1x(0, 1) - ex));
+    if (A4) clear[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-// E += dt curl B - dt J  (yee_e)
-template <class R>
-__global__ void k_adj_yee_e(R *E, const R *B, const R *J, int nx, int ny, R cx, R cy, R dt) {
+// Its transpose: (lE, lB) after the step to (ln, lbn) before it, lJ the
+// current's adjoint.  A4: the transposes of the gathers of the step after are
+// still apart, in S (scatter_pairs); `clear`, the next ones', is left zero.
+template <class R, bool A4>
+__global__ void __launch_bounds__(256) k_adj_fields_T(const R *lE, const R *lB, const R *S, R *lEn, R *lBn, R *lJ,
+                                                      float *clear, int nx, int ny, R hx, R hy, R cx, R cy, R dt) {
   const size_t pl = (size_t)nx * ny;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(k % nx), j = (int)(k / nx);
-    const int im = wrap(i - 1, nx), jm = wrap(j - 1, ny);
-    const R *Bx = B, *By = B + pl, *Bz = B + 2 * pl;
-    E[k] += cy * (Bz[k] - Bz[(size_t)jm * nx + i]) - dt * J[k];
-    E[pl + k] += -cx * (Bz[k] - Bz[(size_t)j * nx + im]) - dt * J[pl + k];
-    E[2 * pl + k] += cx * (By[k] - By[(size_t)j * nx + im]) - cy * (Bx[k] - Bx[(size_t)jm * nx + i]) - dt * J[2 * pl + k];
-  }
-}
-
-// transpose of k_adj_yee_b: lamE += transpose(-c curl) lamB
-template <class R>
-__global__ void k_adj_yee_b_T(const R *lB, R *lE, int nx, int ny, R cx, R cy) {
-  const size_t pl = (size_t)nx * ny;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(k % nx), j = (int)(k / nx);
-    const int im = wrap(i - 1, nx), jm = wrap(j - 1, ny);
-    const R *ax = lB, *ay = lB + pl, *az = lB + 2 * pl;
-    // B.x(i,j) -= cy (Ez(i,j+1) - Ez(i,j)); B.y += cx (Ez(i+1,j) - Ez(i,j));
-    // B.z += -cx (Ey(i+1,j) - Ey(i,j)) + cy (Ex(i,j+1) - Ex(i,j))
-    lE[k] += cy * (az[(size_t)jm * nx + i] - az[k]);
-    lE[pl + k] += -cx * (az[(size_t)j * nx + im] - az[k]);
-    lE[2 * pl + k] += -cy * (ax[(size_t)jm * nx + i] - ax[k]) + cx * (ay[(size_t)j * nx + im] - ay[k]);
-  }
-}
-
-// transpose of k_adj_yee_e: lamB += transpose(dt curl) lamE, lamJ = -dt lamE
-template <class R>
-__global__ void k_adj_yee_e_T(const R *lE, R *lB, R *lJ, int nx, int ny, R cx, R cy, R dt) {
-  const size_t pl = (size_t)nx * ny;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(k % nx), j = (int)(k / nx);
-    const int ip = wrap(i + 1, nx), jp = wrap(j + 1, ny);
-    const R *ax = lE, *ay = lE + pl, *az = lE + 2 * pl;
+    const Ring at(i, j, nx, ny, -2);
+    auto sum = [&](int c, unsigned n) { return A4 ? pair_at((const float *)S, pl, c, n) : R(0); };
+    auto e = [&](int c, unsigned n) { return lE[c * pl + n] + sum(c, n); };
+    auto bb = [&](int c, unsigned n) { return lB[c * pl + n] + sum(3 + c, n); };
+    // B.x(i,j) -= hy (Ez(i,j+1) - Ez(i,j)); B.y += hx (Ez(i+1,j) - Ez(i,j));
+    // B.z += -hx (Ey(i+1,j) - Ey(i,j)) + hy (Ex(i,j+1) - Ex(i,j))
+    auto e1x = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return e(0, n) + hy * (bb(2, at(a, b - 1)) - bb(2, n));
+    };
+    auto e1y = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return e(1, n) + -hx * (bb(2, at(a - 1, b)) - bb(2, n));
+    };
+    auto e1z = [&](int a, int b) {
+      const unsigned n = at(a, b);
+      return e(2, n) + (-hy * (bb(0, at(a, b - 1)) - bb(0, n)) + hx * (bb(1, at(a - 1, b)) - bb(1, n)));
+    };
     // E.x += cy (Bz(i,j) - Bz(i,j-1)); E.y += -cx (Bz(i,j) - Bz(i-1,j));
     // E.z += cx (By(i,j) - By(i-1,j)) - cy (Bx(i,j) - Bx(i,j-1))
-    lB[k] += -cy * (az[k] - az[(size_t)jp * nx + i]);
-    lB[pl + k] += cx * (az[k] - az[(size_t)j * nx + ip]);
-    lB[2 * pl + k] += cy * (ax[k] - ax[(size_t)jp * nx + i]) - cx * (ay[k] - ay[(size_t)j * nx + ip]);
-    lJ[k] = -dt * ax[k];
-    lJ[pl + k] = -dt * ay[k];
-    lJ[2 * pl + k] = -dt * az[k];
+    auto b1x = [&](int a, int b) { return bb(0, at(a, b)) + -cy * (e1z(a, b) - e1z(a, b + 1)); };
+    auto b1y = [&](int a, int b) { return bb(1, at(a, b)) + cx * (e1z(a, b) - e1z(a + 1, b)); };
+    auto b1z = [&](int a, int b) {
+      return bb(2, at(a, b)) + (cy * (e1x(a, b) - e1x(a, b + 1)) - cx * (e1y(a, b) - e1y(a + 1, b)));
+    };
+    const R ex = e1x(0, 0), ey = e1y(0, 0), ez = e1z(0, 0);
+    lJ[k] = -dt * ex;
+    lJ[pl + k] = -dt * ey;
+    lJ[2 * pl + k] = -dt * ez;
+    const R bx = b1x(0, 0), by = b1y(0, 0), bz = b1z(0, 0);
+    lBn[k] = bx;
+    lBn[pl + k] = by;
+    lBn[2 * pl + k] = bz;
+    lEn[k] = ex + hy * (b1z(0, -1) - bz);
+    lEn[pl + k] = ey + -hx * (b1z(-1, 0) - bz);
+    lEn[2 * pl + k] = ez + (-hy * (b1x(0, -1) - bx) + hx * (b1y(-1, 0) - by));
+    if (A4) {
+      float2 *pairs = reinterpret_cast<float2 *>(clear);
+      pairs[k] = pairs[pl + k] = make_float2(0.f, 0.f);
+      clear[4 * pl + k] = clear[5 * pl + k] = 0.f;
+    }
+  }
+}
+
+// [node][4] -> planes, and planes += the sums of pairs
+__global__ void k_adj_planes(const float *a, float *f, size_t pl) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
+    const float4 v = reinterpret_cast<const float4 *>(a)[k];
+    f[k] = v.x;
+    f[pl + k] = v.y;
+    f[2 * pl + k] = v.z;
+  }
+}
+__global__ void k_adj_add_planes(const float *a, float *E, float *B, size_t pl) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      E[c * pl + k] += pair_at(a, pl, c, (unsigned)k);
+      B[c * pl + k] += pair_at(a, pl, 3 + c, (unsigned)k);
+    }
   }
 }
 
@@ -968,6 +1220,12 @@ struct Engine : EngineBase {
   int *birth = nullptr;    // step at which each particle starts (null: all at 0)
   DevState<R> cur, nxt;
   R *E = nullptr, *B = nullptr, *J = nullptr, *tmp = nullptr;
+  // V4: the deposit's current [node][4] and the sums of the gathers'
+  // transposes (scatter_pairs); one of the two is added to while the other,
+  // read by the field kernel before, is zero
+  bool v4 = false;
+  float *Jn[2] = {nullptr, nullptr}, *Sn[2] = {nullptr, nullptr};
+  int jn = 0, sn = 0;
   std::vector<std::pair<R, R>> passes;  // current filter passes along x
   std::vector<char> shifts;             // window moves of the last forward run, per step
   // checkpoints (state + E + B) every K steps, and the pre-step states of
@@ -1060,15 +1318,20 @@ struct Engine : EngineBase {
     TRY_(alloc(&lamE, 3 * pl));
     TRY_(alloc(&lamB, 3 * pl));
     TRY_(alloc(&lamJ, 3 * pl));
+    v4 = sizeof(R) == 4 && !mw;
+    for (int k = 0; v4 && k < 2; ++k) {
+      TRY_(alloc(&Jn[k], 4 * pl));
+      TRY_(alloc(&Sn[k], 6 * pl));
+    }
     TRY_(alloc(&dwv, np));
     TRY_(alloc(&d_cross, np));
     TRY_(alloc(&d_ncross, 1));
     TRY_(alloc(&d_scr, 16));
     // the forward run keeps the pre-step states of its last two segments
     // when they take at most 8 GiB (the reverse sweep then recomputes one
-    // segment fewer), else of the last one
-    const double slot_bytes = (double)state_span() + 6.0 * sizeof(R) * (double)pl;
-    kseg = (2.0 * K * slot_bytes <= 8.0 * (1 << 30)) ? 2 : 1;
+    // segment fewer), else of the last one; a longer run asks for more
+    // (keep_room)
+    kseg = (2.0 * K * slot_bytes() <= 8.0 * (1 << 30)) ? 2 : 1;
     seg_s.resize((size_t)kseg * K);
     seg_f.resize((size_t)kseg * K);
     for (int k = 0; k < kseg * K; ++k) {
@@ -1158,11 +1421,9 @@ struct Engine : EngineBase {
     return ZC_OK;
   }
 
-  // keeps the pre-step fields of a step in slot k (the particles of a kept
-  // step are written there by the step before it)
-  zc_status keep_pre_fields(int k) {
-    ACK(cudaMemcpyAsync(seg_f[k], E, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(seg_f[k] + 3 * pl, B, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
+  zc_status copy_fields(R *dE, R *dB, const R *sE, const R *sB) {
+    ACK(cudaMemcpyAsync(dE, sE, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
+    ACK(cudaMemcpyAsync(dB, sB, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
     return ZC_OK;
   }
 
@@ -1181,21 +1442,32 @@ struct Engine : EngineBase {
     }
   }
 
-  // one step of the forward engine: cur -> nxt, E, B advanced
-  zc_status step(int n, double *ekin) {
-    TRY_(step_into(n, cur, nxt, ekin));
-    std::swap(cur, nxt);
-    return ZC_OK;
-  }
-
-  // one step of the forward engine: particles src -> dst, E, B advanced
-  zc_status step_into(int n, const DevState<R> &src, const DevState<R> &dst, double *ekin) {
+  // one step of the forward engine: particles src -> dst, fields (Ei, Bi) ->
+  // (Eo, Bo), other buffers unless the window moves
+  zc_status step_into(int n, const DevState<R> &src, const DevState<R> &dst, R *Ei, R *Bi, R *Eo, R *Bo,
+                      double *ekin) {
     const Params<R> P = params(n, shifts[n]);
-    ACK(cudaMemsetAsync(J, 0, sizeof(R) * 3 * pl, st));
-    k_adj_push<R><<<grid_for(np, 256), 256, 0, st>>>(src.view(np), dst.view(np), w, birth, planes(E), planes(B),
-                                                      planes(J), ekin, P);
+    const int grid = grid_for(np, 256);
+    if constexpr (sizeof(R) == 4) {
+      if (v4)
+        k_adj_push<R, true><<<grid, 256, 0, st>>>(src.view(np), dst.view(np), w, birth, planes(Ei), planes(Bi),
+                                                  planes(Jn[jn]), ekin, P);
+    }
+    if (!v4) {
+      ACK(cudaMemsetAsync(J, 0, sizeof(R) * 3 * pl, st));
+      k_adj_push<R, false><<<grid, 256, 0, st>>>(src.view(np), dst.view(np), w, birth, planes(Ei), planes(Bi),
+                                                 planes(J), ekin, P);
+    }
     ACK(cudaGetLastError());
     // current filter passes along x (current_smooth, em2d/current.c:427-459)
+    bool nodes = v4;  // the current is still [node][4]
+    if constexpr (sizeof(R) == 4) {
+      if (v4 && !passes.empty()) {
+        k_adj_planes<<<grid_for(pl), 256, 0, st>>>(Jn[jn], J, pl);
+        ACK(cudaMemsetAsync(Jn[jn], 0, sizeof(R) * 4 * pl, st));
+        nodes = false;
+      }
+    }
     for (const auto &ps : passes) {
       k_adj_smooth_x<R><<<grid_for(3 * pl), 256, 0, st>>>(J, tmp, nx, ny, mw, ps.first, ps.second);
       std::swap(J, tmp);
@@ -1203,25 +1475,29 @@ struct Engine : EngineBase {
     const R hx = (R)(0.5 * dt / dx), hy = (R)(0.5 * dt / dy);
     const R cx = (R)(dt / dx), cy = (R)(dt / dy);
     if (mw) {
-      k_adj_yee_b_mw<R><<<grid_for(pl), 256, 0, st>>>(E, B, nx, ny, hx, hy);
-      k_adj_yee_e_mw<R><<<grid_for(pl), 256, 0, st>>>(E, B, J, nx, ny, cx, cy, (R)dt);
-      k_adj_yee_b_mw<R><<<grid_for(pl), 256, 0, st>>>(E, B, nx, ny, hx, hy);
+      if (Eo != Ei) TRY_(copy_fields(Eo, Bo, Ei, Bi));
+      k_adj_yee_b_mw<R><<<grid_for(pl), 256, 0, st>>>(Eo, Bo, nx, ny, hx, hy);
+      k_adj_yee_e_mw<R><<<grid_for(pl), 256, 0, st>>>(Eo, Bo, J, nx, ny, cx, cy, (R)dt);
+      k_adj_yee_b_mw<R><<<grid_for(pl), 256, 0, st>>>(Eo, Bo, nx, ny, hx, hy);
       if (P.shift) {
-        k_adj_shift<R><<<grid_for(3 * pl), 256, 0, st>>>(E, tmp, nx, 3 * pl);
-        ACK(cudaMemcpyAsync(E, tmp, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
-        k_adj_shift<R><<<grid_for(3 * pl), 256, 0, st>>>(B, tmp, nx, 3 * pl);
-        ACK(cudaMemcpyAsync(B, tmp, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
+        k_adj_shift<R><<<grid_for(3 * pl), 256, 0, st>>>(Eo, tmp, nx, 3 * pl);
+        ACK(cudaMemcpyAsync(Eo, tmp, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
+        k_adj_shift<R><<<grid_for(3 * pl), 256, 0, st>>>(Bo, tmp, nx, 3 * pl);
+        ACK(cudaMemcpyAsync(Bo, tmp, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
       }
+    } else if (nodes) {
+      if constexpr (sizeof(R) == 4)
+        k_adj_fields<R, true><<<grid_for(pl), 256, 0, st>>>(Ei, Bi, Jn[jn], Eo, Bo, (float4 *)Jn[1 - jn], nx, ny, hx,
+                                                            hy, cx, cy, (R)dt);
+      jn = 1 - jn;
     } else {
-      k_adj_yee_b<R><<<grid_for(pl), 256, 0, st>>>(E, B, nx, ny, hx, hy);
-      k_adj_yee_e<R><<<grid_for(pl), 256, 0, st>>>(E, B, J, nx, ny, cx, cy, (R)dt);
-      k_adj_yee_b<R><<<grid_for(pl), 256, 0, st>>>(E, B, nx, ny, hx, hy);
+      k_adj_fields<R, false><<<grid_for(pl), 256, 0, st>>>(Ei, Bi, J, Eo, Bo, nullptr, nx, ny, hx, hy, cx, cy, (R)dt);
     }
     ACK(cudaGetLastError());
     return ZC_OK;
   }
 
-  zc_status save_checkpoint(const DevState<R> &from) {
+  zc_status save_checkpoint(const DevState<R> &from, const R *fE, const R *fB) {
     if (nck == (int)ck_s.size()) {
       DevState<R> s;
       R *f = nullptr;
@@ -1231,17 +1507,14 @@ struct Engine : EngineBase {
       ck_f.push_back(f);
     }
     TRY_(copy_state(ck_s[nck], from));
-    ACK(cudaMemcpyAsync(ck_f[nck], E, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(ck_f[nck] + 3 * pl, B, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
+    TRY_(copy_fields(ck_f[nck], ck_f[nck] + 3 * pl, fE, fB));
     ++nck;
     return ZC_OK;
   }
 
-  zc_status restore_checkpoint(int k, const DevState<R> &to) {
+  zc_status restore_checkpoint(int k, const DevState<R> &to, R *tE, R *tB) {
     TRY_(copy_state(to, ck_s[k]));
-    ACK(cudaMemcpyAsync(E, ck_f[k], sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(B, ck_f[k] + 3 * pl, sizeof(R) * 3 * pl, cudaMemcpyDeviceToDevice, st));
-    return ZC_OK;
+    return copy_fields(tE, tB, ck_f[k], ck_f[k] + 3 * pl);
   }
 
   // the objective of the current fields; with seed, the adjoint of its
@@ -1262,9 +1535,41 @@ struct Engine : EngineBase {
     return ZC_OK;
   }
 
+  double slot_bytes() const { return (double)state_span() + 6.0 * sizeof(R) * (double)pl; }
+
+  // Room for the pre-step states of nsteps steps, as far as 8 GiB go; without
+  // the memory the reverse sweep recomputes more.  (200 steps of 10^6 particles
+  // take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep of 33.)
+  zc_status keep_room(int nsteps) {
+    const int want = (nsteps - 1) / K + 1;
+    const int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
+    if (fit <= kseg) return ZC_OK;
+    const int more = (fit - kseg) * K;
+    const size_t a = (state_span() + 255) / 256 * 256, b = (6 * sizeof(R) * pl + 255) / 256 * 256;
+    char *m = nullptr;
+    if (cudaMalloc((void **)&m, (a + b) * more) != cudaSuccess) {
+      cudaGetLastError();
+      return ZC_OK;
+    }
+    owned.push_back(m);
+    const size_t off = (3 * sizeof(int) * (size_t)np + 15) / 16 * 16;
+    for (int k = 0; k < more; ++k, m += a + b) {
+      DevState<R> s;
+      s.ix = reinterpret_cast<int *>(m);
+      s.iy = s.ix + np;
+      s.alive = s.iy + np;
+      s.v = reinterpret_cast<R *>(m + off);
+      seg_s.push_back(s);
+      seg_f.push_back(reinterpret_cast<R *>(m + a));
+    }
+    kseg = fit;
+    return ZC_OK;
+  }
+
   zc_status forward(int nsteps, double *obj, double *kin) override {
     if (!have_state) return afail(ZC_ESTATE, "adjoint engine: no initial state");
     if (nsteps <= 0) return afail(ZC_EINVAL, "adjoint engine: nsteps must be > 0");
+    TRY_(keep_room(nsteps));
     plan_shifts(nsteps);
     ACK(cudaEventRecord(e0, st));
     nck = 0;
@@ -1274,18 +1579,33 @@ struct Engine : EngineBase {
     // reverse sweep starts with them and need not recompute those segments
     const int last0 = ((nsteps - 1) / K) * K;
     keep0 = std::max(0, last0 - (kseg - 1) * K);
+    if (v4) {
+      ACK(cudaMemsetAsync(Jn[0], 0, sizeof(R) * 4 * pl, st));
+      jn = 0;
+    }
     for (int n = 0; n < nsteps; ++n) {
       double *ek = n == nsteps - 1 ? d_scr + 1 : nullptr;
       if (n < keep0) {
-        if (n % K == 0) TRY_(save_checkpoint(cur));
-        TRY_(step(n, ek));
+        if (n % K == 0) TRY_(save_checkpoint(cur, E, B));
+        if (mw) {
+          TRY_(step_into(n, cur, nxt, E, B, E, B, ek));
+        } else {  // (the adjoint fields' buffers are free until the reverse sweep)
+          TRY_(step_into(n, cur, nxt, E, B, lamE, lamB, ek));
+          std::swap(E, lamE);
+          std::swap(B, lamB);
+        }
+        std::swap(cur, nxt);
         continue;
       }
       const int k = n - keep0;
-      if (k == 0) TRY_(copy_state(seg_s[0], cur));
-      if (n % K == 0) TRY_(save_checkpoint(seg_s[k]));
-      TRY_(keep_pre_fields(k));
-      TRY_(step_into(n, seg_s[k], n + 1 < nsteps ? seg_s[k + 1] : cur, ek));
+      if (k == 0) {
+        TRY_(copy_state(seg_s[0], cur));
+        TRY_(copy_fields(seg_f[0], seg_f[0] + 3 * pl, E, B));
+      }
+      if (n % K == 0) TRY_(save_checkpoint(seg_s[k], seg_f[k], seg_f[k] + 3 * pl));
+      const bool more = n + 1 < nsteps;
+      TRY_(step_into(n, seg_s[k], more ? seg_s[k + 1] : cur, seg_f[k], seg_f[k] + 3 * pl, more ? seg_f[k + 1] : E,
+                     more ? seg_f[k + 1] + 3 * pl : B, ek));
     }
     steps_done = nsteps;
     ACK(cudaEventRecord(e1, st));
@@ -1318,15 +1638,35 @@ struct Engine : EngineBase {
       k_adj_yee_b_T_mw<R><<<grid_for(pl), 256, 0, st>>>(lamB, lamE, nx, ny, hx, hy);
       k_adj_yee_e_T_mw<R><<<grid_for(pl), 256, 0, st>>>(lamE, lamB, lamJ, nx, ny, cx, cy, (R)dt);
       k_adj_yee_b_T_mw<R><<<grid_for(pl), 256, 0, st>>>(lamB, lamE, nx, ny, hx, hy);
-    } else {
-      k_adj_yee_b_T<R><<<grid_for(pl), 256, 0, st>>>(lamB, lamE, nx, ny, hx, hy);
-      k_adj_yee_e_T<R><<<grid_for(pl), 256, 0, st>>>(lamE, lamB, lamJ, nx, ny, cx, cy, (R)dt);
-      k_adj_yee_b_T<R><<<grid_for(pl), 256, 0, st>>>(lamB, lamE, nx, ny, hx, hy);
+    } else {  // into the forward fields' buffers, which the sweep no longer needs
+      if constexpr (sizeof(R) == 4)
+        k_adj_fields_T<R, true><<<grid_for(pl), 256, 0, st>>>(lamE, lamB, Sn[sn], E, B, lamJ, Sn[1 - sn], nx,
+                                                              ny, hx, hy, cx, cy, (R)dt);
+      else
+        k_adj_fields_T<R, false><<<grid_for(pl), 256, 0, st>>>(lamE, lamB, nullptr, E, B, lamJ, nullptr, nx, ny, hx,
+                                                               hy, cx, cy, (R)dt);
+      sn = 1 - sn;
+      std::swap(E, lamE);
+      std::swap(B, lamB);
     }
     for (int k = (int)passes.size() - 1; k >= 0; --k) {
       k_adj_smooth_x_T<R><<<grid_for(3 * pl), 256, 0, st>>>(lamJ, tmp, nx, ny, mw, passes[k].first, passes[k].second);
       std::swap(lamJ, tmp);
     }
+    ACK(cudaGetLastError());
+    return ZC_OK;
+  }
+
+  // the particle part of a reverse step; gE, gB receive the gathers' transpose
+  template <bool V4>
+  zc_status push_reverse(const DevState<R> &s, R *f, R *gE, R *gB, const Params<R> &P) {
+    ACK(cudaMemsetAsync(d_ncross, 0, sizeof(int), st));
+    const int grid = std::min(grid_for(np, 128), 152 * (sizeof(R) == 4 ? kRevCtas : 3));
+    k_adj_push_rev<R, V4><<<grid, 128, 0, st>>>(s.view(np), w, birth, planes(f), planes(f + 3 * pl), planes(lamJ),
+                                                lam.view(np), gE, gB, dwv, d_cross, d_ncross, P);
+    k_adj_push_rev_cross<R, V4><<<grid_for(np / 4, 128), 128, 0, st>>>(s.view(np), w, birth, planes(f),
+                                                                       planes(f + 3 * pl), planes(lamJ), lam.view(np),
+                                                                       gE, gB, dwv, d_cross, d_ncross, P);
     ACK(cudaGetLastError());
     return ZC_OK;
   }
@@ -1339,6 +1679,11 @@ struct Engine : EngineBase {
     TRY_(objective(nullptr, true));
     ACK(cudaMemsetAsync(lam.v, 0, sizeof(R) * 5 * (size_t)np, st));
     ACK(cudaMemsetAsync(dwv, 0, sizeof(R) * np, st));
+    if (v4) {
+      ACK(cudaMemsetAsync(Sn[0], 0, sizeof(R) * 6 * pl, st));
+      ACK(cudaMemsetAsync(Jn[0], 0, sizeof(R) * 4 * pl, st));
+      sn = jn = 0;
+    }
     for (int sgi = nck - 1; sgi >= 0; --sgi) {
       const int n0 = sgi * K, n1 = std::min(steps_done, n0 + K);
       // slots of this segment: kept by the forward run, or recomputed from
@@ -1347,10 +1692,11 @@ struct Engine : EngineBase {
       const bool kept = n0 >= keep0;
       const int s0 = kept ? n0 - keep0 : 0;
       if (!kept) {
-        TRY_(restore_checkpoint(sgi, seg_s[0]));
-        for (int n = n0; n < n1; ++n) {
-          TRY_(keep_pre_fields(n - n0));
-          if (n + 1 < n1) TRY_(step_into(n, seg_s[n - n0], seg_s[n - n0 + 1], nullptr));
+        TRY_(restore_checkpoint(sgi, seg_s[0], seg_f[0], seg_f[0] + 3 * pl));
+        for (int n = n0; n + 1 < n1; ++n) {
+          const int k = n - n0;
+          TRY_(step_into(n, seg_s[k], seg_s[k + 1], seg_f[k], seg_f[k] + 3 * pl, seg_f[k + 1], seg_f[k + 1] + 3 * pl,
+                         nullptr));
         }
       }
       // walk the segment backwards
@@ -1359,14 +1705,15 @@ struct Engine : EngineBase {
         TRY_(field_reverse(n));
         const Params<R> P = params(n, shifts[n]);
         ACK(cudaMemsetAsync(d_ncross, 0, sizeof(int), st));
-        k_adj_push_rev<R><<<grid_for(np, 128), 128, 0, st>>>(seg_s[k].view(np), w, birth, planes(seg_f[k]),
-                                                              planes(seg_f[k] + 3 * pl), planes(lamJ), lam.view(np),
-                                                              lamE, lamB, dwv, d_cross, d_ncross, P);
-        k_adj_push_rev_cross<R><<<grid_for(np / 4, 128), 128, 0, st>>>(
-            seg_s[k].view(np), w, birth, planes(seg_f[k]), planes(seg_f[k] + 3 * pl), planes(lamJ), lam.view(np),
-            lamE, lamB, dwv, d_cross, d_ncross, P);
-        ACK(cudaGetLastError());
+        if constexpr (sizeof(R) == 4) {
+          if (v4) TRY_((push_reverse<true>(seg_s[k], seg_f[k], Sn[sn], nullptr, P)));
+        }
+        if (!v4) TRY_((push_reverse<false>(seg_s[k], seg_f[k], lamE, lamB, P)));
       }
+    }
+    if constexpr (sizeof(R) == 4) {
+      if (v4) k_adj_add_planes<<<grid_for(pl), 256, 0, st>>>(Sn[sn], lamE, lamB, pl);
+      ACK(cudaGetLastError());
     }
     ACK(cudaEventRecord(e1, st));
     const State<R> l = lam.view(np);
@@ -1379,7 +1726,7 @@ struct Engine : EngineBase {
     TRY_(download(dEh, lamE, 3 * pl));
     TRY_(download(dBh, lamB, 3 * pl));
     // the engine's state goes back to the start of the run
-    TRY_(restore_checkpoint(0, cur));
+    TRY_(restore_checkpoint(0, cur, E, B));
     ACK(cudaStreamSynchronize(st));
     cudaEventElapsedTime(&bwd_ms, e0, e1);
     steps_done = 0;
