@@ -19,6 +19,7 @@ struct PushConst {
   // sums in units of 2^-40 take each integer times js_det (2^40 / js)
   float js, js_invl, js_twol, js_inv2l, js_two2l, js_lo;
   int js_l;
+  int js_run;                             // |v| js < 2^43: a lane's sums of two parts hold it (RunSums)
   long long js_det;
 };
 

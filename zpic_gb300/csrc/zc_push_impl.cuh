@@ -16,9 +16,8 @@
 //                 kept sorted by cell, so the lanes of a warp mostly share a
 //                 cell: their gathers are broadcasts, and the current of the
 //                 segment of a particle that stays in its cell is summed in
-//                 the lane's registers (deterministic builds: across the lanes
-//                 of a cell, with a segmented warp-shuffle reduction) before
-//                 it is deposited.  The fast and exact builds deposit with
+//                 the lane's registers (deterministic builds: as integers)
+//                 before it is deposited.  The fast and exact builds deposit with
 //                 float reductions on the global J planes, which L2 performs
 //                 natively; the deterministic builds accumulate a shared
 //                 integer J tile (exact, order-independent sums) and add it
@@ -113,6 +112,8 @@ template <class LAY>
 struct TileCurrentSplit {
   int *p;  // planes h, m, l of LAY::N nodes each
   const PushConst *C;
+  __device__ __forceinline__ static int column(unsigned cell) { return (int)(cell & (LAY::WX - 3)); }
+  __device__ __forceinline__ static int row(unsigned cell) { return (int)((cell >> 16) & (LAY::HY - 3)); }
   __device__ __forceinline__ void add(int c, int i, int j, float v) const {
     int h, m, l;
     jsplit(v, *C, h, m, l);
@@ -309,6 +310,50 @@ __device__ __forceinline__ void add_current(const D &dep, int ix, int iy, const 
   dep.add(2, ix + 1, iy + 1, c.v[7]);
 }
 
+// A lane's running sums of the deterministic builds: each contribution counts
+// as rint(v js) = h 2^22 + l, |l| <= 2^21, and |h| <= 2^21 where |v| js < 2^43
+// (PushConst::js_run); 512 of them fit 32 bits.  Two parts are enough for sums
+// that short; the tile's sums take the three of jsplit.
+struct RunSums {
+  int h[8], l[8];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) h[q] = l[q] = 0;
+  }
+  __device__ __forceinline__ void add(const SegCurrent &cur, float js) {
+    constexpr int pa[4] = {0, 1, 4, 5};  // pairs (0, 2), (1, 3), (4, 6), (5, 7), as they were computed
+    const float2 sh = make_float2(kShifter, kShifter);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int q = pa[k];
+      const float2 x = __fmul2_rn(make_float2(cur.v[q], cur.v[q + 2]), make_float2(js, js));  // exact
+      const float2 th = __ffma2_rn(x, make_float2(0x1p-22f, 0x1p-22f), sh);
+      const float2 r =  // exact remainder
+          __ffma2_rn(__ffma2_rn(th, make_float2(-1.f, -1.f), sh), make_float2(0x1p22f, 0x1p22f), x);
+      const float2 tl = __fadd2_rn(r, sh);
+      h[q] += __float_as_int(th.x) - kShifterBits;
+      h[q + 2] += __float_as_int(th.y) - kShifterBits;
+      l[q] += __float_as_int(tl.x) - kShifterBits;
+      l[q + 2] += __float_as_int(tl.y) - kShifterBits;
+    }
+  }
+  // to the tile's three planes, as jsplit cuts an integer; the sums start again
+  template <class DEP>
+  __device__ __forceinline__ void flush(const DEP &dep, unsigned cell) {
+    const int i = DEP::column(cell), j = DEP::row(cell), L = dep.C->js_l;
+    constexpr int c[8] = {0, 0, 1, 1, 2, 2, 2, 2}, di[8] = {0, 0, 0, 1, 0, 1, 0, 1}, dj[8] = {0, 1, 0, 0, 0, 0, 1, 1};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const long long v = (long long)h[q] * (1 << 22) + l[q];
+      const int vl = (int)((unsigned)v << (32 - L)) >> (32 - L);
+      const long long w = (v - vl) >> L;
+      const int vm = (int)((unsigned)w << (32 - L)) >> (32 - L);
+      dep.addi(c[q], i + di[q], j + dj[q], (int)((w - vm) >> L), vm, vl);
+      h[q] = l[q] = 0;
+    }
+  }
+};
+
 // splits segment `a` at the y cell edge: `a` keeps the part before the edge,
 // the returned segment holds the rest (particles.c:842-871)
 __device__ __forceinline__ Seg split_y(Seg &a, int dj) {
@@ -488,12 +533,13 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 // no block-wide barrier.
 //
 // Every warp takes an equal, contiguous share of the tile's slots, 32 slots
-// (a unit) at a time.  In the float builds lane l meets the particles
-// l kLaneRun ... l kLaneRun + kLaneRun - 1 of a chunk of the sorted order one
-// after another, and sums their single-segment currents in registers while
-// they stay in one cell; a lane adds its sums to J when its cell changes.
-// The deterministic builds read every chunk in cell order across the lanes
-// and pre-reduce with segmented warp sums of fixed-point parts.
+// (a unit) at a time.  Lane l meets the particles l kLaneRun ...
+// l kLaneRun + kLaneRun - 1 of a chunk of the sorted order one after another,
+// and sums their single-segment currents in registers while they stay in one
+// cell; a lane adds its sums to J when its cell changes.  The deterministic
+// builds do that with integers (RunSums): 118 us for 4.2 M particles on 512^2
+// cells, where the sums over the lanes of a cell, with 24 words a shuffle
+// step, took 188 to 213; 354 against 683 us for 16.8 M.
 //
 // What bounds it (fast build, 2048^2 cells, 67 M particles): no single unit.
 // A launch takes 0.940 ms against 0.49 ms for its 48 bytes a particle at the
@@ -502,9 +548,9 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 // use, and a third of a warp's time spent waiting for its next particles.
 // It took 0.993 ms and 446 instructions a unit (307 now) before the work of
 // cell-crossing particles moved out of the main loop, the float pairs, the
-// contiguous shares and the particle prefetch in registers; writing the tile back in cell order from here (in
-// place of the sort pass) was slower (1.13 ms): scattered 16-byte stores
-// make L2 fetch what they do not cover.
+// contiguous shares and the particle prefetch in registers; writing the tile
+// back in cell order from here (in place of the sort pass) was slower
+// (1.13 ms): scattered 16-byte stores make L2 fetch what they do not cover.
 // ---------------------------------------------------------------------------
 // resident CTAs per SM the float builds are compiled for: 6 (up to 80
 // registers a thread) measured faster than 7 (72, spilling in the main loop;
@@ -514,6 +560,9 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 #ifndef ZC_PUSH_MIN_CTAS
 #define ZC_PUSH_MIN_CTAS 6
 #endif
+// the deterministic builds: 768 threads per SM (80 registers each; 512^2, 32 x
+// 16 tiles: 118 us; 512 threads, no spills: 120; 1024, 64 registers: 199)
+constexpr int kDetThreads = 768;
 //
 // SPLIT: a tile is worked on by a cluster of `parts` CTAs (this one is
 // `rank`), for grids with too few tiles to fill the GPU.  Each stages the
@@ -606,10 +655,6 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   const int c_end = min(n_own, c_begin + 32 * (share + (gwarp < extra ? 1 : 0)));
   // this lane's slot in the unit that starts at slot c
   const auto slot_of = [&](int c) {
-    if constexpr (DET) {
-      const int c0 = c & ~(kChunk - 1), j = (c & (kChunk - 1)) + lane;
-      if (c0 + kChunk <= n_own) return c0 + (j % kLaneRun) * 32 + j / kLaneRun;
-    }
     return c + lane;
   };
   // a lane without a particle carries the last unit's particle, a hole's
@@ -677,12 +722,13 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   }();
   float ks = 0.f, kc = 0.f;
   long long khi = 0, klo = 0;  // DET: fixed-point kinetic energy of this thread's particles
-  // float builds: this lane's running single-segment current and its cell
-  // word (kHole: none)
+  // this lane's running single-segment current and its cell word (kHole: none)
   SegCurrent acc;
 #pragma unroll
   for (int q = 0; q < 8; ++q) acc.v[q] = 0.f;
-  unsigned acc_cell = kHole;
+  RunSums run;  // DET: the same as integers
+  run.clear();
+  unsigned acc_cell = kHole, nadd = 0;
   // the bits of a cell word that all cells of this tile share
   const unsigned tile_mask = ~((unsigned)(TX - 1) | (unsigned)(TY - 1) << 16);
   const unsigned tile_word = (unsigned)cx0 | (unsigned)cy0 << 16;
@@ -834,46 +880,18 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
     SegCurrent cur = segment_current(a, Cl.qnx, Cl.qny);
 
     if constexpr (DET) {
-      // segmented warp reduction of the single-segment currents over runs
-      // of lanes that start in the same cell (the lanes read the chunk in
-      // cell order), as many halving steps as the longest run needs; each
-      // lane's contributions rounded to fixed point first, then summed as
+      // every contribution rounded to fixed point first, then summed as
       // integers: the same total whatever lanes hold which particles
-      const int key = valid ? (li + lj * TX) : -1 - lane;
-      const int knext = __shfl_down_sync(0xffffffffu, key, 1);
-      const int kprev = __shfl_up_sync(0xffffffffu, key, 1);
-      const unsigned lastmask = __ballot_sync(0xffffffffu, lane == 31 || knext != key);
-      const int run_last = __ffs(lastmask & (0xffffffffu << lane)) - 1;
-      const unsigned maxlen = __reduce_max_sync(0xffffffffu, (unsigned)(run_last - lane + 1));
-      const bool head = valid && (lane == 0 || kprev != key);
-      int ih[8], im[8], il[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) jsplit(cur.v[q], Cl, ih[q], im[q], il[q]);
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        if ((unsigned)off >= maxlen) break;
-        const bool take = lane + off <= run_last;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int oh = __shfl_down_sync(0xffffffffu, ih[q], off);
-          const int om = __shfl_down_sync(0xffffffffu, im[q], off);
-          const int ol = __shfl_down_sync(0xffffffffu, il[q], off);
-          if (take) {
-            ih[q] += oh;
-            im[q] += om;
-            il[q] += ol;
-          }
-        }
-      }
-      if (head) {
-        dep.addi(0, li, lj, ih[0], im[0], il[0]);
-        dep.addi(0, li, lj + 1, ih[1], im[1], il[1]);
-        dep.addi(1, li, lj, ih[2], im[2], il[2]);
-        dep.addi(1, li + 1, lj, ih[3], im[3], il[3]);
-        dep.addi(2, li, lj, ih[4], im[4], il[4]);
-        dep.addi(2, li + 1, lj, ih[5], im[5], il[5]);
-        dep.addi(2, li, lj + 1, ih[6], im[6], il[6]);
-        dep.addi(2, li + 1, lj + 1, ih[7], im[7], il[7]);
+      if (Cl.js_run) {
+        // the lane's running sums: to the J tile when its cell changes, and
+        // before they can overflow
+        const bool full = (++nadd & 511) == 0;
+        const bool change = (single && cw != acc_cell) || full;
+        if (change && acc_cell != kHole) run.flush(dep, acc_cell);
+        run.add(cur, Cl.js);
+        acc_cell = single ? cw : (full ? kHole : acc_cell);
+      } else if (single) {  // charges that the sums' two parts are too short for
+        add_current(dep, li, lj, cur);
       }
     } else {
       // the lane's running sum: added to J when the lane's cell changes
@@ -932,10 +950,9 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   // own slots, 32 at a time (a unit), the next unit loaded into registers
   // while one is pushed (staging it in shared memory costs as many
   // shared-memory passes as half the field gather).  In a full chunk lane l
-  // of the float builds takes slot 32 k + l at step k, which holds the
-  // chunk's particle l kLaneRun + k in cell order; the deterministic builds
-  // take the particle 32 k + l of the cell order, at its tile_slot.  Every
-  // particle goes back to the slot it came from.
+  // takes slot 32 k + l at step k, which holds the chunk's particle
+  // l kLaneRun + k in cell order.  Every particle goes back to the slot it came
+  // from.
   for (int c = c_begin; c < c_end;) {
     const float4 uu = nu;
     const unsigned cw = (unsigned)__float_as_int(uu.w);
@@ -972,8 +989,10 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   }
 
   finish();  // what is left in the queue
-  if constexpr (!DET)  // the lanes' last sums
-    if (acc_cell != kHole) add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
+  if (acc_cell != kHole) {  // the lanes' last sums
+    if constexpr (DET) run.flush(dep, acc_cell);
+    else add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
+  }
 
   if constexpr (SPLIT) {
     cluster_arrive();  // every part's leavers and arrivals are counted
@@ -1095,7 +1114,7 @@ __device__ __forceinline__ void push_spill(const float *EB, const FixedJ &fj, co
 // particles in one launch
 // ---------------------------------------------------------------------------
 template <int TX, int TY, int NT, bool DET>
-__global__ void __launch_bounds__(NT, DET ? 1024 / NT : ZC_PUSH_MIN_CTAS)
+__global__ void __launch_bounds__(NT, DET ? kDetThreads / NT : ZC_PUSH_MIN_CTAS)
     k_push_tiles(const __grid_constant__ CUtensorMap tm_eb, const __grid_constant__ PushSpecies A, int *err,
                  FixedJ fj) {
   push_tile<TX, TY, NT, DET, false>(tm_eb, A, err, fj, blockIdx.x, 0, 1);
@@ -1108,7 +1127,7 @@ __global__ void __launch_bounds__(NT) k_push_spill(const float *EB, FixedJ fj, G
 }
 
 template <int TX, int TY, int NT, bool DET>
-__global__ void __launch_bounds__(NT, DET ? 512 / NT : 4)
+__global__ void __launch_bounds__(NT, DET ? kDetThreads / NT : 4)
     k_push_all(const __grid_constant__ CUtensorMap tm_eb, const __grid_constant__ PushAll P, const float *EB, Grid G,
                int *err, FixedJ fj) {
   const int b = blockIdx.x, ntile = P.nsp * P.ntiles * P.parts;
