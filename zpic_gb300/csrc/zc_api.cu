@@ -970,6 +970,7 @@ YeeConst yee_const(const zc_sim *s) {
   Y.cye = s->dt / s->dx[1];
   Y.dt = s->dt;
   Y.mw = s->mw;
+  Y.shift = 0;
   return Y;
 }
 
@@ -984,10 +985,16 @@ ZeroWords next_spill_counts(zc_sim *s) {
   return zero;
 }
 
+// whether the window moves after iteration `iter` (emf.c:650)
+bool window_moves(const zc_sim *s, int iter) { return s->mw && (iter * s->dt) > s->dx[0] * (s->n_move + 1); }
+
 // a field advance is done: counters, window move (emf_move_window, emf.c:650)
-zc_status emf_advanced(zc_sim *s) {
+// unless the field kernel made it
+zc_status emf_advanced(zc_sim *s, bool shifted = false) {
   s->iter += 1;
-  if (s->mw && (s->iter * s->dt) > s->dx[0] * (s->n_move + 1)) {
+  if (shifted) {
+    s->n_move += 1;
+  } else if (window_moves(s, s->iter)) {
     Phase ph(s, ZC_PHASE_WINDOW, 1);
     const int o = 1 - s->eb_cur;
     CK(launch_window_shift(s->EB[s->eb_cur], s->EB[o], s->G, s->st));
@@ -1043,17 +1050,19 @@ zc_status fields_impl(zc_sim *s, double *epart, bool *done) {
     std::memcpy(X.v0, v, sizeof v);
   }
   const ZeroWords zero = next_spill_counts(s);
+  YeeConst Y = yee_const(s);
+  Y.shift = !s->EBp && window_moves(s, s->iter + 1);
   {
     Phase ph(s, ZC_PHASE_YEE, 1);
     CK(launch_fields(&s->tmY_EB[s->eb_cur], &s->tmF_J[s->jr], raw_j(s), s->J[1], s->J[s->jr ? 0 : 2], s->EB[o], X,
-                     s->G, yee_const(s), px, py, s->d_err, epart, zero, s->st));
+                     s->G, Y, px, py, s->d_err, epart, zero, s->st));
   }
   s->jr ^= 1;
   s->j0_zero = true;
   s->j_cur = 1;
   s->j_plain = px.n == 0 && py.n == 0;
   s->eb_cur = o;
-  return emf_advanced(s);
+  return emf_advanced(s, Y.shift);
 }
 
 // Before a call that works on the raw current by itself: without a filter it

@@ -470,9 +470,19 @@ __global__ void __launch_bounds__(32 * kS4Warps, ZC_S4_MINB) k_smooth4(const flo
 // Out of place: EB in (TMA) -> EB out.
 // ---------------------------------------------------------------------------
 // a field value stored at (bx, by), with external fields also where the
-// particles read it (emf_update_part_fld, em2d/emf.c:838-914)
-__device__ __forceinline__ void put_field(float *EB, const ExtField &X, const Grid &G, int c, int bx, int by, float v) {
+// particles read it (emf_update_part_fld, em2d/emf.c:838-914).  shift: the
+// window moves after this step, so the value goes one cell left and the
+// right-most columns become zero (emf_move_window, em2d/emf.c:648-675; never
+// with external fields).  A move of a 2000 x 256 grid by a launch of its own
+// took 9 us; 16 steps of the wakefield 2205 us, now 2153.
+__device__ __forceinline__ void put_field(float *EB, const ExtField &X, const Grid &G, int c, int bx, int by, float v,
+                                          int shift) {
   const size_t k = gidx(G, c, bx, by);
+  if (shift) {
+    if (bx >= 1 && bx <= G.nx) EB[k - 1] = v;
+    if (bx >= G.nx) EB[k] = 0.f;
+    return;
+  }
   EB[k] = v;
   if (X.out) {
     const int t = c < 3 ? X.Et : X.Bt;
@@ -484,11 +494,11 @@ __device__ __forceinline__ void put_field(float *EB, const ExtField &X, const Gr
 
 // a value stored at (bx, by) and at its periodic guard images (xm, ym; -1: none)
 __device__ __forceinline__ void put_mirrored(float *EB, const ExtField &X, const Grid &G, int c, int bx, int by,
-                                             int xm, int ym, float v) {
-  put_field(EB, X, G, c, bx, by, v);
-  if (xm >= 0) put_field(EB, X, G, c, xm, by, v);
-  if (ym >= 0) put_field(EB, X, G, c, bx, ym, v);
-  if (xm >= 0 && ym >= 0) put_field(EB, X, G, c, xm, ym, v);
+                                             int xm, int ym, float v, int shift) {
+  put_field(EB, X, G, c, bx, by, v, shift);
+  if (xm >= 0) put_field(EB, X, G, c, xm, by, v, shift);
+  if (ym >= 0) put_field(EB, X, G, c, bx, ym, v, shift);
+  if (xm >= 0 && ym >= 0) put_field(EB, X, G, c, xm, ym, v, shift);
 }
 
 // J of the output tile and the row and column past it
@@ -543,7 +553,7 @@ __device__ __forceinline__ void yee_tile(float *sEB, const YeeCurrent &J, int bx
         z[G.plane] = 0.f;
         z[2 * G.plane] = 0.f;
       }
-      float *o = EBout + at;
+      float *o = EBout + at - Y.shift;
       o[0] = Ex[k];
       o += G.plane;
       o[0] = Ey[k];
@@ -611,19 +621,19 @@ __device__ __forceinline__ void yee_tile(float *sEB, const YeeCurrent &J, int bx
       if (gxc || gyc) continue;
       const int xm = Y.mw ? -1 : (bx == nx ? 0 : (bx <= 2 ? nx + bx : -1));
       const int ym = by == ny ? 0 : (by <= 2 ? ny + by : -1);
-      put_mirrored(EBout, ext, G, 0, bx, by, xm, ym, Ex[s]);
-      put_mirrored(EBout, ext, G, 1, bx, by, xm, ym, Ey[s]);
-      put_mirrored(EBout, ext, G, 2, bx, by, xm, ym, Ez[s]);
-      put_mirrored(EBout, ext, G, 3, bx, by, xm, ym, bxv);
-      put_mirrored(EBout, ext, G, 4, bx, by, xm, ym, byv);
-      put_mirrored(EBout, ext, G, 5, bx, by, xm, ym, bzv);
+      put_mirrored(EBout, ext, G, 0, bx, by, xm, ym, Ex[s], Y.shift);
+      put_mirrored(EBout, ext, G, 1, bx, by, xm, ym, Ey[s], Y.shift);
+      put_mirrored(EBout, ext, G, 2, bx, by, xm, ym, Ez[s], Y.shift);
+      put_mirrored(EBout, ext, G, 3, bx, by, xm, ym, bxv, Y.shift);
+      put_mirrored(EBout, ext, G, 4, bx, by, xm, ym, byv, Y.shift);
+      put_mirrored(EBout, ext, G, 5, bx, by, xm, ym, bzv, Y.shift);
     } else {
-      put_field(EBout, ext, G, 0, bx, by, Ex[s]);
-      put_field(EBout, ext, G, 1, bx, by, Ey[s]);
-      put_field(EBout, ext, G, 2, bx, by, Ez[s]);
-      put_field(EBout, ext, G, 3, bx, by, bxv);
-      put_field(EBout, ext, G, 4, bx, by, byv);
-      put_field(EBout, ext, G, 5, bx, by, bzv);
+      put_field(EBout, ext, G, 0, bx, by, Ex[s], Y.shift);
+      put_field(EBout, ext, G, 1, bx, by, Ey[s], Y.shift);
+      put_field(EBout, ext, G, 2, bx, by, Ez[s], Y.shift);
+      put_field(EBout, ext, G, 3, bx, by, bxv, Y.shift);
+      put_field(EBout, ext, G, 4, bx, by, byv, Y.shift);
+      put_field(EBout, ext, G, 5, bx, by, bzv, Y.shift);
     }
     if (epart && bx >= 1 && bx <= nx && by >= 1 && by <= ny) {
       se[0] += Ex[s] * Ex[s];

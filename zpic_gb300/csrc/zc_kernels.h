@@ -243,6 +243,7 @@ struct YeeConst {
   float cxb, cyb;                         // (dt/2)/dx, (dt/2)/dy  (emf.c:507-508)
   float cxe, cye, dt;                     // dt/dx, dt/dy, dt      (emf.c:540-541)
   int mw;                                 // moving window: x guard cells are not periodic
+  int shift;                              // the window moves after this step: fields stored one cell left
 };
 
 cudaError_t launch_aos_to_planes(const float *aos, float *planes, const Grid &G, int ncomp, cudaStream_t st);
