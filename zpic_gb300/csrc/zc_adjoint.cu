@@ -1128,23 +1128,6 @@ __global__ void k_adj_objective(const R *E, const R *B, R *lE, R *lB, int nx, in
   if (threadIdx.x == 0 && acc) atomicAdd(acc, s);
 }
 
-// sum of squares of n values (field energy), double accumulation
-template <class R>
-__global__ void k_adj_sumsq(const R *f, size_t n, double *out) {
-  __shared__ double sred[8];
-  double s = 0;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    s += (double)f[k] * (double)f[k];
-  s = zc::block_sum_double<256>(s, sred);
-  if (threadIdx.x == 0) atomicAdd(out, s);
-}
-
-template <class R>
-__global__ void k_adj_scale(const R *src, R *dst, size_t n, R a) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    dst[k] = a * src[k];
-}
-
 template <class R>
 __global__ void k_to_double(const R *src, double *dst, size_t n) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
@@ -1319,9 +1302,11 @@ struct Engine : EngineBase {
     TRY_(alloc(&lamB, 3 * pl));
     TRY_(alloc(&lamJ, 3 * pl));
     v4 = sizeof(R) == 4 && !mw;
-    for (int k = 0; v4 && k < 2; ++k) {
-      TRY_(alloc(&Jn[k], 4 * pl));
-      TRY_(alloc(&Sn[k], 6 * pl));
+    if (v4) {
+      TRY_(alloc(&Jn[0], 2 * (4 + 6) * pl));
+      Jn[1] = Jn[0] + 4 * pl;
+      Sn[0] = Jn[1] + 4 * pl;
+      Sn[1] = Sn[0] + 6 * pl;
     }
     TRY_(alloc(&dwv, np));
     TRY_(alloc(&d_cross, np));
@@ -1332,13 +1317,7 @@ struct Engine : EngineBase {
     // segment fewer), else of the last one; a longer run asks for more
     // (keep_room)
     kseg = (2.0 * K * slot_bytes() <= 8.0 * (1 << 30)) ? 2 : 1;
-    seg_s.resize((size_t)kseg * K);
-    seg_f.resize((size_t)kseg * K);
-    for (int k = 0; k < kseg * K; ++k) {
-      TRY_(alloc_state(seg_s[k]));
-      TRY_(alloc(&seg_f[k], 6 * pl));
-    }
-    return ZC_OK;
+    return add_slots(kseg * K) ? ZC_OK : afail(ZC_ENOMEM, "adjoint engine: device allocation failed");
   }
 
   ~Engine() override {
@@ -1537,23 +1516,17 @@ struct Engine : EngineBase {
 
   double slot_bytes() const { return (double)state_span() + 6.0 * sizeof(R) * (double)pl; }
 
-  // Room for the pre-step states of nsteps steps, as far as 8 GiB go; without
-  // the memory the reverse sweep recomputes more.  (200 steps of 10^6 particles
-  // take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep of 33.)
-  zc_status keep_room(int nsteps) {
-    const int want = (nsteps - 1) / K + 1;
-    const int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
-    if (fit <= kseg) return ZC_OK;
-    const int more = (fit - kseg) * K;
+  // n more slots for pre-step states, one allocation; false without the memory
+  bool add_slots(int n) {
     const size_t a = (state_span() + 255) / 256 * 256, b = (6 * sizeof(R) * pl + 255) / 256 * 256;
     char *m = nullptr;
-    if (cudaMalloc((void **)&m, (a + b) * more) != cudaSuccess) {
+    if (cudaMalloc((void **)&m, (a + b) * n) != cudaSuccess) {
       cudaGetLastError();
-      return ZC_OK;
+      return false;
     }
     owned.push_back(m);
     const size_t off = (3 * sizeof(int) * (size_t)np + 15) / 16 * 16;
-    for (int k = 0; k < more; ++k, m += a + b) {
+    for (int k = 0; k < n; ++k, m += a + b) {
       DevState<R> s;
       s.ix = reinterpret_cast<int *>(m);
       s.iy = s.ix + np;
@@ -1562,7 +1535,17 @@ struct Engine : EngineBase {
       seg_s.push_back(s);
       seg_f.push_back(reinterpret_cast<R *>(m + a));
     }
-    kseg = fit;
+    return true;
+  }
+
+  // Room for the pre-step states of nsteps steps, as far as 8 GiB go; without
+  // the memory the reverse sweep recomputes more.  (200 steps of 10^6 particles
+  // take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep of 33.)
+  zc_status keep_room(int nsteps) {
+    const int want = (nsteps - 1) / K + 1;
+    const int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
+    if (fit <= kseg) return ZC_OK;
+    if (add_slots((fit - kseg) * K)) kseg = fit;
     return ZC_OK;
   }
 
