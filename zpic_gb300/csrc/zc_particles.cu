@@ -20,6 +20,22 @@
 
 namespace zc {
 
+// Raises a kernel's dynamic shared-memory limit, once a device.  The limit
+// belongs to the kernel, not to a simulation: it is set to the largest size
+// that any launch asks for, so that no thread lowers it below what another
+// thread is about to launch with.
+template <class K>
+static cudaError_t opt_in_smem(K *kernel, int bytes, std::atomic<unsigned long long> &opted) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (opted.load() & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) opted.fetch_or(bit);
+  return e;
+}
+
 // ---------------------------------------------------------------------------
 // K2: migrate the outboxes into the destination tiles, one CTA per tile
 // ---------------------------------------------------------------------------
@@ -814,7 +830,8 @@ cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *n
     W.w1 = (int)w1;
     W.w2 = (int)w2;
     const int bytes = (int)(w1 * w2 * 4);
-    const cudaError_t e = cudaFuncSetAttribute(k_pha_window, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    static std::atomic<unsigned long long> opted{0};
+    const cudaError_t e = opt_in_smem(k_pha_window, (int)kMaxWindow, opted);
     if (e != cudaSuccess) return e;
     const int resident = 152 * (int)std::max<long long>(1, std::min<long long>(4, kMaxWindow / (bytes + 1024)));
     k_pha_window<<<whole ? std::min(ntiles, resident) : ntiles, 512, bytes, st>>>(buf, off, np, ntiles, pha, P, W, L);
@@ -905,18 +922,10 @@ cudaError_t launch_cellsort(const Particles &src, const Particles &dst, const in
     k_cellsort_direct<ZC_SORT_NT><<<ntiles, ZC_SORT_NT, 0, st>>>(src, dst, off, np, L);
     return cudaGetLastError();
   }
-  // the shared-memory opt-in, once per device
   static std::atomic<unsigned long long> opted{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const cudaError_t e =
+      opt_in_smem(k_cellsort<ZC_SORT_NT>, 1024 * (int)sizeof(int) + kSortStageMax * kSortStageBytes, opted);
   if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(opted.load() & bit)) {
-    e = cudaFuncSetAttribute(k_cellsort<ZC_SORT_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             1024 * (int)sizeof(int) + kSortStageMax * kSortStageBytes);
-    if (e != cudaSuccess) return e;
-    opted.fetch_or(bit);
-  }
   const int S = std::min(max_n, kSortStageMax);
   const size_t smem = 1024 * sizeof(int) + (size_t)S * kSortStageBytes;
   k_cellsort<ZC_SORT_NT><<<ntiles, ZC_SORT_NT, smem, st>>>(src, dst, off, np, L, S, err);
