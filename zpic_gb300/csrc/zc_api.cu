@@ -667,14 +667,13 @@ int spill_blocks(const zc_sim *s) {
 }
 
 // the species' kinetic sum after a push of `parts` parts a tile (0: a launch
-// of its own)
+// of its own); deterministic: a value a tile, whatever its parts
 KinSum kin_sum(const zc_sim *s, const SpeciesState &p, int parts) {
-  const int tiles = s->ntiles * std::max(parts, 1);
   KinSum K;
   K.part = p.d_ekin_tile;
   K.fix = s->deterministic ? p.d_ekin_fix : nullptr;
   K.out = p.d_ekin;
-  K.n = tiles + (s->deterministic ? 0 : (parts ? kSpillParts : spill_blocks(s)));
+  K.n = s->deterministic ? s->ntiles : s->ntiles * std::max(parts, 1) + (parts ? kSpillParts : spill_blocks(s));
   K.q_mq = p.q * p.m_q;
   return K;
 }

@@ -218,8 +218,8 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// thread-block cluster: barrier in two halves, and an addition to an int of
-// rank 0's shared memory (the variable is at the same place in every CTA)
+// thread-block cluster: barrier in two halves, and additions to a variable in
+// rank 0's shared memory (it is at the same place in every CTA)
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
@@ -230,6 +230,11 @@ __device__ __forceinline__ int rank0_add(int *v, int n) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(v)));
   asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(n) : "memory");
   return old;
+}
+__device__ __forceinline__ void rank0_add(unsigned long long *v, unsigned long long n) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(v)));
+  asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(a), "l"(n) : "memory");
 }
 
 // contiguous bulk copy global -> shared, completing on an mbarrier (both

@@ -82,7 +82,7 @@ struct PushSpecies {
   TileSet T;
   Outbox Oin, O;                          // pending incoming (previous step), leavers (this step)
   Spill Sin, S;                           // spilled particles: to push, and those of this step
-  double *ekin;                           // kinetic energy of every tile part
+  double *ekin;                           // kinetic energy of every tile part (deterministic: every tile)
   double *ekin_spill;                     // and of every block of the spill push
   unsigned long long *ekin_fix;           // deterministic mode: the spill push's fixed-point words
   PushConst C;

@@ -994,8 +994,27 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
     else add_current(dep, acc_cell & (TX - 1), (acc_cell >> 16) & (TY - 1), acc);
   }
 
+  if constexpr (DET) {
+    // kinetic energy: integer sums, exact in any order, of the whole tile
+    // (its parts' too, so that the one rounding does not depend on which
+    // part held which particle)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      khi += __shfl_down_sync(0xffffffffu, khi, off);
+      klo += __shfl_down_sync(0xffffffffu, klo, off);
+    }
+    if (lane == 0) {
+      if constexpr (SPLIT) {
+        if (khi) rank0_add(&s_ekin[0], (unsigned long long)khi);
+        if (klo) rank0_add(&s_ekin[1], (unsigned long long)klo);
+      } else {
+        if (khi) atomicAdd(&s_ekin[0], (unsigned long long)khi);
+        if (klo) atomicAdd(&s_ekin[1], (unsigned long long)klo);
+      }
+    }
+  }
   if constexpr (SPLIT) {
-    cluster_arrive();  // every part's leavers and arrivals are counted
+    cluster_arrive();  // every part's leavers, arrivals and energies are counted
     cluster_wait();
   } else {
     __syncthreads();
@@ -1003,20 +1022,9 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   if (threadIdx.x == 0 && (!SPLIT || rank == 0)) {
     T.np[t] = n_own + min(s_app, T.cap[t] - n_own);
     O.cnt[t] = min(s_leave, O.cap);
+    if constexpr (DET) A.ekin[t] = efix_join((long long)s_ekin[0], (long long)s_ekin[1]);
   }
   if constexpr (DET) {
-    // integer sums: exact in any order
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      khi += __shfl_down_sync(0xffffffffu, khi, off);
-      klo += __shfl_down_sync(0xffffffffu, klo, off);
-    }
-    if (lane == 0) {
-      if (khi) atomicAdd(&s_ekin[0], (unsigned long long)khi);
-      if (klo) atomicAdd(&s_ekin[1], (unsigned long long)klo);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) A.ekin[t * parts + rank] = efix_join((long long)s_ekin[0], (long long)s_ekin[1]);
     // the integer J tile goes to the global fixed-point planes (units of
     // 2^-40) with 64-bit integer atomics (cells outside the buffer hold no
     // deposits)
