@@ -2098,6 +2098,7 @@ zc_status zc_spec_advance(zc_sim *s, int k) {
   DeviceGuard g(s->device);
   CK(cudaEventRecord(s->ev0, s->st));
   TRY(restore_current(s));
+  s->j0_zero = false;  // the deposits below: the next step clears them
   TRY(spec_advance_impl(s, k));
   TRY(fixed_current(s));
   TRY(kin_energies(s, k, 1, 0));
