@@ -748,7 +748,8 @@ PushLaunch push_launch(const zc_sim *s) {
   return a;
 }
 
-zc_status species_pushed(zc_sim *s, int k, int shift);
+void species_pushed(SpeciesState &p, int shift);
+zc_status inject_column(zc_sim *s, int k);
 
 // deterministic mode: the float J that the rest of the step reads, from the
 // fixed-point sums
@@ -787,7 +788,8 @@ zc_status spec_advance_impl(zc_sim *s, int k) {
     Phase ph(s, ZC_PHASE_SPILL, 1);
     CK(launch_push_spill(a, spill_blocks(s), s->st));
   }
-  return species_pushed(s, k, shift);
+  species_pushed(s->sp[k], shift);
+  return shift ? inject_column(s, k) : ZC_OK;
 }
 
 // every species in one launch, each tile in `parts` parts
@@ -804,24 +806,34 @@ zc_status push_all(zc_sim *s, int parts) {
     Phase ph(s, ZC_PHASE_PUSH, all.nsp);  // (the profile counts species' pushes)
     CK(launch_push_tiles(a, s->st));
   }
-  for (int k = 0; k < all.nsp; ++k) TRY(species_pushed(s, k, shift[k]));
-  return ZC_OK;
+  // All of them are pushed: the host says so before a provider can fail, and
+  // one species' failure does not cost another its column.
+  for (int k = 0; k < all.nsp; ++k) species_pushed(s->sp[k], shift[k]);
+  zc_status r = ZC_OK;
+  for (int k = 0; k < all.nsp; ++k) {
+    const zc_status one = shift[k] ? inject_column(s, k) : ZC_OK;
+    if (r == ZC_OK) r = one;
+  }
+  return r;
 }
 
-// the host side of a push, and the column a window move uncovers
-zc_status species_pushed(zc_sim *s, int k, int shift) {
-  SpeciesState &p = s->sp[k];
-  cudaStream_t st = s->st;
+// the host side of a push
+void species_pushed(SpeciesState &p, int shift) {
   p.ob_in = 1 - p.ob_in;
   p.pending = true;
   p.cur = 1 - p.cur;
   p.spill_cur = 1 - p.spill_cur;
   p.iter += 1;
-  if (shift && p.dinj) {
-    p.n_move += 1;
+  p.n_move += shift;
+}
+
+// the column that a window move uncovers
+zc_status inject_column(zc_sim *s, int k) {
+  SpeciesState &p = s->sp[k];
+  cudaStream_t st = s->st;
+  if (p.dinj) {
     TRY(inject_column_device(s, p));
-  } else if (shift) {
-    p.n_move += 1;
+  } else {
     if (!s->inj) return fail(ZC_ESTATE, "moving window needs an injection provider (zc_set_injector)");
     const zc_part *parts = nullptr;
     int n = 0;
