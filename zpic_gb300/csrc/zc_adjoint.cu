@@ -1476,8 +1476,9 @@ struct Engine : EngineBase {
     return ZC_OK;
   }
 
-  zc_status save_checkpoint(const DevState<R> &from, const R *fE, const R *fB) {
-    if (nck == (int)ck_s.size()) {
+  // room for n checkpoints
+  zc_status checkpoint_room(int n) {
+    while ((int)ck_f.size() < n) {
       DevState<R> s;
       R *f = nullptr;
       TRY_(alloc_state(s));
@@ -1485,6 +1486,10 @@ struct Engine : EngineBase {
       ck_s.push_back(s);
       ck_f.push_back(f);
     }
+    return ZC_OK;
+  }
+
+  zc_status save_checkpoint(const DevState<R> &from, const R *fE, const R *fB) {
     TRY_(copy_state(ck_s[nck], from));
     TRY_(copy_fields(ck_f[nck], ck_f[nck] + 3 * pl, fE, fB));
     ++nck;
@@ -1538,21 +1543,29 @@ struct Engine : EngineBase {
     return true;
   }
 
-  // Room for the pre-step states of nsteps steps, as far as 8 GiB go; without
-  // the memory the reverse sweep recomputes more.  (200 steps of 10^6 particles
-  // take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep of 33.)
-  zc_status keep_room(int nsteps) {
+  // Room for the pre-step states of nsteps steps, as far as 8 GiB and half of
+  // the memory that is free go (what a run cannot do without is allocated
+  // before); without it the reverse sweep recomputes more.  (200 steps of 10^6
+  // particles take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep
+  // of 33.)
+  void keep_room(int nsteps) {
     const int want = (nsteps - 1) / K + 1;
-    const int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
-    if (fit <= kseg) return ZC_OK;
-    if (add_slots((fit - kseg) * K)) kseg = fit;
-    return ZC_OK;
+    int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
+    if (fit <= kseg) return;
+    size_t free_mem = 0, total = 0;
+    if (cudaMemGetInfo(&free_mem, &total) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    fit = (int)std::min((double)fit, kseg + 0.5 * (double)free_mem / (K * slot_bytes()));
+    if (fit > kseg && add_slots((fit - kseg) * K)) kseg = fit;
   }
 
   zc_status forward(int nsteps, double *obj, double *kin) override {
     if (!have_state) return afail(ZC_ESTATE, "adjoint engine: no initial state");
     if (nsteps <= 0) return afail(ZC_EINVAL, "adjoint engine: nsteps must be > 0");
-    TRY_(keep_room(nsteps));
+    TRY_(checkpoint_room((nsteps - 1) / K + 1));
+    keep_room(nsteps);
     plan_shifts(nsteps);
     ACK(cudaEventRecord(e0, st));
     nck = 0;
