@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -1248,6 +1249,15 @@ struct Guard1 {
   ~Guard1() { cudaSetDevice(old); }
 };
 
+// The calls that are waiting for steps on a device right now, over all threads
+// (see run_steps).
+std::atomic<int> g_waiting[64];
+struct Waiting {
+  std::atomic<int> &n;
+  explicit Waiting(int device) : n(g_waiting[device & 63]) { n.fetch_add(1); }
+  ~Waiting() { n.fetch_sub(1); }
+};
+
 constexpr int kPushThreads = 256;
 constexpr int kMaxCtas = 152 * 4;  // the push CTAs resident together (4 per SM)
 
@@ -1540,13 +1550,17 @@ zc_status run_block(zc1_sim *s) {
 // no species or too many, or the grids and every CTA's share of the particles
 // do not fit its shared memory (then the two kernels a step, in graphs).
 //
-// The CTAs: one a multiprocessor when the caller waits for the steps.  One who
-// does not may have other simulations' steps beside these, and launches that
-// fill the GPU would run one after another: a quarter of the multiprocessors
-// then (64 runs of the 1000-cell deck side by side: 21.7 G particles/s against
-// 8.3 with the full grid and 12.9 with the two kernels; one run alone takes
-// 15.2 us a step against 11.0 and 22).  A single step that nobody waits for is
-// left to the two kernels: 25.0 us against 26.9.
+// The CTAs: one a multiprocessor when one caller waits for the steps.  One who
+// does not wait may have other simulations' steps beside these, and launches
+// that fill the GPU would run one after another: a quarter of the
+// multiprocessors then (64 runs of the 1000-cell deck side by side: 21.7 G
+// particles/s against 8.3 with the full grid and 12.9 with the two kernels; one
+// run alone takes 15.2 us a step against 11.0 and 22).  Callers that wait in
+// several threads share the GPU likewise, half each or a quarter (that deck
+// with 64000 particles, us a step of one run with 1, 2, 4, 8, 32 threads: 11.9
+// 7.0 4.3 3.7 3.7, with the full grid 11.9 10.4 9.6 9.2 8.8, with the two
+// kernels 22 12.6 7.6 5.9 5.8).  A single step that nobody waits for is left to
+// the two kernels: 25.0 us against 26.9.
 zc_status run_steps(zc1_sim *s, int most, bool waits, int *done) {
   *done = 0;
   if (!s->run_smem || s->profile || s->sp.empty() || (int)s->sp.size() > kRunSpecies) return ZC_OK;
@@ -1558,7 +1572,8 @@ zc_status run_steps(zc1_sim *s, int most, bool waits, int *done) {
   for (auto &p : s->sp) np = std::max(np, p.np_bound);
   // one CTA a multiprocessor, at least a warp of particles each (a
   // simulation's own cap counts CTAs of kPushThreads)
-  const int room = waits ? s->sms : std::max(1, s->sms / 4);
+  const int sharers = waits ? std::min(4, std::max(1, g_waiting[s->device & 63].load())) : 4;
+  const int room = std::max(1, s->sms / sharers);
   const int most_ctas =
       s->push_ctas > 0 ? std::max(1, std::min(s->sms, s->push_ctas * kPushThreads / kRunThreads)) : room;
   const int grid = (int)std::max<long long>(1, std::min<long long>(most_ctas, np / 256));
@@ -1888,6 +1903,8 @@ zc_status zc1_get_current(zc1_sim *s, float *J) {
 zc_status zc1_step_async(zc1_sim *s, int nsteps) { return enqueue_steps(s, nsteps, false); }
 
 zc_status zc1_step(zc1_sim *s, int nsteps) {
+  if (!s) return fail1(ZC_EINVAL, "null simulation handle");
+  Waiting here(s->device);
   TRY1(enqueue_steps(s, nsteps, true));
   return zc1_synchronize(s);
 }
