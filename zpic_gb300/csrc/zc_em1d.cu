@@ -1165,7 +1165,7 @@ struct Species1 {
   long long np_bound = 0;    // upper bound of the device count
   Parts buf[2] = {};
   SpecState1 *d_st = nullptr;
-  float *d_lat = nullptr;    // in-cell positions of an injected cell's particles
+  float *d_lat = nullptr;    // in-cell positions of an injected cell's particles (null: none injected)
 };
 
 }  // namespace zc1
@@ -1803,10 +1803,12 @@ zc_status zc1_add_species(zc1_sim *s, const zc1_species_desc *d, const zc1_part 
     CK1(cudaMemcpy(p.buf[0].uy, uy.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
     CK1(cudaMemcpy(p.buf[0].uz, uz.data(), sizeof(float) * np, cudaMemcpyHostToDevice));
   }
-  std::vector<float> lat(p.inj.ppc);
-  for (int i = 0; i < p.inj.ppc; ++i) lat[i] = (float)((i + 0.5) / p.inj.ppc);
-  CK1(cudaMalloc(&p.d_lat, sizeof(float) * lat.size()));
-  CK1(cudaMemcpy(p.d_lat, lat.data(), sizeof(float) * lat.size(), cudaMemcpyHostToDevice));
+  if (s->mw && p.inj.type != 1) {  // only a window that injects reads them
+    std::vector<float> lat(p.inj.ppc);
+    for (int i = 0; i < p.inj.ppc; ++i) lat[i] = (float)((i + 0.5) / p.inj.ppc);
+    CK1(cudaMalloc(&p.d_lat, sizeof(float) * lat.size()));
+    CK1(cudaMemcpy(p.d_lat, lat.data(), sizeof(float) * lat.size(), cudaMemcpyHostToDevice));
+  }
   SpecState1 h{};
   h.np[0] = np;
   CK1(cudaMemcpy(p.d_st, &h, sizeof(SpecState1), cudaMemcpyHostToDevice));
