@@ -639,13 +639,18 @@ int column_lattice(const zc_sim *s, const SpeciesState &p, int n_move, ColumnInj
 // The parts every tile is split into when all species are pushed in one
 // launch (push_all), or 0 for one launch a species.  A grid of few tiles does
 // not fill the GPU with one CTA a tile, and its step is bound by its chain of
-// launches.  So species go together when their tiles fit the GPU in one round
-// (kTogetherCtas: 4 CTAs of that kernel a multiprocessor), and tiles are split
-// while the parts still do and leave every warp a unit of 32 slots.  Measured
+// launches.  So species go together up to kTogetherCtas tiles, and tiles are
+// split while the parts run in one round (push_all_ctas) and leave every warp a
+// unit of 32 slots (in the deterministic builds, with twice the warps, every
+// other one: 33.0 against 34.2 us a step at 64^2 cells with 2 a cell).  Measured
 // (128^2 cells, two species of 16 a cell, 16x16 tiles): 137 us a step with a
 // push of 64 CTAs a species, a spill launch and a kinetic sum each, 36 with
 // one push launch of 512 CTAs; later in the run, with filaments (tiles of
-// several times the mean), 200 and 65.  Twice the CTAs (two rounds): 43.
+// several times the mean), 200 and 65.  Twice the CTAs (two rounds): 43; 512 of
+// the deterministic build (456 places), one species: 52.2, with 256: 43.9.
+// kTogetherCtas is the places of the float builds.  Between a deterministic
+// build's places and it, together is the better of two (256^2 cells, two
+// species: 65.7 against 75.8) and 2% the worse for one (512^2: 194 against 191).
 // Runs of a batch share the GPU with the others: together, not split.
 constexpr int kTogetherCtas = 608;
 int push_parts(const zc_sim *s) {
@@ -655,8 +660,9 @@ int push_parts(const zc_sim *s) {
   if (s->batches > 0) return 1;
   int units = 0;
   for (const auto &p : s->sp) units = std::max(units, p.ppc[0] * p.ppc[1] * s->TX * s->TY / 32);
+  const int places = 152 * push_all_ctas(s->TX, s->TY, s->deterministic);
   int parts = 1;
-  while (parts < kMaxParts && 2 * parts * ctas <= kTogetherCtas && 2 * parts * kPushWarps <= units) parts *= 2;
+  while (parts < kMaxParts && 2 * parts * ctas <= places && 2 * parts * kPushWarps <= units) parts *= 2;
   return parts;
 }
 

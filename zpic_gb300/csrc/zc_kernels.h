@@ -92,6 +92,13 @@ struct PushSpecies {
 // CTAs, then kSpillParts blocks for the spilled particles of each species
 constexpr int kMaxTogether = 8, kMaxParts = 8, kSpillParts = 8;
 constexpr int kPushWarps = 4;             // warps of a push CTA (float builds)
+// CTAs of that launch that a multiprocessor holds: 4 of the float builds (up to
+// 128 registers, 128 threads); of the deterministic ones 3 of 256 threads (80
+// registers), or 2 with the 91 KB of a 32x32 tile's current and fields, and 6
+// of 128 threads (tiles of less than 256 cells)
+__host__ __device__ constexpr int push_all_ctas(int TX, int TY, bool det) {
+  return !det ? 4 : (TX * TY >= 1024 ? 2 : (TX * TY >= 256 ? 3 : 6));
+}
 struct PushAll {
   int nsp, ntiles, parts;
   PushSpecies sp[kMaxTogether];

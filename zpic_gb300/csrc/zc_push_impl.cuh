@@ -1138,6 +1138,8 @@ template <int TX, int TY, int NT, bool DET>
 __global__ void __launch_bounds__(NT, DET ? kDetThreads / NT : 4)
     k_push_all(const __grid_constant__ CUtensorMap tm_eb, const __grid_constant__ PushAll P, const float *EB, Grid G,
                int *err, FixedJ fj) {
+  // (the rule that splits tiles counts on these places)
+  static_assert(push_all_ctas(TX, TY, DET) <= (DET ? kDetThreads / NT : 4), "more places than the launch bounds give");
   const int b = blockIdx.x, ntile = P.nsp * P.ntiles * P.parts;
   if (b < ntile) {
     const int q = b / P.parts, k = q / P.ntiles;
