@@ -340,15 +340,16 @@ struct RunSums {
   // to the tile's three planes, as jsplit cuts an integer; the sums start again
   template <class DEP>
   __device__ __forceinline__ void flush(const DEP &dep, unsigned cell) {
-    const int i = DEP::column(cell), j = DEP::row(cell), L = dep.C->js_l;
+    const int i = DEP::column(cell), j = DEP::row(cell), L = dep.C->js_l, s = 22 - L;
     constexpr int c[8] = {0, 0, 1, 1, 2, 2, 2, 2}, di[8] = {0, 0, 0, 1, 0, 1, 0, 1}, dj[8] = {0, 1, 0, 0, 0, 0, 1, 1};
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const long long v = (long long)h[q] * (1 << 22) + l[q];
-      const int vl = (int)((unsigned)v << (32 - L)) >> (32 - L);
-      const long long w = (v - vl) >> L;
-      const int vm = (int)((unsigned)w << (32 - L)) >> (32 - L);
-      dep.addi(c[q], i + di[q], j + dj[q], (int)((w - vm) >> L), vm, vl);
+      // (h 2^22 + l = vh 2^2L + vm 2^L + vl: the low L bits of l, then those of
+      // r + h 2^s, which makes r - vm a multiple of 2^min(s, L); no 64-bit shifts)
+      const int vl = (int)((unsigned)l[q] << (32 - L)) >> (32 - L), r = (l[q] - vl) >> L;
+      const int vm = (int)((((unsigned)h[q] << s) + (unsigned)r) << (32 - L)) >> (32 - L);
+      const int vh = L >= s ? (h[q] + ((r - vm) >> s)) >> (L - s) : (h[q] << (s - L)) + ((r - vm) >> L);
+      dep.addi(c[q], i + di[q], j + dj[q], vh, vm, vl);
       h[q] = l[q] = 0;
     }
   }
