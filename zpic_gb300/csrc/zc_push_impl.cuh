@@ -596,9 +596,17 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   // per-warp queue of the particles that need more than the common case (see
   // `finish`): x, y before and ux, uy, uz after the push, the cell word and
   // the own slot; finished 32 at a time, so at most 31 wait when the next
-  // unit's 32 lanes queue theirs
+  // unit's 32 lanes queue theirs.  The exact builds keep mx, my and q v_z too
+  // (a square root and a division that the fast builds make again in a few
+  // instructions), unless the tile's own memory leaves no room (32x32: a CTA
+  // less a multiprocessor).
+#ifdef ZC_FAST
+  constexpr bool KEEP = false;
+#else
+  constexpr bool KEEP = TX * TY <= 512;
+#endif
   constexpr int QCAP = 63;
-  __shared__ float qf[NW][5][QCAP];
+  __shared__ float qf[NW][KEEP ? 8 : 5][QCAP];
   __shared__ unsigned qc[NW][QCAP];
   __shared__ int qs[NW][QCAP];
   __shared__ int nb[8], s_nnb;        // distinct neighbour tiles
@@ -754,7 +762,13 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
     int di = 0, dj = 0, code = 0, dest = 0;  // code: 0 gone, 1 stays, 2 leaves
     if (act) {
       float mx, my, qvz;
-      displacement(ux, uy, uz, mx, my, qvz, Cl);  // as the push had it
+      if constexpr (KEEP) {
+        mx = qf[warp][5][e];
+        my = qf[warp][6][e];
+        qvz = qf[warp][7][e];
+      } else {
+        displacement(ux, uy, uz, mx, my, qvz, Cl);  // as the push had it
+      }
       errbits |= !(fabsf(mx) < 1.0f && fabsf(my) < 1.0f) ? ERR_ESCAPE : 0;
       float x1 = x + mx, y1 = y + my;
       di = (x1 >= 1.0f) - (x1 < 0.0f);
@@ -858,6 +872,11 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
           qf[warp][2][e] = ux;
           qf[warp][3][e] = uy;
           qf[warp][4][e] = uz;
+          if constexpr (KEEP) {
+            qf[warp][5][e] = mx;
+            qf[warp][6][e] = my;
+            qf[warp][7][e] = qvz;
+          }
           qc[warp][e] = cw;
           qs[warp][e] = oslot;
         }
