@@ -2353,7 +2353,7 @@ zc_status zc_species_phasespace(zc_sim *s, int k, int quant1, int quant2, const 
   TRY(density_buffer(s, n, &d));
   CK(cudaMemcpyAsync(d, buf, n * sizeof(float), cudaMemcpyHostToDevice, s->st));
   CK(launch_phasespace(p.buf[p.cur], p.d_off, p.d_np, s->ntiles, p.spill[p.spill_cur], p.d_spill_cnt + p.spill_cur,
-                       p.spill_cap, d, P, layout(s), s->st));
+                       p.spill_cap, d, P, layout(s), p.ppc[0] * p.ppc[1] * s->TX * s->TY, s->st));
   CK(cudaMemcpyAsync(buf, d, n * sizeof(float), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
   return ZC_OK;

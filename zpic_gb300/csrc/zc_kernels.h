@@ -226,7 +226,7 @@ struct PhaConst {
 };
 cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
                               const int *spill_cnt, int spill_cap, float *pha, const PhaConst &P,
-                              const LayoutConst &L, cudaStream_t st);
+                              const LayoutConst &L, int per_tile, cudaStream_t st);  // per_tile: particles of a full tile
 cudaError_t launch_charge(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
                           const int *spill_cnt, int spill_cap, float *rho, int nx, int ny, float q, int mw,
                           cudaStream_t st);

@@ -811,7 +811,7 @@ __global__ void k_pha_list(Particles list, const int *n_ptr, int n_cap, float *p
 
 cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *np, int ntiles, const Particles &spill,
                               const int *spill_cnt, int spill_cap, float *pha, const PhaConst &P,
-                              const LayoutConst &L, cudaStream_t st) {
+                              const LayoutConst &L, int per_tile, cudaStream_t st) {
   // the window: the columns a tile spans and two each side on a position
   // axis, all of a momentum axis
   auto width = [](int q, int n, double span) {
@@ -820,13 +820,24 @@ cudaError_t launch_phasespace(const Particles &buf, const int *off, const int *n
   PhaWindow W;
   W.pos1 = P.q1 <= 2;
   W.pos2 = P.q2 <= 2;
-  const long long w1 = width(P.q1, P.n1, std::fabs((P.q1 == 1 ? L.TX * P.dx : L.TY * P.dy) * P.rdx1));
-  const long long w2 = width(P.q2, P.n2, std::fabs((P.q2 == 1 ? L.TX * P.dx : L.TY * P.dy) * P.rdx2));
+  const double s1 = std::fabs((P.q1 == 1 ? L.TX * P.dx : L.TY * P.dy) * P.rdx1);
+  const double s2 = std::fabs((P.q2 == 1 ? L.TX * P.dx : L.TY * P.dy) * P.rdx2);
+  const long long w1 = width(P.q1, P.n1, s1), w2 = width(P.q2, P.n2, s2);
   constexpr long long kMaxWindow = 200 * 1024;  // bytes: a multiprocessor's shared memory
-  // (a window that follows the tile is cleared and added for every tile: not
-  // more values than a tile has particles' corners to add)
+  // (a window that follows the tile is cleared and added for every tile: 8192
+  // values at most)
   const bool whole = !W.pos1 && !W.pos2;
-  if (w1 * w2 * 4 <= (whole ? kMaxWindow : 32 * 1024)) {
+  // A grid of two positions has no values that all particles crowd on, but the
+  // sorted particles of a warp meet in a few of the window's: through the window
+  // where a tile spans one or two values (us a call, grid values themselves /
+  // window, 512^2 cells with 16 a cell: 32^2 values 1022 / 471, 64^2 384 / 385,
+  // 90^2 229 / 348, 256^2 142 / 154), hardly more than one along a row of cells
+  // (16 x 1024: 327 / 160), a dozen or more along a column (512^2: 169 / 154;
+  // 2000 x 256 cells, 512^2: 275 / 211), or where it holds many particles (64 a
+  // cell: 497 / 299 at 64^2, 166 / 128 at 256^2).
+  const double sx = P.q1 == 1 ? s1 : s2, sy = P.q1 == 1 ? s2 : s1;
+  const bool meet = W.pos1 && W.pos2 && !(sx <= 1.5 || sx * sy <= 2 || sy >= 12 || per_tile >= 8192);
+  if (!meet && w1 * w2 * 4 <= (whole ? kMaxWindow : 32 * 1024)) {
     W.w1 = (int)w1;
     W.w2 = (int)w2;
     const int bytes = (int)(w1 * w2 * 4);
