@@ -627,8 +627,13 @@ __global__ void k_adj_push(State<R> s, State<R> o, const R *w, const int *birth,
                            Planes<R> J, double *ekin, Params<R> P) {
   const size_t pl = (size_t)E.pitch() * P.ny;
   double ek = 0;
+  // a block's particles: a share of its own with the vector reductions (40 steps
+  // of 10^6 particles, float32: 2.35 ms against 2.44), else every gridDim-th
+  // round (float64: 30.5 ms against 32.9; float32 with a window 5.75, 6.06)
   const Share mine(P.np);
-  for (int p = mine.first + threadIdx.x; p < mine.end; p += blockDim.x) {
+  const int first = V4 ? mine.first : (int)(blockIdx.x * blockDim.x), end = V4 ? mine.end : P.np;
+  const int stride = V4 ? (int)blockDim.x : (int)(gridDim.x * blockDim.x);
+  for (int p = first + (int)threadIdx.x; p < end; p += stride) {
     const int ix = s.ix[p], iy = s.iy[p];
     const R x = s.x[p], y = s.y[p];
     const R u[3] = {s.ux[p], s.uy[p], s.uz[p]};
