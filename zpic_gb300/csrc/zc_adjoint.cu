@@ -885,6 +885,34 @@ __global__ void __launch_bounds__(256) k_adj_fields(const R *E, const R *B, cons
   }
 }
 
+// The same in float64 on a large grid, a kernel each (yee_b: Bo may be B): the
+// fused kernel takes four times the arithmetic, which float64, slow here, does
+// not hide behind the launches.  Both give the same bits.
+template <class R>
+__global__ void k_adj_yee_b(const R *E, const R *B, R *Bo, int nx, int ny, R hx, R hy) {
+  const size_t pl = (size_t)nx * ny;
+  const R *Ex = E, *Ey = E + pl, *Ez = E + 2 * pl;
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(k % nx), j = (int)(k / nx);
+    const size_t right = (size_t)j * nx + wrap(i + 1, nx), up = (size_t)wrap(j + 1, ny) * nx + i;
+    Bo[k] = B[k] + -hy * (Ez[up] - Ez[k]);
+    Bo[pl + k] = B[pl + k] + hx * (Ez[right] - Ez[k]);
+    Bo[2 * pl + k] = B[2 * pl + k] + (-hx * (Ey[right] - Ey[k]) + hy * (Ex[up] - Ex[k]));
+  }
+}
+template <class R>
+__global__ void k_adj_yee_e(const R *E, const R *B, const R *J, R *Eo, int nx, int ny, R cx, R cy, R dt) {
+  const size_t pl = (size_t)nx * ny;
+  const R *Bx = B, *By = B + pl, *Bz = B + 2 * pl;
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < pl; k += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(k % nx), j = (int)(k / nx);
+    const size_t left = (size_t)j * nx + wrap(i - 1, nx), down = (size_t)wrap(j - 1, ny) * nx + i;
+    Eo[k] = E[k] + (cy * (Bz[k] - Bz[down]) - dt * J[k]);
+    Eo[pl + k] = E[pl + k] + (-cx * (Bz[k] - Bz[left]) - dt * J[pl + k]);
+    Eo[2 * pl + k] = E[2 * pl + k] + (cx * (By[k] - By[left]) - cy * (Bx[k] - Bx[down]) - dt * J[2 * pl + k]);
+  }
+}
+
 // Its transpose: (lE, lB) after the step to (ln, lbn) before it, lJ the
 // current's adjoint.  A4: the transposes of the gathers of the step after are
 // still apart, in S (scatter_pairs); `clear`, the next ones', is left zero.
@@ -1145,6 +1173,10 @@ __global__ void k_from_double(const double *src, R *dst, size_t n) {
     dst[k] = (R)src[k];
 }
 
+// cells from which float64 fields are advanced by a kernel each (40 steps with
+// few particles, ms, fused / apart: 192^2 cells 2.12 / 2.20, 256^2 2.53 / 2.36,
+// 512^2 4.43 / 3.00, 1024^2 12.6 / 5.79)
+constexpr size_t kApartCells = 65536;
 int grid_for(size_t n, int per = 256) { return (int)std::max<size_t>(1, std::min<size_t>((n + per - 1) / per, 152 * 8)); }
 
 zc_status afail(zc_status s, const char *msg) {
@@ -1474,6 +1506,10 @@ struct Engine : EngineBase {
         k_adj_fields<R, true><<<grid_for(pl), 256, 0, st>>>(Ei, Bi, Jn[jn], Eo, Bo, (float4 *)Jn[1 - jn], nx, ny, hx,
                                                             hy, cx, cy, (R)dt);
       jn = 1 - jn;
+    } else if (sizeof(R) == 8 && pl >= kApartCells) {
+      k_adj_yee_b<R><<<grid_for(pl), 256, 0, st>>>(Ei, Bi, Bo, nx, ny, hx, hy);
+      k_adj_yee_e<R><<<grid_for(pl), 256, 0, st>>>(Ei, Bo, J, Eo, nx, ny, cx, cy, (R)dt);
+      k_adj_yee_b<R><<<grid_for(pl), 256, 0, st>>>(Eo, Bo, Bo, nx, ny, hx, hy);
     } else {
       k_adj_fields<R, false><<<grid_for(pl), 256, 0, st>>>(Ei, Bi, J, Eo, Bo, nullptr, nx, ny, hx, hy, cx, cy, (R)dt);
     }
