@@ -1741,7 +1741,6 @@ struct Engine : EngineBase {
         const int k = s0 + n - n0;
         TRY_(field_reverse(n));
         const Params<R> P = params(n, shifts[n]);
-        ACK(cudaMemsetAsync(d_ncross, 0, sizeof(int), st));
         if constexpr (sizeof(R) == 4) {
           if (v4) TRY_((push_reverse<true>(seg_s[k], seg_f[k], Sn[sn], nullptr, P)));
         }
