@@ -626,7 +626,6 @@ zc_status set_current_scale(zc_sim *s, const SpeciesState &p, PushConst &C) {
   C.js_twol = (float)std::ldexp(1.0, L);
   C.js_inv2l = (float)std::ldexp(1.0, -2 * L);
   C.js_two2l = (float)std::ldexp(1.0, 2 * L);
-  C.js_lo = (float)std::ldexp(1.0, -kx);
   C.js_l = L;
   C.js_run = vmax < std::ldexp(1.0, 43 - kx) ? 1 : 0;
   C.js_det = s->deterministic ? 1LL : 0LL;  // 2^(40 - k), k = 40

@@ -15,9 +15,9 @@ struct PushConst {
   int mw;                                 // absorbing boundaries along x
   // tile current as integers (see jsplit): a contribution v counts as
   // rint(v js) = h 2^2L + m 2^L + l; js_invl = 2^-L, js_twol = 2^L,
-  // js_inv2l = 2^-2L, js_two2l = 2^2L, js_lo = 1 / js; deterministic global
+  // js_inv2l = 2^-2L, js_two2l = 2^2L; deterministic global
   // sums in units of 2^-40 take each integer times js_det (2^40 / js)
-  float js, js_invl, js_twol, js_inv2l, js_two2l, js_lo;
+  float js, js_invl, js_twol, js_inv2l, js_two2l;
   int js_l;
   int js_run;                             // |v| js < 2^43: a lane's sums of two parts hold it (RunSums)
   long long js_det;
