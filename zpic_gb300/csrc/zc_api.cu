@@ -597,18 +597,21 @@ zc_status check_errors(zc_sim *s, bool relayout_spill) {
   return act_on_errors(s, s->h_pinned[0], relayout_spill);
 }
 
-// Scale of the push's integer current tile (jsplit).  Every contribution
-// is below vmax = 1.5 |q| in magnitude: a segment's Jx is qnx dx' with |dx'|
-// <= |mx| = (dt/dx) |ux| / gamma < dt/dx, so |Jx| < |q| (Jy alike), and its Jz
-// corner weights times qvz/2 stay below 1.25 |q| (the margin covers the
-// fast build's approximate square roots); a warp adds at most 32 of them at
-// once.  A tile takes at most n = 3 (largest tile + 8 outboxes)
-// contributions per node (three segments per particle).  With 2^cl >= n, L =
-// min(22, 31 - cl) keeps the sums of the |m|, |l| <= 2^(L-1) below 2^30; js
-// = 2^k with k = 40 (the unit of the deterministic sums) unless n vmax js
-// 2^-2L <= 2^30 (the sum of the |h| below 2^31) or 32 vmax js 2^-2L < 2^22
-// (the shifter's range) need less.  Deterministic runs require k = 40, so
-// that their sums do not depend on the tile layout.
+// Scale of the push's integer current tile (jsplit, RunSums).  Every
+// contribution is below vmax = 1.5 |q| in magnitude: a segment's Jx is qnx dx'
+// with |dx'| <= |mx| = (dt/dx) |ux| / gamma < dt/dx, so |Jx| < |q| (Jy alike),
+// and its Jz corner weights times qvz/2 stay below 1.25 |q| (the margin covers
+// the fast build's approximate square roots).  A tile takes at most n = 3
+// (largest tile + 8 outboxes) contributions per node (three segments per
+// particle), one by one or summed by a lane before they are cut.  With 2^cl >=
+// n, L = min(22, 31 - cl) keeps the sums of the |m|, |l| <= 2^(L-1) below 2^30;
+// js = 2^k with k = 40 (the unit of the deterministic sums) unless n vmax js
+// 2^-2L <= 2^30 (the sum of the |h| below 2^31) or vmax js 2^-2L <= 2^16 need
+// less (jsplit's shifter takes 2^22; the margin stays, since the bound decides
+// which charges a deterministic run accepts).  Deterministic runs require k =
+// 40, so that their sums do not depend on the tile layout.  js_run: vmax js <
+// 2^43, so that the two parts of a lane's running sums are at most 2^21 a
+// contribution and 2^30 for 512 of them.
 zc_status set_current_scale(zc_sim *s, const SpeciesState &p, PushConst &C) {
   const double vmax = std::max(1.5 * std::fabs((double)p.q), 1e-30);
   const long long n = 3LL * ((long long)p.max_cap + 8LL * p.ob[0].cap) + 1;

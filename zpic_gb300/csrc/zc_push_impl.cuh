@@ -667,7 +667,8 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
     return c + lane;
   };
   // a lane without a particle carries the last unit's particle, a hole's
-  // zero momenta, or these zeros: finite values whose results `valid` masks;
+  // momenta (zero at first, then pushed along at its cell's centre), or these
+  // zeros: finite values whose results `valid` masks;
   // its position is set to the cell centre (a hole's is stale)
   float4 nu = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 nxy = make_float2(0.f, 0.f);
