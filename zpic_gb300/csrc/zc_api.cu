@@ -2298,7 +2298,8 @@ zc_status zc_energy_async(zc_sim *s, double emf[6], double *kin) {
   return queue_energy(s, emf, kin);
 }
 
-// room for a density of n values, kept for the next one
+// room for a density of n values, kept for the next one (up to 64 MB: see
+// density_done)
 static zc_status density_buffer(zc_sim *s, size_t n, float **d) {
   if (n > s->dens_n) {
     dfree(s->dens);  // (the calls that use it wait for the device)
@@ -2308,6 +2309,11 @@ static zc_status density_buffer(zc_sim *s, size_t n, float **d) {
   }
   *d = s->dens;
   return ZC_OK;
+}
+static void density_done(zc_sim *s) {
+  if (s->dens_n * sizeof(float) <= (size_t)64 << 20) return;
+  dfree(s->dens);
+  s->dens_n = 0;
 }
 
 zc_status zc_species_charge(zc_sim *s, int k, float *charge) {
@@ -2324,6 +2330,7 @@ zc_status zc_species_charge(zc_sim *s, int k, float *charge) {
                    p.spill_cap, d, s->nx, s->ny, p.q, s->mw, s->st));
   CK(cudaMemcpyAsync(charge, d, n * sizeof(float), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
+  density_done(s);
   return ZC_OK;
 }
 
@@ -2358,6 +2365,7 @@ zc_status zc_species_phasespace(zc_sim *s, int k, int quant1, int quant2, const 
                        p.spill_cap, d, P, layout(s), p.ppc[0] * p.ppc[1] * s->TX * s->TY, s->st));
   CK(cudaMemcpyAsync(buf, d, n * sizeof(float), cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
+  density_done(s);
   return ZC_OK;
 }
 
