@@ -198,11 +198,17 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // thread-block cluster: barrier in two halves, and additions to a variable in
-// rank 0's shared memory (it is at the same place in every CTA)
+// rank 0's shared memory (it is at the same place in every CTA).  The aligned
+// forms want a warp's threads together, also after loops that they left apart
+// (bounded waits).
 __device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ int rank0_add(int *v, int n) {
   uint32_t a;
   int old;
