@@ -338,7 +338,11 @@ ZC_API zc_status zc_last_step_ms(zc_sim *sim, float *ms);
  * bracketed by CUDA events on the handle's stream; with 2, only the push
  * (ZC_PHASE_PUSH), so that the rest of the step runs as without profiling.
  * zc_get_profile returns, per phase, the summed device milliseconds and the
- * number of kernel launches since the last reset.  The reference's own
+ * number of kernel launches since the last reset.  Of the push it counts a
+ * species' push each, also where a small grid's species go in one launch (with
+ * their spill lists).  Where fold, filter, Yee advance and external fields go in
+ * one launch (up to 4 filter passes an axis, grids of at least 6 cells), that is
+ * ZC_PHASE_YEE, and the other three have nothing.  The reference's own
  * counters are wall-clock totals of spec_advance and emf_advance
  * (em2d/particles.c:26-59, em2d/emf.c:27-37). */
 enum {
@@ -349,7 +353,7 @@ enum {
     ZC_PHASE_ZERO,          /* current zeroing */
     ZC_PHASE_FOLD,          /* current guard-cell fold */
     ZC_PHASE_SMOOTH,        /* current filter passes */
-    ZC_PHASE_YEE,           /* fused Yee advance */
+    ZC_PHASE_YEE,           /* fused Yee advance, or the whole field phase */
     ZC_PHASE_EMF_GC,        /* field guard cells */
     ZC_PHASE_EXT,           /* external fields */
     ZC_PHASE_WINDOW,        /* moving-window shift and injection */

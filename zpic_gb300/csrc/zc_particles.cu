@@ -899,7 +899,7 @@ cudaError_t launch_push_spill(const PushLaunch &a, int nblocks, cudaStream_t st)
 
 // The integer, rounded once, times a power of two: exact from there on.  (By way
 // of doubles and their division, slow units here, a step of 512^2 cells took
-// 148.4 us, 146.1 now.)
+// 148.4 us instead of 146.1.)
 __global__ void k_fixed_to_float(const unsigned long long *src, float *dst, size_t n) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
     dst[k] = __ll2float_rn((long long)src[k]) * (float)(1.0 / kJFixScale);

@@ -538,9 +538,9 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 // l kLaneRun + kLaneRun - 1 of a chunk of the sorted order one after another,
 // and sums their single-segment currents in registers while they stay in one
 // cell; a lane adds its sums to J when its cell changes.  The deterministic
-// builds do that with integers (RunSums): 118 us for 4.2 M particles on 512^2
+// builds do that with integers (RunSums): 115 us for 4.2 M particles on 512^2
 // cells, where the sums over the lanes of a cell, with 24 words a shuffle
-// step, took 188 to 213; 354 against 683 us for 16.8 M.
+// step, took 188 to 213; 332 against 683 us for 16.8 M.
 //
 // What bounds it (fast build, 2048^2 cells, 67 M particles): no single unit.
 // A launch takes 0.940 ms against 0.49 ms for its 48 bytes a particle at the
@@ -562,7 +562,8 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
 #define ZC_PUSH_MIN_CTAS 6
 #endif
 // the deterministic builds: 768 threads per SM (80 registers each; 512^2, 32 x
-// 16 tiles: 118 us; 512 threads, no spills: 120; 1024, 64 registers: 199)
+// 16 tiles, measured before a lane's sums were cut in 32 bits: 118 us; 512
+// threads, no spills: 120; 1024, 64 registers: 199)
 constexpr int kDetThreads = 768;
 //
 // SPLIT: a tile is worked on by a cluster of `parts` CTAs (this one is
