@@ -675,11 +675,12 @@ int spill_blocks(const zc_sim *s) {
 }
 
 // the species' kinetic sum after a push of `parts` parts a tile (0: a launch
-// of its own); deterministic: a value a tile, whatever its parts
+// of its own); deterministic: two words a tile, whatever its parts
 KinSum kin_sum(const zc_sim *s, const SpeciesState &p, int parts) {
   KinSum K;
   K.part = p.d_ekin_tile;
-  K.fix = s->deterministic ? p.d_ekin_fix : nullptr;
+  K.words = s->deterministic ? reinterpret_cast<const long long *>(p.d_ekin_tile) : nullptr;
+  K.fix = p.d_ekin_fix;
   K.out = p.d_ekin;
   K.n = s->deterministic ? s->ntiles : s->ntiles * std::max(parts, 1) + (parts ? kSpillParts : spill_blocks(s));
   K.q_mq = p.q * p.m_q;
@@ -734,6 +735,7 @@ zc_status species_push(zc_sim *s, SpeciesState &p, int parts, PushSpecies &a, in
   a.S = spill_of(p, out);
   a.ekin = p.d_ekin_tile;
   a.ekin_spill = p.d_ekin_tile + (size_t)s->ntiles * std::max(parts, 1);
+  a.ekin_words = reinterpret_cast<long long *>(p.d_ekin_tile);
   a.ekin_fix = p.d_ekin_fix;
   a.C = C;
   return ZC_OK;

@@ -1264,19 +1264,13 @@ __global__ void k_energy_direct(const double *partial, int nblocks, float dx, fl
 __global__ void __launch_bounds__(256) k_energy_history_row(const double *partial, int nblocks, float dx, float dy,
                                                             const KinSum *ks, int nsp, double *hist, int *hist_n,
                                                             int cap, int cols) {
-  __shared__ double sred[8];
   const int t = threadIdx.x, c = t >> 5, lane = t & 31;
   // each species' kinetic energy from its partials, by the whole block (as
   // k_kin_sums makes it), before the row
   for (int k = 0; k < nsp; ++k) {
     const KinSum &K = ks[k];
-    double s = 0;
-    for (int i = t; i < K.n; i += 256) s += K.part[i];
-    s = block_sum_double<256>(s, sred);
-    if (t == 0) {
-      if (K.fix) s += efix_join((long long)K.fix[0], (long long)K.fix[1]);
-      *K.out = K.q_mq * s * dx * dy;  // spec->energy (particles.c:1231)
-    }
+    const double s = kin_total<256>(K);
+    if (t == 0) *K.out = K.q_mq * s * dx * dy;  // spec->energy (particles.c:1231)
   }
   __syncthreads();
   const int n = *hist_n;

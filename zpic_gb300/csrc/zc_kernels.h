@@ -72,9 +72,21 @@ __device__ __forceinline__ void efix_split(float v, long long &hi, long long &lo
   hi = __float2ll_rn(hf);
   lo = __float2ll_rn(__fmul_rn(__fsub_rn(t, hf), 4294967296.0f));  // 2^32
 }
-__host__ __device__ __forceinline__ double efix_join(long long hi, long long lo) {
-  return (double)hi / kEFixHi + (double)lo / kEFixLo;
-}
+// Sums of such pairs, exact: a counts 2^2, c 2^-30, d 2^-62.  What value() makes
+// of them depends on the sum alone, not on how it was put together.
+struct EfixSum {
+  long long a = 0, c = 0, d = 0;
+  __device__ __forceinline__ void add(long long hi, long long lo) {
+    a += hi >> 32;
+    c += (hi & 0xffffffffLL) + (lo >> 32);
+    d += lo & 0xffffffffLL;
+  }
+  __device__ __forceinline__ double value() const {
+    const long long c1 = c + (d >> 32);
+    return (double)(a + (c1 >> 32)) * 4.0 +
+           ((double)(c1 & 0xffffffffLL) * (1.0 / kEFixHi) + (double)(d & 0xffffffffLL) * (1.0 / kEFixLo));
+  }
+};
 
 // one species' push
 struct PushSpecies {
@@ -82,9 +94,10 @@ struct PushSpecies {
   TileSet T;
   Outbox Oin, O;                          // pending incoming (previous step), leavers (this step)
   Spill Sin, S;                           // spilled particles: to push, and those of this step
-  double *ekin;                           // kinetic energy of every tile part (deterministic: every tile)
+  double *ekin;                           // kinetic energy of every tile part
   double *ekin_spill;                     // and of every block of the spill push
-  unsigned long long *ekin_fix;           // deterministic mode: the spill push's fixed-point words
+  long long *ekin_words;                  // deterministic mode: every tile's two fixed-point words instead,
+  unsigned long long *ekin_fix;           // and the spill push's
   PushConst C;
 };
 
@@ -231,14 +244,50 @@ cudaError_t launch_charge(const Particles &buf, const int *off, const int *np, i
                           const int *spill_cnt, int spill_cap, float *rho, int nx, int ny, float q, int mw,
                           cudaStream_t st);
 // the kinetic-energy sum of one species into *out: n partials of tile parts
-// and spill blocks; with fix, the two 64-bit fixed-point words of efix_join
+// and spill blocks (part); deterministic mode: n tiles' fixed-point words, two
+// each (words), and the spill push's two (fix)
 struct KinSum {
   const double *part;
+  const long long *words;
   const unsigned long long *fix;
   double *out;
   int n;
   float q_mq;
 };
+#ifdef __CUDACC__
+// the sum of K's partials, by a block of NT threads; in thread 0.  Partials in
+// a fixed order; words as integers, rounded once, so that neither the tiles nor
+// the particles that spilled have a part in the bits.
+template <int NT>
+__device__ __forceinline__ double kin_total(const KinSum &K) {
+  __shared__ double sred[NT / 32];
+  __shared__ EfixSum swords[NT / 32];
+  if (!K.words) {
+    double s = 0;
+    for (int i = threadIdx.x; i < K.n; i += NT) s += K.part[i];
+    return block_sum_double<NT>(s, sred);
+  }
+  EfixSum e;
+  for (int i = threadIdx.x; i < K.n; i += NT) e.add(K.words[2 * (size_t)i], K.words[2 * (size_t)i + 1]);
+  if (threadIdx.x == 0) e.add((long long)K.fix[0], (long long)K.fix[1]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    e.a += __shfl_down_sync(0xffffffffu, e.a, o);
+    e.c += __shfl_down_sync(0xffffffffu, e.c, o);
+    e.d += __shfl_down_sync(0xffffffffu, e.d, o);
+  }
+  if ((threadIdx.x & 31) == 0) swords[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < NT / 32; ++w) {
+      e.a += swords[w].a;
+      e.c += swords[w].c;
+      e.d += swords[w].d;
+    }
+  __syncthreads();
+  return e.value();
+}
+#endif
 // one block a species
 struct KinSums {
   KinSum k[kMaxTogether];

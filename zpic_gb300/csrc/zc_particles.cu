@@ -865,18 +865,12 @@ __global__ void k_charge_fold(float *rho, int nx, int ny, int mw) {
     for (int i = threadIdx.x; i < nx + 1; i += blockDim.x) rho[i] += rho[i + ny * nrow];
 }
 
-// sums of the kinetic-energy partials in a fixed order, one block a species
+// sums of the kinetic-energy partials, one block a species
 __global__ void __launch_bounds__(256) k_kin_sums(const __grid_constant__ KinSums S, float dx, float dy) {
-  __shared__ double sred[8];
   const KinSum &K = S.k[blockIdx.x];
-  double s = 0;
-  for (int i = threadIdx.x; i < K.n; i += 256) s += K.part[i];
-  s = block_sum_double<256>(s, sred);
-  if (threadIdx.x == 0) {
-    if (K.fix) s += efix_join((long long)K.fix[0], (long long)K.fix[1]);
-    // spec->energy = q * m_q * energy * dx * dy  (particles.c:1231)
-    *K.out = K.q_mq * s * dx * dy;
-  }
+  const double s = kin_total<256>(K);
+  // spec->energy = q * m_q * energy * dx * dy  (particles.c:1231)
+  if (threadIdx.x == 0) *K.out = K.q_mq * s * dx * dy;
 }
 
 // ---------------------------------------------------------------------------

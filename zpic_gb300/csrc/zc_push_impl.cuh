@@ -1018,8 +1018,7 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
 
   if constexpr (DET) {
     // kinetic energy: integer sums, exact in any order, of the whole tile
-    // (its parts' too, so that the one rounding does not depend on which
-    // part held which particle)
+    // (its parts' too)
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       khi += __shfl_down_sync(0xffffffffu, khi, off);
@@ -1044,7 +1043,10 @@ __device__ __forceinline__ void push_tile(const CUtensorMap &tm_eb, const PushSp
   if (threadIdx.x == 0 && (!SPLIT || rank == 0)) {
     T.np[t] = n_own + min(s_app, T.cap[t] - n_own);
     O.cnt[t] = min(s_leave, O.cap);
-    if constexpr (DET) A.ekin[t] = efix_join((long long)s_ekin[0], (long long)s_ekin[1]);
+    if constexpr (DET) {
+      A.ekin_words[2 * (size_t)t] = (long long)s_ekin[0];
+      A.ekin_words[2 * (size_t)t + 1] = (long long)s_ekin[1];
+    }
   }
   if constexpr (DET) {
     // the integer J tile goes to the global fixed-point planes (units of
