@@ -631,9 +631,8 @@ __global__ void k_adj_push(State<R> s, State<R> o, const R *w, const int *birth,
   // of 10^6 particles, float32: 2.35 ms against 2.44), else every gridDim-th
   // round (float64: 30.5 ms against 32.9; float32 with a window 5.75, 6.06)
   const Share mine(P.np);
-  const int first = V4 ? mine.first : (int)(blockIdx.x * blockDim.x), end = V4 ? mine.end : P.np;
-  const int stride = V4 ? (int)blockDim.x : (int)(gridDim.x * blockDim.x);
-  for (int p = first + (int)threadIdx.x; p < end; p += stride) {
+  for (int p = (V4 ? mine.first : blockIdx.x * blockDim.x) + threadIdx.x; p < (V4 ? mine.end : P.np);
+       p += V4 ? blockDim.x : gridDim.x * blockDim.x) {
     const int ix = s.ix[p], iy = s.iy[p];
     const R x = s.x[p], y = s.y[p];
     const R u[3] = {s.ux[p], s.uy[p], s.uz[p]};
