@@ -1530,6 +1530,7 @@ struct Engine : EngineBase {
   }
 
   zc_status save_checkpoint(const DevState<R> &from, const R *fE, const R *fB) {
+    TRY_(checkpoint_room(nck + 1));
     TRY_(copy_state(ck_s[nck], from));
     TRY_(copy_fields(ck_f[nck], ck_f[nck] + 3 * pl, fE, fB));
     ++nck;
@@ -1584,28 +1585,29 @@ struct Engine : EngineBase {
   }
 
   // Room for the pre-step states of nsteps steps, as far as 8 GiB and half of
-  // the memory that is free go (what a run cannot do without is allocated
-  // before); without it the reverse sweep recomputes more.  (200 steps of 10^6
-  // particles take 6.7 GB; recomputing 160 of them took 8 ms of a reverse sweep
-  // of 33.)
-  void keep_room(int nsteps) {
+  // the memory that is free go (what a run cannot do without, its checkpoints,
+  // is allocated before); without it the reverse sweep recomputes more.  (200
+  // steps of 10^6 particles take 6.7 GB; recomputing 160 of them took 8 ms of a
+  // reverse sweep of 33.)
+  zc_status keep_room(int nsteps) {
     const int want = (nsteps - 1) / K + 1;
     int fit = (int)std::min(8.0 * (1 << 30) / (K * slot_bytes()), (double)want);
-    if (fit <= kseg) return;
+    if (fit <= kseg) return ZC_OK;  // (checkpoints then come while the GPU works)
+    TRY_(checkpoint_room(want));
     size_t free_mem = 0, total = 0;
     if (cudaMemGetInfo(&free_mem, &total) != cudaSuccess) {
       cudaGetLastError();
-      return;
+      return ZC_OK;
     }
     fit = (int)std::min((double)fit, kseg + 0.5 * (double)free_mem / (K * slot_bytes()));
     if (fit > kseg && add_slots((fit - kseg) * K)) kseg = fit;
+    return ZC_OK;
   }
 
   zc_status forward(int nsteps, double *obj, double *kin) override {
     if (!have_state) return afail(ZC_ESTATE, "adjoint engine: no initial state");
     if (nsteps <= 0) return afail(ZC_EINVAL, "adjoint engine: nsteps must be > 0");
-    TRY_(checkpoint_room((nsteps - 1) / K + 1));
-    keep_room(nsteps);
+    TRY_(keep_room(nsteps));
     plan_shifts(nsteps);
     ACK(cudaEventRecord(e0, st));
     nck = 0;
